@@ -35,6 +35,7 @@
 #include "host_common.cuh"
 #include "kernels.cuh"
 #include "kernels_warp.cuh"
+#include "kernels_chunk.cuh"
 
 using namespace dmpm;
 using namespace dmpm_host;
@@ -487,6 +488,7 @@ struct dmpm_batch::Impl {
     WArgs args(int t) const {
         WArgs a{};
         a.n = (int)P[t + 1];
+        a.chunk = scatter_chunk(a.n);
         a.np = np0;
         a.npl = S[t];
         a.npn = S[t + 1];
@@ -500,6 +502,7 @@ struct dmpm_batch::Impl {
         a.n_items_dev = e.item_end + (A[t + 1] - 1);
         a.ig = ig;
         a.item_inst = e.item_inst;
+        a.pinst = pinst;
         a.st = st[t];
         a.st_next = st[t + 1];
         a.xlo = 1;
@@ -528,7 +531,7 @@ struct dmpm_batch::Impl {
         DMPM_CK(cudaMemsetAsync(grid[t], 0, Gt * sizeof(node4<float>), b->stream));
         k_stress<false><<<(unsigned)((a.n + pb - 1) / pb), pb, 0, b->stream>>>(a);
         launched();
-        k_p2g_w<false, ITEMS_BATCH><<<wb, DMPM_P2G_THREADS, 0, b->stream>>>(a);
+        k_p2g_c<true, false><<<chunk_blocks(a.n, a.chunk), DMPM_CHUNK_THREADS, 0, b->stream>>>(a);
         launched();
         k_gop_inplace<<<(unsigned)((Gt + 255) / 256), 256, 0, b->stream>>>(grid[t], Gt, a.dt, a.fext[0], a.fext[1],
                                                                              a.fext[2]);
@@ -579,9 +582,9 @@ struct dmpm_batch::Impl {
         const unsigned wb = warp_blocks(t);
         const bool ex = prm.adjoint_mode == DMPM_ADJ_EXACT;
         DMPM_CK(cudaMemsetAsync(gadj, 0, Gt * sizeof(node4<float>), b->stream));
-        const unsigned ws = scatter_blocks(t);
-        if (ex) k_adj_scatter_w<true, false, ITEMS_BATCH><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, b->stream>>>(a);
-        else k_adj_scatter_w<false, false, ITEMS_BATCH><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, b->stream>>>(a);
+        const unsigned cb = chunk_blocks(a.n, a.chunk);
+        if (ex) k_adj_scatter_c<true, true, false><<<cb, DMPM_CHUNK_THREADS, 0, b->stream>>>(a);
+        else k_adj_scatter_c<false, true, false><<<cb, DMPM_CHUNK_THREADS, 0, b->stream>>>(a);
         launched();
         const unsigned gb = (unsigned)((Gt + 255) / 256);
         if (ex) k_adj_gop_w<true><<<gb, 256, 0, b->stream>>>(grid[t], gadj, gadj2, Gt, a.dt, a.fext[0], a.fext[1], a.fext[2]);

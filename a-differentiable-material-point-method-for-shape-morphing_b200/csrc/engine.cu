@@ -28,6 +28,7 @@
 #include "kernels.cuh"
 #include "kernels_warp.cuh"
 #include "kernels_brick.cuh"
+#include "kernels_chunk.cuh"
 #include "host_common.cuh"
 
 using namespace dmpm;
@@ -1027,6 +1028,7 @@ template <class T> class Engine : public EngineBase {
         WArgs a{};
         const dmpm_params& P = ctx_->prm;
         a.n = n_;
+        a.chunk = scatter_chunk(n_);
         a.np = a.npl = a.npn = np_;
         a.geo = geo_;
         a.dt = (float)P.dt;
@@ -1102,8 +1104,8 @@ template <class T> class Engine : public EngineBase {
                 else k_p2g_fix_b<4, false><<<brick_blocks(k_p2g_fix_b<4, false>), bt, 0, ctx_->stream>>>(a);
             } else if (dm && gen) k_p2g_w<true, ITEMS_PERSISTENT, true><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
             else if (dm) k_p2g_w<false, ITEMS_PERSISTENT, true><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
-            else if (gen) k_p2g_w<true, ITEMS_PERSISTENT><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
-            else k_p2g_w<false, ITEMS_PERSISTENT><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
+            else if (gen) k_p2g_c<false, true><<<chunk_blocks(n_, a.chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a);
+            else k_p2g_c<false, false><<<chunk_blocks(n_, a.chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a);
             launched();
             if (dm) {
                 k_fix_to_node4<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, 0, (node4<float>*)g);
@@ -1366,12 +1368,15 @@ template <class T> class Engine : public EngineBase {
                 launch_adj_scatter_fix(a, ex, P.warp_general != 0, ush, ws);
                 launched();
                 k_fix_to_node4<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, 1, (node4<float>*)gadj_);
-            } else if (P.warp_general) {
-                if (ex) k_adj_scatter_w<true, true, ITEMS_PERSISTENT><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, ctx_->stream>>>(a);
-                else k_adj_scatter_w<false, true, ITEMS_PERSISTENT><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, ctx_->stream>>>(a);
             } else {
-                if (ex) k_adj_scatter_w<true, false, ITEMS_PERSISTENT><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, ctx_->stream>>>(a);
-                else k_adj_scatter_w<false, false, ITEMS_PERSISTENT><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, ctx_->stream>>>(a);
+                const unsigned cb = chunk_blocks(n_, a.chunk), ct = DMPM_CHUNK_THREADS;
+                if (P.warp_general) {
+                    if (ex) k_adj_scatter_c<true, false, true><<<cb, ct, 0, ctx_->stream>>>(a);
+                    else k_adj_scatter_c<false, false, true><<<cb, ct, 0, ctx_->stream>>>(a);
+                } else {
+                    if (ex) k_adj_scatter_c<true, false, false><<<cb, ct, 0, ctx_->stream>>>(a);
+                    else k_adj_scatter_c<false, false, false><<<cb, ct, 0, ctx_->stream>>>(a);
+                }
             }
             launched();
             pend();

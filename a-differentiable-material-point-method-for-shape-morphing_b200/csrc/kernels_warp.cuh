@@ -353,6 +353,7 @@ struct InstGeo {
 // have their own strides.
 struct WArgs {
     int n;
+    int chunk;             // particles per warp of the chunk kernels (kernels_chunk.cuh): 8, 16 or 32
     size_t np, npl, npn;
     GridGeom geo;
     float dt, drag, s, fext[3];
@@ -360,6 +361,7 @@ struct WArgs {
     const uint32_t* n_items_dev;  // item count on the device (grid-stride launches), or null: items.n_items
     const InstGeo* ig;            // batch: per-instance grids, indexed by item_inst
     const uint16_t* item_inst;
+    const uint16_t* pinst;        // batch: instance of each particle
     const float* st;       // layer n state
     float* st_next;        // layer n+1 state
     int xlo;               // st and st_next carry the low parts of compensated positions (planes PXL)
