@@ -23,16 +23,40 @@
 
 namespace dmpm {
 
+// J F^{-T} is the cofactor matrix of F, a quadratic form of its entries, and
+// d(J F^{-T})[dF] is linear in both: no division where J is not clamped
+template <class T> DMPM_HD m3<T> cofactors(const m3<T>& F) {
+    m3<T> C;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) C.a[i][j] = cof3(F, i, j);
+    return C;
+}
+template <class T> DMPM_HD m3<T> cofactors_derivative(const m3<T>& F, const m3<T>& dF) {
+    m3<T> C;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+            C.a[i][j] = dF.a[i1][j1] * F.a[i2][j2] + F.a[i1][j1] * dF.a[i2][j2] - dF.a[i1][j2] * F.a[i2][j1] -
+                        F.a[i1][j2] * dF.a[i2][j1];
+        }
+    return C;
+}
+
 template <class T> DMPM_HD m3<T> pk_from_polar(const m3<T>& F, const m3<T>& R, T lam, T mu) {
-    T J = det3(F);
-    J = J > T(1e-6) ? J : T(1e-6);
-    const m3<T> Fit = inv_transpose3(F);
-    const T c = lam * (J - T(1)) * J;
+    const T det = det3(F);
+    const bool clamped = !(det > T(1e-6));
+    const T J = clamped ? T(1e-6) : det;
+    const m3<T> JFit = clamped ? J * inv_transpose3(F) : cofactors(F);
+    const T c = lam * (J - T(1));
     m3<T> P;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) P.a[i][j] = T(2) * mu * (F.a[i][j] - R.a[i][j]) + c * Fit.a[i][j];
+        for (int j = 0; j < 3; j++) P.a[i][j] = T(2) * mu * (F.a[i][j] - R.a[i][j]) + c * JFit.a[i][j];
     return P;
 }
 
@@ -71,6 +95,37 @@ template <class T> DMPM_HD m3<T> rotation_derivative(const m3<T>& R, const m3<T>
     return R * X;
 }
 
+// The same derivative from the symmetric system (tr(S) I - S) x = w, w the
+// axial vector of R^T dF - dF^T R, by the adjugate: one division.
+template <class T> DMPM_HD m3<T> rotation_derivative_sym(const m3<T>& R, const m3<T>& S, const m3<T>& dF, bool guard) {
+    const T k00 = S.a[1][1] + S.a[2][2], k11 = S.a[0][0] + S.a[2][2], k22 = S.a[0][0] + S.a[1][1];
+    const T k01 = -S.a[0][1], k02 = -S.a[0][2], k12 = -S.a[1][2];
+    const T c00 = k11 * k22 - k12 * k12, c01 = k02 * k12 - k01 * k22, c02 = k01 * k12 - k02 * k11;
+    const T c11 = k00 * k22 - k02 * k02, c12 = k01 * k02 - k00 * k12, c22 = k00 * k11 - k01 * k01;
+    const T D = k00 * c00 + k01 * c01 + k02 * c02;
+    if (guard && fabs(D) > T(4.85165195409790278e8)) return rotation_derivative(R, S, dF, true);  // log|D| > 20
+    T w[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const int i = (a + 2) % 3, j = (a + 1) % 3;  // W_21, W_02, W_10
+        T s = T(0);
+#pragma unroll
+        for (int k = 0; k < 3; k++) s += R.a[k][i] * dF.a[k][j] - dF.a[k][i] * R.a[k][j];
+        w[a] = s;
+    }
+    const T id = T(1) / D;
+    const T x0 = id * (c00 * w[0] + c01 * w[1] + c02 * w[2]), x1 = id * (c01 * w[0] + c11 * w[1] + c12 * w[2]),
+            x2 = id * (c02 * w[0] + c12 * w[1] + c22 * w[2]);
+    m3<T> r;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {  // R [x]_x
+        r.a[i][0] = R.a[i][1] * x2 - R.a[i][2] * x1;
+        r.a[i][1] = R.a[i][2] * x0 - R.a[i][0] * x2;
+        r.a[i][2] = R.a[i][0] * x1 - R.a[i][1] * x0;
+    }
+    return r;
+}
+
 // sum_ij d(J F^{-T})_ab / dF_ij dF_ij by central differences, delta = 1e-6.
 template <class T> DMPM_HD m3<T> djfit_fd_mult(const m3<T>& F, const m3<T>& dF) {
     const T delta = T(1e-6);
@@ -96,30 +151,34 @@ template <class T> DMPM_HD m3<T> djfit_fd_mult(const m3<T>& F, const m3<T>& dF) 
     return acc;
 }
 
-template <bool EXACT, class T>
+// FD (REFCOMPAT only): d(J F^{-T}) by the reference's finite differences and dR
+// from its own linear system; without it by the closed forms above, which are
+// what the differences (noise ~1e-10 of their size) approximate.
+template <bool EXACT, bool FD = !EXACT, class T>
 DMPM_HD m3<T> d2_mult_from_polar(const m3<T>& F, const m3<T>& R, const m3<T>& S, T lam, T mu, const m3<T>& dF) {
     const T detF = det3(F);
-    const m3<T> Fit = inv_transpose3(F);
+    const bool clamped = !(detF > T(1e-6));
+    const T J = clamped ? T(1e-6) : detF;
     m3<T> ret = (T(2) * mu) * dF;
-    if (!EXACT) {
-        const T J = detF > T(1e-6) ? detF : T(1e-6);
+    if (FD) {
+        const m3<T> Fit = inv_transpose3(F);
         ret = ret + (lam * J * ddot(J * Fit, dF)) * Fit;
         ret = ret + (lam * (J - T(1))) * djfit_fd_mult(F, dF);
-        ret = ret - (T(2) * mu) * rotation_derivative(R, S, dF, true);
-    } else {
-        const bool clamped = !(detF > T(1e-6));
-        const T J = clamped ? T(1e-6) : detF;
-        const m3<T> FdF = Fit * mtm(dF, Fit);  // F^{-T} dF^T F^{-T}
-        if (!clamped) {
-            const T c = ddot(Fit, dF);
-            ret = ret + (lam * J * J * c) * Fit;
-            ret = ret + (lam * (J - T(1)) * J) * (c * Fit - FdF);
-        } else {
-            ret = ret - (lam * (J - T(1)) * J) * FdF;
-        }
-        ret = ret - (T(2) * mu) * rotation_derivative(R, S, dF, false);
+        return ret - (T(2) * mu) * rotation_derivative(R, S, dF, true);
     }
-    return ret;
+    if (!clamped) {
+        const m3<T> C = cofactors(F);
+        ret = ret + (lam * ddot(C, dF)) * C;
+        ret = ret + (lam * (J - T(1))) * cofactors_derivative(F, dF);
+    } else if (EXACT) {
+        const m3<T> Fit = inv_transpose3(F);
+        ret = ret - (lam * (J - T(1)) * J) * (Fit * mtm(dF, Fit));  // F^{-T} dF^T F^{-T}
+    } else {
+        const m3<T> Fit = inv_transpose3(F);
+        ret = ret + (lam * J * ddot(J * Fit, dF)) * Fit;
+        ret = ret + (lam * (J - T(1))) * cofactors_derivative(F, dF);
+    }
+    return ret - (T(2) * mu) * rotation_derivative_sym(R, S, dF, !EXACT);
 }
 
 template <bool EXACT, class T> DMPM_HD m3<T> d2_mult(const m3<T>& F, T lam, T mu, const m3<T>& dF) {

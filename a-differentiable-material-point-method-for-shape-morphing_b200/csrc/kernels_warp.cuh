@@ -1200,7 +1200,7 @@ __device__ __forceinline__ void finalize_particle(const WArgs& a, int p, const I
     const m3<float> Cnext = mat(FS_CNEXT);
     const m3<float> dFn = mat(FS_AF);
     const m3<float> Tr = mtm(m3_eye<float>() + a.dt * Cnext, dFn);
-    const m3<float> d2 = m3_cast<float>(d2_mult_from_polar<EXACT>(Fed, Rd, Sd, lam, mu, m3_cast<double>(dLdP)));
+    const m3<float> d2 = m3_cast<float>(d2_mult_from_polar<EXACT, false>(Fed, Rd, Sd, lam, mu, m3_cast<double>(dLdP)));
     m3<float> dLdF, dLdFe;
     if (EXACT) {
         dLdFe = (1.f - a.s) * Tr + dFstress + d2;

@@ -263,29 +263,38 @@ template <class T> DMPM_HD void polar3(const m3<T>& F, m3<T>& R, m3<T>& S) {
             S.a[i][j] = V.a[i][0] * s[0] * V.a[j][0] + V.a[i][1] * s[1] * V.a[j][1] + V.a[i][2] * s[2] * V.a[j][2];
 }
 
-// one scaled Newton step X <- (z X + c X^-T) / 2, c = cbrt(det X), z = 1 / c;
-// true when the squared change is at most tol times the squared norm
+// one Newton step X <- (z X + X^-T / z) / 2 with z = det(X)^(-1/3), or z = 1
+// where det X is within 1/16 of 1 (the scaling gains nothing there and costs a
+// cube root); true when the squared change is at most tol times 3, the squared
+// norm of a rotation
 template <class T> DMPM_HD bool newton_step(m3<T>& X, T tol) {
-    const m3<T> Xit = inv_transpose3(X);
-    const T c = cbrt(det3(X));
-    const T z = T(1) / c;
-    T diff = T(0), nrm = T(0);
+    m3<T> C;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) C.a[i][j] = cof3(X, i, j);
+    const T det = C.a[0][0] * X.a[0][0] + C.a[1][0] * X.a[1][0] + C.a[2][0] * X.a[2][0];
+    T zx = T(0.5), zc = T(0.5) / det;  // X^-T = C / det
+    if (fabs(det - T(1)) > T(0.0625)) {
+        const T c = cbrt(det);
+        zx /= c;
+        zc *= c;
+    }
+    T diff = T(0);
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            const T y = T(0.5) * (z * X.a[i][j] + c * Xit.a[i][j]);
+            const T y = zx * X.a[i][j] + zc * C.a[i][j];
             diff += (y - X.a[i][j]) * (y - X.a[i][j]);
-            nrm += y * y;
             X.a[i][j] = y;
         }
-    return diff <= tol * nrm;
+    return diff <= T(3) * tol;
 }
-
 
 // Polar decomposition F = R S of a matrix with det F > 0 by the scaled Newton
 // iteration  X <- (z X + X^{-T} / z) / 2,  z = det(X)^{-1/3}  (Higham 1986,
-// determinant scaling), which converges quadratically to the rotation of the
+// determinant scaling; unscaled near det X = 1), which converges quadratically to the rotation of the
 // polar decomposition -- for det F > 0 the same R that polar3 obtains from
 // the SVD -- in a few inverse-transposes instead of an SVD.  Returns false,
 // leaving R and S unset, when det F is not comfortably positive or the
