@@ -106,10 +106,6 @@ struct BEpoch {
 struct dmpm_batch {
     int device = 0;
     cudaStream_t stream = nullptr;
-    // second stream for the finalize's transport part, forked from and joined
-    // back into stream by the two events
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     std::string err;
     struct Impl;
     std::unique_ptr<Impl> impl;
@@ -148,7 +144,7 @@ struct dmpm_batch::Impl {
     std::vector<float*> st, aux;
     std::vector<node4<float>*> grid;
     float* adj[2] = {nullptr, nullptr};
-    float *adjn = nullptr, *gath = nullptr;
+    float* adjn = nullptr;
     node4<float>*gadj = nullptr, *gadj2 = nullptr;
     double* ctrl_acc = nullptr;
     std::vector<BEpoch> ep;
@@ -391,7 +387,7 @@ struct dmpm_batch::Impl {
         size_t tot = 0;
         for (int t = 1; t <= smax; t++) tot += (size_t)NSTATE_X * S[t] * 4;               // states
         for (int t = 0; t < smax; t++) tot += (size_t)kAux * S[t] * 4 + node_prefix[A[t + 1]] * 16;  // aux, grids
-        tot += 2 * (size_t)NSTATE * np0 * 4 + (12 + 18) * np0 * 4 + 9 * np0 * 8 + 3 * Gtot * 16;
+        tot += 2 * (size_t)NSTATE * np0 * 4 + 12 * np0 * 4 + 9 * np0 * 8 + 3 * Gtot * 16;
         return tot;
     }
 
@@ -418,7 +414,6 @@ struct dmpm_batch::Impl {
         adj[0] = (float*)layers.alloc((size_t)NSTATE * np0 * 4);
         adj[1] = (float*)layers.alloc((size_t)NSTATE * np0 * 4);
         adjn = (float*)layers.alloc((size_t)12 * np0 * 4);
-        gath = (float*)layers.alloc((size_t)18 * np0 * 4);
         ctrl_acc = (double*)layers.alloc((size_t)9 * np0 * 8);
         gadj = (node4<float>*)layers.alloc(Gtot * sizeof(node4<float>));
         gadj2 = (node4<float>*)layers.alloc(2 * Gtot * sizeof(node4<float>));
@@ -517,12 +512,6 @@ struct dmpm_batch::Impl {
         const size_t most = (P[t + 1] * 32 + 255) / 256;  // one item per particle at most
         return (unsigned)std::max<size_t>(1, std::min<size_t>(most, (size_t)sms * ctas_per_sm()));
     }
-    // the adjoint scatter's persistent grid: its own blocks per SM (kernels_warp.cuh), not the tuned setting
-    unsigned scatter_blocks(int t) const {
-        const size_t most = (P[t + 1] * 32 + DMPM_ADJ_SCATTER_THREADS - 1) / DMPM_ADJ_SCATTER_THREADS;
-        return (unsigned)std::max<size_t>(1, std::min<size_t>(most, (size_t)sms * DMPM_ADJ_SCATTER_CTAS));
-    }
-
     void step(int t) {
         WArgs a = args(t);
         const size_t Gt = node_prefix[A[t + 1]];
@@ -574,7 +563,6 @@ struct dmpm_batch::Impl {
         a.adj_next = adj[(t + 1) & 1];
         a.adj = adj[t & 1];
         a.adjn = adjn;
-        a.gath = gath;
         a.gadj = gadj;
         a.gadj2 = gadj2;
         a.ctrl_acc = ctrl_acc;
@@ -590,16 +578,8 @@ struct dmpm_batch::Impl {
         if (ex) k_adj_gop_w<true><<<gb, 256, 0, b->stream>>>(grid[t], gadj, gadj2, Gt, a.dt, a.fext[0], a.fext[1], a.fext[2]);
         else k_adj_gop_w<false><<<gb, 256, 0, b->stream>>>(grid[t], gadj, gadj2, Gt, a.dt, a.fext[0], a.fext[1], a.fext[2]);
         launched();
-        if (ex) k_adj_gather_w<true, ITEMS_BATCH><<<wb, DMPM_GATHER_THREADS, 0, b->stream>>>(a);
-        else k_adj_gather_w<false, ITEMS_BATCH><<<wb, DMPM_GATHER_THREADS, 0, b->stream>>>(a);
+        launch_gather<true>(a, ex, b->stream);
         launched();
-        DMPM_CK(cudaEventRecord(b->ev_fork, b->stream));
-        DMPM_CK(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
-        launch_finalize_split(a, ex, b->stream, b->side);
-        launched();
-        launched();
-        DMPM_CK(cudaEventRecord(b->ev_join, b->side));
-        DMPM_CK(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
     }
 
     // the whole gradient evaluation, enqueued on the stream (capturable: no
@@ -805,13 +785,6 @@ int dmpm_batch_create(int device, int count, const dmpm_instance* instances, dmp
         delete b;
         return DMPM_ERR_CUDA;
     }
-    if (cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        dmpm_batch_destroy(b);
-        return DMPM_ERR_CUDA;
-    }
     b->impl.reset(new dmpm_batch::Impl(b));
     const int st = bguard(b, [&](dmpm_batch::Impl& im) { im.create(instances, count); return DMPM_OK; });
     if (st != DMPM_OK) {
@@ -826,12 +799,8 @@ int dmpm_batch_destroy(dmpm_batch* b) {
     if (!b) return DMPM_ERR_ARG;
     cudaSetDevice(b->device);
     cudaStreamSynchronize(b->stream);
-    if (b->side) cudaStreamSynchronize(b->side);
     b->impl.reset();
     cudaStreamDestroy(b->stream);
-    if (b->side) cudaStreamDestroy(b->side);
-    if (b->ev_fork) cudaEventDestroy(b->ev_fork);
-    if (b->ev_join) cudaEventDestroy(b->ev_join);
     delete b;
     return DMPM_OK;
 }

@@ -843,7 +843,6 @@ template <class T> class Engine : public EngineBase {
                 for (int i = 0; i < k_; i++) seg_G_[i] = (T*)layer_arena_.alloc(g_bytes);
             }
             adjn_ = (T*)layer_arena_.alloc(12 * np_ * sizeof(T));
-            gath_ = (T*)layer_arena_.alloc(18 * np_ * sizeof(T));
             alloc_sort();
         }
         if (P.keep_intermediates) {
@@ -1339,7 +1338,6 @@ template <class T> class Engine : public EngineBase {
             a.adj_next = (const float*)adj_of(i + 1, false);
             a.adj = (float*)adj_of(i, true);
             a.adjn = (float*)adjn_;
-            a.gath = (float*)gath_;
             a.gadj = (node4<float>*)gadj_;
             a.gadj2 = (node4<float>*)gadj2_;
             a.ctrl_grad = (float*)layers_[i].ctrl_grad;
@@ -1357,8 +1355,7 @@ template <class T> class Engine : public EngineBase {
             } else {
                 DMPM_CK(cudaMemsetAsync(gadj_, 0, G_ * sizeof(node4<T>), ctx_->stream));
             }
-            const unsigned ws = warp_blocks(DMPM_ADJ_SCATTER_CTAS, DMPM_ADJ_SCATTER_THREADS),
-                           wg = warp_blocks(DMPM_GATHER_CTAS, DMPM_GATHER_THREADS);
+            const unsigned ws = warp_blocks(DMPM_ADJ_SCATTER_CTAS, DMPM_ADJ_SCATTER_THREADS);
             const int ush = set_units(a, ep);
             pbeg(K_ADJ_SCATTER);
             if (dm) {
@@ -1391,40 +1388,9 @@ template <class T> class Engine : public EngineBase {
                                           sizeof(node4<T>), G_, cudaMemcpyDeviceToDevice, ctx_->stream));
             }
             pbeg(K_ADJ_GATHER);
-            if (ex) {
-                k_adj_gather_w<true, ITEMS_PERSISTENT><<<wg, DMPM_GATHER_THREADS, 0, ctx_->stream>>>(a);
-            } else {
-                k_adj_gather_w<false, ITEMS_PERSISTENT><<<wg, DMPM_GATHER_THREADS, 0, ctx_->stream>>>(a);
-            }
+            launch_gather<false>(a, ex, ctx_->stream);
             launched();
             pend();
-            if (DMPM_SPLIT_FINALIZE && !prof_) {
-                // fork: the transport part on the side stream after the gather,
-                // join: the main stream continues after both parts
-                side_stream();
-                DMPM_CK(cudaEventRecord(ev_fork_, ctx_->stream));
-                DMPM_CK(cudaStreamWaitEvent(side_, ev_fork_, 0));
-                launch_finalize_split(a, ex, ctx_->stream, side_);
-                launched();
-                launched();
-                DMPM_CK(cudaEventRecord(ev_join_, side_));
-                DMPM_CK(cudaStreamWaitEvent(ctx_->stream, ev_join_, 0));
-            } else if (DMPM_SPLIT_FINALIZE) {
-                // profiled: the two parts one after the other, each timed
-                pbeg(K_ADJ_TRANSPORT);
-                launch_finalize_part(a, ex, FIN_TRANSPORT, ctx_->stream);
-                launched();
-                pend();
-                pbeg(K_ADJ_FINALIZE);
-                launch_finalize_part(a, ex, FIN_STRESS, ctx_->stream);
-                launched();
-                pend();
-            } else {
-                pbeg(K_ADJ_FINALIZE);
-                launch_finalize(a, ex, ctx_->stream);
-                launched();
-                pend();
-            }
             return;
         }
         AdjArgs<T> a{};
@@ -1497,8 +1463,6 @@ template <class T> class Engine : public EngineBase {
         if (control < 0 || control > top) throw ArgError{"control_layer out of range"};
         if (top < L_ - 1 && !layers_[top].adj) throw StateError{"set keep_adjoints to start the adjoint below the last layer"};
         reset_status();
-        // the finalize's second stream exists before any capture of the adjoint steps
-        if (kWarp && DMPM_SPLIT_FINALIZE) side_stream();
         if (ctrl_acc_) DMPM_CK(cudaMemsetAsync(ctrl_acc_, 0, 9 * np_ * sizeof(double), ctx_->stream));
         if (k_ == 1) {
             auto body = [&]() {
@@ -1786,25 +1750,9 @@ template <class T> class Engine : public EngineBase {
         harvest();
         for (cudaEvent_t e : event_pool_) cudaEventDestroy(e);
         if (host_misc_) cudaFreeHost(host_misc_);
-        if (side_) {
-            cudaStreamSynchronize(side_);
-            cudaStreamDestroy(side_);
-            cudaEventDestroy(ev_fork_);
-            cudaEventDestroy(ev_join_);
-        }
-    }
-
-    // second stream (and its fork/join events) for work that runs beside the main stream
-    void side_stream() {
-        if (side_) return;
-        DMPM_CK(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
-        DMPM_CK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
-        DMPM_CK(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
     }
 
    private:
-    cudaStream_t side_ = nullptr;
-    cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
     struct LayerSlots {
         T* G = nullptr;
         T* st = nullptr;
@@ -1863,7 +1811,6 @@ template <class T> class Engine : public EngineBase {
     T* gscratch_ = nullptr;
     std::vector<T*> seg_G_;
     T* adjn_ = nullptr;
-    T* gath_ = nullptr;
     std::vector<Epoch> epochs_;
     uint32_t* sk_[2] = {nullptr, nullptr};
     uint32_t* sv_[2] = {nullptr, nullptr};

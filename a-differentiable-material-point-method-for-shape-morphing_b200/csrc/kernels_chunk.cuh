@@ -30,7 +30,7 @@
 // lane) read 21 words per particle.  Groups of strays cost: without the
 // grouping (a group per run of the sorted order) 32.8 and 42.6 us.
 #pragma once
-#include "kernels_warp.cuh"
+#include "kernels_brick.cuh"
 
 namespace dmpm {
 
@@ -273,6 +273,274 @@ inline int scatter_chunk(int n) {
 inline unsigned chunk_blocks(int n, int chunk) {
     const int per = chunk * (DMPM_CHUNK_THREADS / 32);
     return (unsigned)((n + per - 1) / per);
+}
+
+// ------------------------------------------------------------------ adjoint gather + finalize
+// One thread per particle of the sorted order, reading the nodes where they lie:
+// the particles of a warp share one to three cells, so their reads are
+// broadcasts from L1.  The thread keeps the 18 sums of its particle in registers
+// and goes on to the finalize with them (as two kernels the sums made a round
+// trip of 144 bytes per particle, and the finalize a second and a third launch).
+// Small clouds give a particle four threads, one per stencil slab (SPLIT).
+//
+// Measured per step on the 64^3, 267k-particle rollout (event times): 98 us, and
+// the warp-item gather with the two finalize kernels behind it 82.6 + 41.4 (+ 14.6
+// beside them); 79k particles with the reference's adjoint 33 against 27 + 57 us;
+// 8.7k particles 14.7 against 12.6 + 8.7.  The node sums take 55 us of the 98 (in a
+// kernel of their own): 22.3 M warp instructions at 42 % issue with 16 warps per
+// SM, which wait for L1 and L2 at each of the 16 stencil rows.  What did not help:
+// the warp's nodes copied to shared memory as one box first (58.6 us: the waits
+// went, 8 M instructions came), 12 warps without spills or 20 with more (58 /
+// 71-80 us), all of the finalize's inputs staged or prefetched during the sums
+// (within 2 us either way).
+
+// copy 4 bytes to shared memory asynchronously, through L1
+__device__ __forceinline__ void async4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Two floats in one 64-bit register pair: sm_100a multiplies and adds both in one
+// instruction.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpk(f32x2 p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float sum2(f32x2 p) {
+    float a, b;
+    unpk(p, a, b);
+    return a + b;
+}
+// the record pair (dLdp, dLdm), (v, m) of a node: one 32-byte load
+__device__ __forceinline__ void load_pair(const node4<float>* p, f32x2 (&f)[4]) {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(f[0]), "=l"(f[1]), "=l"(f[2]), "=l"(f[3]) : "l"(p));
+}
+// Nodes of a particle's stencil by offset (i, j, k) from its base.  INSIDE: the
+// whole stencil lies in the grid; otherwise nodes outside it read as zero.
+template <bool INSIDE, int R> struct StencilNodes {
+    const node4<float>* g;  // the base node's first record (dereferenced inside the grid only)
+    int si, sj, b0, b1, b2, d0, d1, d2;
+    __device__ __forceinline__ StencilNodes(const node4<float>* grid, const GridGeom& geo, int goff, const int base[3])
+        : g(grid + (ptrdiff_t)R * ((base[0] * geo.dim[1] + base[1]) * geo.dim[2] + base[2] + goff)),
+          si(R * geo.dim[1] * geo.dim[2]), sj(R * geo.dim[2]), b0(base[0]), b1(base[1]), b2(base[2]), d0(geo.dim[0]),
+          d1(geo.dim[1]), d2(geo.dim[2]) {}
+    __device__ __forceinline__ const node4<float>* row(int i, int j) const { return g + (ptrdiff_t)(i * si + j * sj); }
+    __device__ __forceinline__ bool in(int i, int j, int k) const {
+        return INSIDE || ((unsigned)(b0 + i) < (unsigned)d0 && (unsigned)(b1 + j) < (unsigned)d1 &&
+                          (unsigned)(b2 + k) < (unsigned)d2);
+    }
+};
+__device__ __forceinline__ bool stencil_inside(const GridGeom& g, const int base[3]) {
+    bool in = true;
+#pragma unroll
+    for (int c = 0; c < 3; c++) in &= base[c] >= 0 && base[c] + 3 < g.dim[c];
+    return in;
+}
+
+// The gather's sums (the algebra of kernels.cuh:k_adj_gather): g = M (9, row-major), X, u, z.
+// The columns of G and of dLdC_next are read from the particle's staged inputs
+// (col: 18 values, 32 floats apart) where they are needed, so that
+// they hold no registers; k3 = 3/dx^2 scales the second.
+template <int SPLIT, class Nodes>
+__device__ __forceinline__ void gather_sums(const Nodes& f, const float t[3], float dx, float k3, float mp,
+                                            const float mvp[3], const float vn[3], const float* col, float2* w1s,
+                                            float (&g)[18]) {
+    auto G = [&](int r, int c) { return col[(r + 3 * c) * 32]; };
+    auto C = [&](int r, int c) { return col[(9 + r + 3 * c) * 32]; };
+    float n2[4], d2[4], s2[4];
+    axis_stencil(t[2], dx, n2, d2, s2);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float q1 = (float)j - t[1];
+        w1s[j * 32] = make_float2(bsp(q1), bsp_slope(q1));
+    }
+    // a node's packed fields: (o.x, o.y), (o.z, o.w), (v.x, v.y), (v.z, m); sigma is their product with
+    // (h.x, h.y), (h.z, m_p), (e.x, e.y), (e.z, 0)
+    const f32x2 K[4] = {pk(G(0, 2), G(1, 2)), pk(G(2, 2), 0.f), pk(k3 * C(0, 2), k3 * C(1, 2)), pk(k3 * C(2, 2), 0.f)};
+    f32x2 u[2] = {0, 0}, z[2] = {0, 0}, M[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+    float X[3] = {0.f, 0.f, 0.f};
+    const int i0 = SPLIT == 4 ? (int)(threadIdx.x & 3) : 0;
+#pragma unroll 1
+    for (int i = i0; i < (SPLIT == 4 ? i0 + 1 : 4); i++) {
+        const float q0 = (float)i - t[0], d0 = q0 * dx, n0 = bsp(q0), s0 = bsp_slope(q0), kd0 = k3 * d0;
+        const f32x2 h0[4] = {pk(mvp[0] + G(0, 0) * d0, mvp[1] + G(1, 0) * d0), pk(mvp[2] + G(2, 0) * d0, mp),
+                             pk(vn[0] + C(0, 0) * kd0, vn[1] + C(1, 0) * kd0), pk(vn[2] + C(2, 0) * kd0, 0.f)};
+#pragma unroll 2
+        for (int j = 0; j < 4; j++) {
+            const float2 ns1 = w1s[j * 32];
+            const float d1 = ((float)j - t[1]) * dx, n1 = ns1.x, s1 = ns1.y, kd1 = k3 * d1;
+            const node4<float>* row = f.row(i, j);
+            f32x2 nd[4][4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+#pragma unroll
+                for (int c = 0; c < 4; c++) nd[k][c] = 0;
+                if (f.in(i, j, k)) load_pair(row + 2 * k, nd[k]);
+            }
+            const f32x2 dd = pk(d1, d1), kd = pk(kd1, kd1);
+            const f32x2 h[4] = {fma2(pk(G(0, 1), G(1, 1)), dd, h0[0]), fma2(pk(G(2, 1), 0.f), dd, h0[1]),
+                                fma2(pk(C(0, 1), C(1, 1)), kd, h0[2]), fma2(pk(C(2, 1), 0.f), kd, h0[3])};
+            f32x2 S = 0, T = 0, R[4] = {0, 0, 0, 0}, D[2] = {0, 0};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const f32x2 d = pk(d2[k], d2[k]), n = pk(n2[k], n2[k]), s = pk(s2[k], s2[k]);
+                const f32x2 e = mul2(n, d);
+                f32x2 sig = mul2(nd[k][0], fma2(K[0], d, h[0]));
+#pragma unroll
+                for (int c = 1; c < 4; c++) sig = fma2(nd[k][c], fma2(K[c], d, h[c]), sig);
+                S = fma2(n, sig, S);
+                T = fma2(s, sig, T);
+#pragma unroll
+                for (int c = 0; c < 4; c++) R[c] = fma2(n, nd[k][c], R[c]);
+                D[0] = fma2(e, nd[k][0], D[0]);
+                D[1] = fma2(e, nd[k][1], D[1]);
+            }
+            const float w01 = n0 * n1, w0 = w01 * d0, w1 = w01 * d1, Sr = sum2(S), Tr = sum2(T);
+            const f32x2 w = pk(w01, w01), a0 = pk(w0, w0), a1 = pk(w1, w1);
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                u[c] = fma2(w, R[c], u[c]);
+                z[c] = fma2(w, R[2 + c], z[c]);
+                M[0][c] = fma2(a0, R[c], M[0][c]);
+                M[1][c] = fma2(a1, R[c], M[1][c]);
+                M[2][c] = fma2(w, D[c], M[2][c]);
+            }
+            X[0] += (s0 * n1) * Sr;
+            X[1] += (n0 * s1) * Sr;
+            X[2] += w01 * Tr;
+        }
+    }
+    float skip;
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        unpk(M[r][0], g[3 * r], g[3 * r + 1]);
+        unpk(M[r][1], g[3 * r + 2], skip);
+        g[9 + r] = X[r];
+    }
+    unpk(u[0], g[12], g[13]);
+    unpk(u[1], g[14], skip);
+    unpk(z[0], g[15], g[16]);
+    unpk(z[1], g[17], skip);
+    if (SPLIT == 4) reduce_slabs<18>(g);
+}
+
+// place of a staged slot in the thread's column: G (9), dLdC_next (9)
+constexpr int kStaged = 18;
+__host__ __device__ constexpr bool is_staged(int s) { return (s >= FS_AUX && s < FS_AUX + 9) || (s >= FS_CN && s < FS_CN + 9); }
+__host__ __device__ constexpr int staged_slot(int s) { return s < FS_CN ? s - FS_AUX : 9 + s - FS_CN; }
+// stage slots [lo, hi) of the finalize's inputs (fin_plane) of particle p
+template <int LO, int HI> __device__ __forceinline__ void stage_slots(const WArgs& a, int p, float* col) {
+#pragma unroll
+    for (int s = LO; s < HI; s++) {
+        size_t ld;
+        const float* src = fin_plane(a, s, ld);
+        async4(col + staged_slot(s) * 32, src + p);
+    }
+}
+
+// the finalize's inputs: the gather's sums in registers, G and dLdC_next staged, the rest in memory
+struct FinStaged {
+    const WArgs* a;
+    int p;
+    const float* g;
+    const float* col;
+    __device__ __forceinline__ float operator()(int slot) const {
+        if (slot < FS_F) return g[slot];
+        if (is_staged(slot)) return col[staged_slot(slot) * 32];
+        size_t ld;
+        return fin_plane(*a, slot, ld)[p];
+    }
+    __device__ __forceinline__ double acc(int i) const { return a->ctrl_acc[(size_t)i * a->np + p]; }
+};
+
+// resident blocks per SM the compiler budgets registers for (128 registers)
+#ifndef DMPM_CHUNK_GATHER_MINB
+#define DMPM_CHUNK_GATHER_MINB 4
+#endif
+template <bool EXACT, bool BATCH, int SPLIT>
+__global__ void __launch_bounds__(DMPM_CHUNK_THREADS, DMPM_CHUNK_GATHER_MINB) k_adj_gather_c(WArgs a) {
+    __shared__ float s_col[DMPM_CHUNK_THREADS * kStaged];
+    __shared__ float2 s_w1[DMPM_CHUNK_THREADS * 4];
+    __shared__ float s_dump[DMPM_CHUNK_THREADS];
+    const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) / SPLIT);
+    if ((q & ~(32 / SPLIT - 1)) >= a.n) return;  // the whole warp
+    float* col = s_col + (threadIdx.x >> 5) * 32 * kStaged + (threadIdx.x & 31);
+    float2* w1s = s_w1 + (threadIdx.x >> 5) * 128 + (threadIdx.x & 31);
+    const size_t np = a.np, npl = a.npl;
+    const int p = (int)a.items.order[min(q, a.n - 1)];
+    const int inst = BATCH ? (int)a.pinst[p] : 0;
+    const GridGeom& geo = chunk_geo<BATCH>(a, inst);
+    const int goff = BATCH ? a.ig[inst].goff : 0;
+    stage_slots<FS_AUX, FS_AUX + 9>(a, p, col);
+    stage_slots<FS_CN, FS_CN + 9>(a, p, col);
+    float t[3];
+    int base[3];
+    load_x_base(a.st, npl, p, geo, t, base, a.xlo);
+    {  // the stencils of the warp's first and last particle into L1 (s_dump is not read): 102 -> 98 us
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int src = h ? 31 : 0;
+            int o[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) o[c] = __shfl_sync(0xffffffffu, base[c], src);
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                const int gi = o[0] + 2 * m + (lane >> 4), gj = o[1] + ((lane >> 2) & 3), gk = o[2] + (lane & 3);
+                if (in_grid(geo, gi, gj, gk))
+                    async4(s_dump + threadIdx.x, &a.gadj2[2 * (node_id(geo, gi, gj, gk) + goff)].x);
+            }
+        }
+    }
+    async_commit();
+    const float dx = (float)a.geo.dx, k3 = 3.f / (dx * dx);
+    const float mp = a.cst[(size_t)KM * np + p], cd = EXACT ? (1.f - a.dt * a.drag) : 1.f;
+    float mvp[3], vn[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        mvp[c] = mp * a.st[(size_t)(PV + c) * npl + p] * cd;
+        vn[c] = a.adjn[(size_t)c * np + p];
+    }
+    async_wait<0>();
+    float g[18];
+    if (__all_sync(0xffffffffu, stencil_inside(geo, base)))
+        gather_sums<SPLIT>(StencilNodes<true, 2>(a.gadj2, geo, goff, base), t, dx, k3, mp, mvp, vn, col, w1s, g);
+    else
+        gather_sums<SPLIT>(StencilNodes<false, 2>(a.gadj2, geo, goff, base), t, dx, k3, mp, mvp, vn, col, w1s, g);
+    if (q < a.n && (SPLIT == 1 || (threadIdx.x & 3) == 0))
+        finalize_particle<EXACT>(a, p, FinStaged{&a, p, g, col});
+}
+
+// threads per block of the one-thread-per-particle kernels: the most that leave
+// two blocks for each of 148 SMs
+inline int particle_threads(int n) {
+    const int blocks = 148 * 2;
+    return n >= 128 * blocks ? 128 : n >= 64 * blocks ? 64 : 32;
+}
+// Four threads per particle below 40k particles (8.7k: 14.7 against 18-21 us per
+// step), one above (79k: 33 against 57 us)
+template <bool BATCH> inline void launch_gather(const WArgs& a, bool exact, cudaStream_t st) {
+    const int split = a.n < 40000 ? 4 : 1, t = particle_threads(split * a.n);
+    const unsigned b = (unsigned)((split * a.n + t - 1) / t);
+    if (split == 4 && exact) k_adj_gather_c<true, BATCH, 4><<<b, t, 0, st>>>(a);
+    else if (split == 4) k_adj_gather_c<false, BATCH, 4><<<b, t, 0, st>>>(a);
+    else if (exact) k_adj_gather_c<true, BATCH, 1><<<b, t, 0, st>>>(a);
+    else k_adj_gather_c<false, BATCH, 1><<<b, t, 0, st>>>(a);
 }
 
 }  // namespace dmpm

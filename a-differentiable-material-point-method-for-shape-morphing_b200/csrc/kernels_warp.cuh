@@ -163,7 +163,8 @@ __device__ __forceinline__ float bsp(float q) {
 __device__ __forceinline__ float bsp_slope(float q) {
     const float a = fabsf(q);
     const float inner = (1.5f * a - 2.f) * q;
-    const float outer = (-0.5f * a + 2.f - 2.f / a) * q;
+    const float t = 2.f - a;
+    const float outer = copysignf(0.5f * t * t, -q);  // (-a/2 + 2 - 2/a) q without the division
     return a < 1.f ? inner : (a < 2.f ? outer : 0.f);
 }
 
@@ -279,13 +280,8 @@ __device__ __forceinline__ float advance_x(const float* st, float* st_next, size
 
 // ------------------------------------------------------------------ args
 // Minimum resident blocks per SM (the register cap the compiler works to) for
-// the per-particle FP64 kernels: k_stress at 256 threads per block (2: 128
-// registers, no spills; 1 lets it take 132 and run one block per SM),
-// k_adj_finalize at 128 (4: 128 registers with a 40-byte spill, 11 % faster
-// than the 168-register build on the 64^3, 267k-particle workload), and its
-// FP64 part alone (5: 96 registers with a 144-byte spill, 40.6 against 45.2 us
-// at 4 and 44.4 us at 6 on the same workload: the extra warps hide more of the
-// load latency than the spills cost).
+// k_stress at 256 threads per block (2: 128 registers, no spills; 1 lets it take
+// 132 and run one block per SM)
 // k_stress takes the FP64 polar factors from the scaled Newton iteration
 // (polar_newton) where det(F + dFc) > 0 and from the SVD (polar3) otherwise;
 // 0 uses the SVD everywhere
@@ -295,21 +291,8 @@ __device__ __forceinline__ float advance_x(const float* st, float* st_next, size
 #ifndef DMPM_STRESS_MIN_BLOCKS
 #define DMPM_STRESS_MIN_BLOCKS 2
 #endif
-#ifndef DMPM_FINALIZE_MIN_BLOCKS
-#define DMPM_FINALIZE_MIN_BLOCKS 4
-#endif
-#ifndef DMPM_FINALIZE_STRESS_MIN_BLOCKS
-#define DMPM_FINALIZE_STRESS_MIN_BLOCKS 5
-#endif
-// and for the warp-item kernels: the adjoint gather and P2G in blocks of
-// DMPM_GATHER_THREADS / DMPM_P2G_THREADS (256), the adjoint scatter below in
-// blocks of DMPM_ADJ_SCATTER_THREADS (128)
-#ifndef DMPM_GATHER_MIN_BLOCKS
-#define DMPM_GATHER_MIN_BLOCKS 3
-#endif
-#ifndef DMPM_GATHER_THREADS
-#define DMPM_GATHER_THREADS 256
-#endif
+// and for the warp-item kernels: P2G in blocks of DMPM_P2G_THREADS (256), the
+// adjoint scatter below in blocks of DMPM_ADJ_SCATTER_THREADS (128)
 #ifndef DMPM_SCATTER_MIN_BLOCKS
 #define DMPM_SCATTER_MIN_BLOCKS 3
 #endif
@@ -317,9 +300,6 @@ __device__ __forceinline__ float advance_x(const float* st, float* st_next, size
 #define DMPM_P2G_THREADS 256
 #endif
 // CTAs per SM of the persistent grids (no more than the register budget above lets reside)
-#ifndef DMPM_GATHER_CTAS
-#define DMPM_GATHER_CTAS DMPM_GATHER_MIN_BLOCKS
-#endif
 #ifndef DMPM_SCATTER_CTAS
 #define DMPM_SCATTER_CTAS DMPM_SCATTER_MIN_BLOCKS
 #endif
@@ -327,7 +307,7 @@ __device__ __forceinline__ float advance_x(const float* st, float* st_next, size
 // registers, 28-byte spill, 28 warps) take 53.3 us on the 64^3, 267k-particle
 // workload, against 55.4 us for 4 blocks of 256 (64 registers, 68-byte
 // spill), 59.4 us for 3 of 256 and 55.7 us for 5 of 128 (95 registers, no
-// spill); P2G is faster at 3 blocks of 256 (the gather at 4: 87.0 against 78.9 us)
+// spill); P2G is faster at 3 blocks of 256 
 #ifndef DMPM_ADJ_SCATTER_MIN_BLOCKS
 #define DMPM_ADJ_SCATTER_MIN_BLOCKS 7
 #endif
@@ -375,7 +355,6 @@ struct WArgs {
     const float* adj_next;
     float* adj;
     float* adjn;           // [12][np]: dLdv_next (3), dLdC_next (9)
-    float* gath;           // [18][np]: M (9), X (3), u (3), z (3)
     node4<float>* gadj;    // (dLdv.xyz, 0)
     node4<float>* gadj2;   // per node two records: (dLdp.xyz, dLdm), (v.xyz, m)
     float* ctrl_grad;      // per-layer dL/d dFc [9][np] or null
@@ -941,144 +920,6 @@ __global__ void k_adj_gop_w(const node4<float>* __restrict__ grid, const node4<f
     gadj2[2 * g + 1] = nd;
 }
 
-// adjoint P2G gather: per particle, over its 64 nodes,
-//   M += w d dLdp^T,  X += sigma (N'NN, NN'N, NNN'),  u += w dLdp,  z += w v_g
-//   sigma = m dLdm + dLdp.(m v c_d + G d) + v_g.(dLdv_next + 3/dx^2 dLdC_next d)
-// (the algebra of kernels.cuh:k_adj_gather); written to gath for k_adj_finalize.
-// One warp item of the adjoint gather: the item's particles (lane L, stencil
-// coordinates t, base) read their 64 stencil node pairs from sw, the item's
-// staged copy, or from global memory when sw is null.
-template <bool EXACT>
-__device__ __forceinline__ void gather_item(const WArgs& a, const GridGeom& geo, int goff, const ItemLane& L,
-                                            const float t[3], const int base[3], const node4<float>* sw) {
-    const size_t np = a.np, npl = a.npl;
-    const int p = L.p;
-    LaneW w;
-    float own1[3];
-    lane_weights_k(t, geo, L.s, w, own1, true);
-    const float mp = a.cst[(size_t)KM * np + p];
-    const float cd = EXACT ? (1.f - a.dt * a.drag) : 1.f;
-    const float dx = (float)geo.dx;
-    const float k3 = 3.f / (dx * dx);
-    float mvp[3], vn[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        mvp[c] = mp * a.st[(size_t)(PV + c) * npl + p] * cd;
-        vn[c] = a.adjn[(size_t)c * np + p];
-    }
-    const m3<float> G = load_m3(a.G, npl, p);
-    const m3<float> Cn = load_m3(a.adjn + 3 * np, np, p);
-    // sigma's node-dependent pieces: h_g = mvp + G d,  e_g = vn + k3 Cn d
-    float h0[3], e0[3];
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-        h0[r] = mvp[r] + G.a[r][0] * w.d0;
-        e0[r] = vn[r] + k3 * Cn.a[r][0] * w.d0;
-    }
-    float acc[18];  // M (9, row-major: M[r][c] = sum w d_r dLdp_c), X (3), u (3), z (3)
-#pragma unroll
-    for (int i = 0; i < 18; i++) acc[i] = 0.f;
-    // Factored sums: on this lane d0, n0 and s0 are constant and on a row d1, n1, s1, so
-    //   M[0][c] = d0 u_c (formed after the loop),
-    //   X0 = s0 sum_j n1 S_j,  X1 = n0 sum_j s1 S_j,  X2 = n0 sum_j n1 T_j,
-    // with the row sums S_j = sum_k n2_k sigma, T_j = sum_k s2_k sigma.
-    float S = 0.f, T = 0.f;
-    // one node (j, k) of the lane's slab, with row j's axis-1 values d1, n1
-    auto node = [&](const node4<float>& o, const node4<float>& vg, float d1, float n1, int k) {
-        float h[3], e[3];
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            h[r] = h0[r] + G.a[r][1] * d1 + G.a[r][2] * w.d2[k];
-            e[r] = e0[r] + k3 * Cn.a[r][1] * d1 + k3 * Cn.a[r][2] * w.d2[k];
-        }
-        const float wt = (w.n0 * n1) * w.n2[k];
-        const float sig = mp * o.w + o.x * h[0] + o.y * h[1] + o.z * h[2] + vg.x * e[0] + vg.y * e[1] + vg.z * e[2];
-        S += w.n2[k] * sig;
-        T += w.s2[k] * sig;
-        const float wo[3] = {wt * o.x, wt * o.y, wt * o.z};
-        acc[15] += wt * vg.x;
-        acc[16] += wt * vg.y;
-        acc[17] += wt * vg.z;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            acc[12 + c] += wo[c];
-            acc[3 + c] += d1 * wo[c];
-            acc[6 + c] += w.d2[k] * wo[c];
-        }
-    };
-    auto end_row = [&](float n1, float s1) {
-        acc[9] += n1 * S;
-        acc[10] += s1 * S;
-        acc[11] += n1 * T;
-        S = 0.f;
-        T = 0.f;
-    };
-    if (sw) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            float d1, n1, s1;
-            row_weights(own1, j, d1, n1, s1);
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int n = 16 * L.s + 4 * j + k;
-                node(sw[stage_index<2>(n, 0)], sw[stage_index<2>(n, 1)], d1, n1, k);
-            }
-            end_row(n1, s1);
-        }
-    } else {
-        LaneNodes N = lane_nodes(geo, base, L.s);
-        N.g00 += goff;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            float d1, n1, s1;
-            row_weights(own1, j, d1, n1, s1);
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                if (!((N.mask >> (4 * j + k)) & 1u)) continue;
-                const int g = N.g00 + j * N.sj + k;
-                node(a.gadj2[2 * g], a.gadj2[2 * g + 1], d1, n1, k);
-            }
-            end_row(n1, s1);
-        }
-    }
-    acc[9] *= w.s0;
-    acc[10] *= w.n0;
-    acc[11] *= w.n0;
-#pragma unroll
-    for (int c = 0; c < 3; c++) acc[c] = w.d0 * acc[12 + c];
-    reduce_slabs<18>(acc);
-    if (!L.valid) return;
-    if (L.s == 0) {
-#pragma unroll
-        for (int i = 0; i < 9; i++) a.gath[(size_t)i * np + p] = acc[i];
-    } else if (L.s == 1) {
-#pragma unroll
-        for (int i = 9; i < 18; i++) a.gath[(size_t)i * np + p] = acc[i];
-    }
-}
-
-template <bool EXACT, int MODE>
-__global__ void __launch_bounds__(DMPM_GATHER_THREADS, DMPM_GATHER_MIN_BLOCKS) k_adj_gather_w(WArgs a) {
-    const int nit = item_count(a);
-    const size_t npl = a.npl;
-    __shared__ node4<float> s_rec[8][StageRecords<2>::value];
-    for (int item = first_warp(); item < nit; item = next_item<MODE>(item, nit)) {
-        GridGeom geo;
-        int goff;
-        item_grid<MODE>(a, item, geo, goff);
-        const ItemLane L = item_lane(a.items, item);
-        float t[3];
-        int base[3];
-        load_x_base(a.st, npl, L.p, geo, t, base, a.xlo);
-        node4<float>* sw = nullptr;
-        if (DMPM_STAGE_NODES && warp_uniform_base(base)) {
-            sw = s_rec[threadIdx.x >> 5];
-            stage_stencil<2>(a.gadj2, geo, goff, base, sw);
-        }
-        gather_item<EXACT>(a, geo, goff, L, t, base, sw);
-    }
-}
-
 // ------------------------------------------------------------------ finalize
 // per particle: P, polar factors and dP/dF in FP64, then the adjoint of layer n
 //   dLdP = -3/dx^2 dt vol M^T Fe,  dLdF(stress) = -3/dx^2 dt vol M P,  dLdC = m M^T
@@ -1101,9 +942,8 @@ enum : int {
     FS_COUNT = 94
 };
 
-// first element and stride of a slot's plane
+// first element and stride of a slot's plane (the sums of FS_GATH have none)
 __device__ __forceinline__ const float* fin_plane(const WArgs& a, int slot, size_t& stride) {
-    if (slot < FS_F) { stride = a.np; return a.gath + (size_t)slot * a.np; }
     if (slot < FS_DFC) { stride = a.npl; return a.st + (size_t)(PF + slot - FS_F) * a.npl; }
     if (slot < FS_AUX) { stride = a.np; return a.dfc + (size_t)(slot - FS_DFC) * a.np; }
     if (slot < FS_CST) { stride = a.npl; return a.G + (size_t)(slot - FS_AUX) * a.npl; }
@@ -1115,23 +955,7 @@ __device__ __forceinline__ const float* fin_plane(const WArgs& a, int slot, size
     return a.st_next + (size_t)(PC + slot - FS_CNEXT) * a.npn;
 }
 
-// the finalize inputs of particle p, read from global memory
-struct FinGlobal {
-    const WArgs* a;
-    int p;
-    __device__ __forceinline__ float operator()(int slot) const {
-        size_t st;
-        return fin_plane(*a, slot, st)[p];
-    }
-    __device__ __forceinline__ double acc(int i) const { return a->ctrl_acc[(size_t)i * a->np + p]; }
-};
-// PART selects what one launch computes: 0 everything; FIN_STRESS the FP64 part
-// (P, dP/dF:dLdP, dLdF, the control gradient); FIN_TRANSPORT the FP32 outputs
-// dLdx, dLdv, dLdC, which need neither the polar factors nor dLdF.
-enum : int { FIN_ALL = 0, FIN_STRESS = 1, FIN_TRANSPORT = 2 };
-template <bool EXACT, class In, int PART = FIN_ALL>
-__device__ __forceinline__ void finalize_particle(const WArgs& a, int p, const In& in) {
-    constexpr bool kStress = PART != FIN_TRANSPORT, kTransport = PART != FIN_STRESS;
+template <bool EXACT, class In> __device__ __forceinline__ void finalize_particle(const WArgs& a, int p, const In& in) {
     const size_t np = a.np, npl = a.npl;
     auto mat = [&](int slot) {  // 9 column-major planes -> m3
         m3<float> m;
@@ -1173,10 +997,6 @@ __device__ __forceinline__ void finalize_particle(const WArgs& a, int p, const I
         store_m3(a.adj + (size_t)PC * npl, npl, p, mp * transpose(M));
         return ax0;
     };
-    if constexpr (!kStress) {
-        if (!isfinite(transport())) atomicOr(a.status, ST_NONFINITE_ADJ);
-        return;
-    }
     const m3<float> H = mat(FS_F), dfc = mat(FS_DFC);
     const m3<float> Fe = fe_from_strain(H, dfc);
     const m3<double> Fed = fe_from_strain_d(H, dfc);
@@ -1195,8 +1015,7 @@ __device__ __forceinline__ void finalize_particle(const WArgs& a, int p, const I
     const float kk = -k3 * a.dt * vol;
     const m3<float> dLdP = kk * mtm(M, Fe);
     const m3<float> dFstress = kk * (M * P);
-    float ax0 = 0.f;
-    if constexpr (kTransport) ax0 = transport();
+    const float ax0 = transport();
     const m3<float> Cnext = mat(FS_CNEXT);
     const m3<float> dFn = mat(FS_AF);
     const m3<float> Tr = mtm(m3_eye<float>() + a.dt * Cnext, dFn);
@@ -1220,59 +1039,6 @@ __device__ __forceinline__ void finalize_particle(const WArgs& a, int p, const I
     }
     if (a.dbg_dLdP) store_m3(a.dbg_dLdP, np, p, dLdP);
     if (!isfinite(dLdF.a[0][0] + dLdF.a[1][1] + dLdF.a[2][2] + ax0)) atomicOr(a.status, ST_NONFINITE_ADJ);
-}
-
-// one thread per particle, inputs read from global memory (the REFCOMPAT
-// variant, with its finite-difference dJFit, keeps the compiler's own
-// register budget)
-template <bool EXACT, int PART = FIN_ALL>
-__global__ void __launch_bounds__(128, !EXACT ? 1 : PART == FIN_STRESS ? DMPM_FINALIZE_STRESS_MIN_BLOCKS
-                                                                         : DMPM_FINALIZE_MIN_BLOCKS)
-    k_adj_finalize(WArgs a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < a.n) finalize_particle<EXACT, FinGlobal, PART>(a, p, FinGlobal{&a, p});
-}
-// the transport part alone: few registers, many resident warps
-static __global__ void __launch_bounds__(256) k_adj_finalize_transport(WArgs a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < a.n) finalize_particle<true, FinGlobal, FIN_TRANSPORT>(a, p, FinGlobal{&a, p});
-}
-
-// host side: one thread per particle (a variant that first staged each
-// block's 94 input planes in shared memory with cp.async.bulk copies measured
-// 7 % slower on the 64^3, 267k-particle workload -- 57 KB of shared memory
-// per 128 particles cut residency to 12 warps per SM, and the kernel is bound
-// by its dependent FP64 chains, not by load latency -- so it was dropped)
-inline void launch_finalize(const WArgs& a, bool exact, cudaStream_t st) {
-    if (a.n <= 0) return;
-    const unsigned b = (unsigned)((a.n + 127) / 128);
-    if (exact) k_adj_finalize<true><<<b, 128, 0, st>>>(a);
-    else k_adj_finalize<false><<<b, 128, 0, st>>>(a);
-}
-// The single-scene engine runs the finalize as the two launches below, the
-// transport part on a second stream beside the FP64 part: the FP64 part keeps
-// 128 registers per thread and 16 warps per SM, and the transport part's warps
-// (60 registers) fill the rest of the SMs meanwhile (60.0 against 60.9 ms per
-// gradient evaluation on the 64^3, 267k-particle workload).  0 runs the
-// single kernel.
-#ifndef DMPM_SPLIT_FINALIZE
-#define DMPM_SPLIT_FINALIZE 1
-#endif
-// one part of the finalize (FIN_STRESS or FIN_TRANSPORT) on st
-inline void launch_finalize_part(const WArgs& a, bool exact, int part, cudaStream_t st) {
-    if (a.n <= 0) return;
-    if (part == FIN_TRANSPORT) {
-        k_adj_finalize_transport<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a);
-        return;
-    }
-    const unsigned b = (unsigned)((a.n + 127) / 128);
-    if (exact) k_adj_finalize<true, FIN_STRESS><<<b, 128, 0, st>>>(a);
-    else k_adj_finalize<false, FIN_STRESS><<<b, 128, 0, st>>>(a);
-}
-// the same work as two launches: the FP64 part on st, the transport part on side
-inline void launch_finalize_split(const WArgs& a, bool exact, cudaStream_t st, cudaStream_t side) {
-    launch_finalize_part(a, exact, FIN_TRANSPORT, side);
-    launch_finalize_part(a, exact, FIN_STRESS, st);
 }
 
 }  // namespace dmpm
