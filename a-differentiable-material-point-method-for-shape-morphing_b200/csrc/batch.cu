@@ -508,24 +508,26 @@ struct dmpm_batch::Impl {
         a.status = status;
         return a;
     }
-    unsigned warp_blocks(int t) const {
-        const size_t most = (P[t + 1] * 32 + 255) / 256;  // one item per particle at most
-        return (unsigned)std::max<size_t>(1, std::min<size_t>(most, (size_t)sms * ctas_per_sm()));
-    }
     void step(int t) {
         WArgs a = args(t);
         const size_t Gt = node_prefix[A[t + 1]];
         const int pb = particle_block();
-        const unsigned wb = warp_blocks(t);
         DMPM_CK(cudaMemsetAsync(grid[t], 0, Gt * sizeof(node4<float>), b->stream));
-        k_stress<false><<<(unsigned)((a.n + pb - 1) / pb), pb, 0, b->stream>>>(a);
-        launched();
+        if (t == 0) {  // later steps: formed by the G2P of the step before
+            k_stress<false><<<(unsigned)((a.n + pb - 1) / pb), pb, 0, b->stream>>>(a);
+            launched();
+        }
         k_p2g_c<true, false><<<chunk_blocks(a.n, a.chunk), DMPM_CHUNK_THREADS, 0, b->stream>>>(a);
         launched();
         k_gop_inplace<<<(unsigned)((Gt + 255) / 256), 256, 0, b->stream>>>(grid[t], Gt, a.dt, a.fext[0], a.fext[1],
                                                                              a.fext[2]);
         launched();
-        k_g2p_w<ITEMS_BATCH><<<wb, 256, 0, b->stream>>>(a);
+        if (t + 1 < smax) {
+            a.G_next = aux[t + 1];
+            a.dfc_next = dfc;
+            a.n_next = (int)P[t + 2];
+        }
+        launch_g2p<true>(a, b->stream);
         launched();
     }
 
@@ -567,7 +569,6 @@ struct dmpm_batch::Impl {
         a.gadj2 = gadj2;
         a.ctrl_acc = ctrl_acc;
         const size_t Gt = node_prefix[A[t + 1]];
-        const unsigned wb = warp_blocks(t);
         const bool ex = prm.adjoint_mode == DMPM_ADJ_EXACT;
         DMPM_CK(cudaMemsetAsync(gadj, 0, Gt * sizeof(node4<float>), b->stream));
         const unsigned cb = chunk_blocks(a.n, a.chunk);

@@ -1060,7 +1060,7 @@ template <class T> class Engine : public EngineBase {
     // One ForwardTimeStep: layer l -> out (state of l+1), grid g, G of layer l
     // in Gd.  FP32 path: g_ready = Gd already holds layer l's G (the previous
     // step's G2P formed it), so the stress stage is skipped; Gd_next non-null =
-    // the brick G2P also forms layer l+1's G there.  Returns whether it did.
+    // the G2P also forms layer l+1's G there.  Returns whether it did.
     bool step(int l, const T* st, T* out, node4<T>* g, T* Gd, bool allow_sort, bool g_ready = false,
               T* Gd_next = nullptr) {
         if constexpr (kWarp) {
@@ -1117,18 +1117,15 @@ template <class T> class Engine : public EngineBase {
             pend();
             // the deterministic mode keeps the standalone stress stage: it also raises the
             // next P2G's bounds, which that step clears first
-            const bool fuse = Gd_next && !dm && (ush == 3 || ush == 6);
+            const bool fuse = Gd_next && !dm;
             if (fuse) {
                 a.dfc_next = (const float*)layers_[l + 1].dfc;
                 a.G_next = (float*)Gd_next;
                 a.P_next = ctx_->prm.keep_intermediates ? (float*)layers_[l + 1].dbgP : nullptr;
+                a.n_next = n_;
             }
             pbeg(K_G2P);
-            if (ush == 3 && fuse) k_g2p_b<2, true><<<brick_blocks(k_g2p_b<2, true>), bt, 0, ctx_->stream>>>(a);
-            else if (ush == 6 && fuse) k_g2p_b<4, true><<<brick_blocks(k_g2p_b<4, true>), bt, 0, ctx_->stream>>>(a);
-            else if (ush == 3) k_g2p_b<2><<<brick_blocks(k_g2p_b<2>), bt, 0, ctx_->stream>>>(a);
-            else if (ush == 6) k_g2p_b<4><<<brick_blocks(k_g2p_b<4>), bt, 0, ctx_->stream>>>(a);
-            else k_g2p_w<ITEMS_PERSISTENT><<<warp_blocks(DMPM_G2P_CTAS), 256, 0, ctx_->stream>>>(a);
+            launch_g2p<false>(a, ctx_->stream);
             launched();
             pend();
             return fuse;

@@ -30,7 +30,7 @@
 // lane) read 21 words per particle.  Groups of strays cost: without the
 // grouping (a group per run of the sorted order) 32.8 and 42.6 us.
 #pragma once
-#include "kernels_brick.cuh"
+#include "kernels_warp.cuh"
 
 namespace dmpm {
 
@@ -275,6 +275,19 @@ inline unsigned chunk_blocks(int n, int chunk) {
     return (unsigned)((n + per - 1) / per);
 }
 
+// Per-axis stencil offsets d = x_g - x, weights N(d / dx) and slopes of the
+// four nodes k = 0..3 of the stencil, from the lattice coordinate t of the
+// particle (load_x_base): d = (k - t) dx.
+__device__ __forceinline__ void axis_stencil(float t, float dx, float n[4], float d[4], float* s) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float q = (float)k - t;
+        d[k] = q * dx;
+        n[k] = bsp(q);
+        if (s) s[k] = bsp_slope(q);
+    }
+}
+
 // ------------------------------------------------------------------ adjoint gather + finalize
 // One thread per particle of the sorted order, reading the nodes where they lie:
 // the particles of a warp share one to three cells, so their reads are
@@ -350,6 +363,163 @@ __device__ __forceinline__ bool stencil_inside(const GridGeom& g, const int base
 #pragma unroll
     for (int c = 0; c < 3; c++) in &= base[c] >= 0 && base[c] + 3 < g.dim[c];
     return in;
+}
+
+// a node's (v.x, v.y), (v.z, m): one 16-byte load
+__device__ __forceinline__ void load_node(const node4<float>* p, f32x2 (&f)[2]) {
+    asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(f[0]), "=l"(f[1]) : "l"(p));
+}
+// Start reading the stencils of the warp's first and last particle into L1, R
+// records of 16 bytes per node: copies to a word that nobody reads.
+template <int R>
+__device__ __forceinline__ void warm_stencils(const node4<float>* nodes, const GridGeom& g, int goff, const int base[3],
+                                              float* dump) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        int o[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) o[c] = __shfl_sync(0xffffffffu, base[c], h ? 31 : 0);
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const int gi = o[0] + 2 * m + (lane >> 4), gj = o[1] + ((lane >> 2) & 3), gk = o[2] + (lane & 3);
+            if (in_grid(g, gi, gj, gk)) async4(dump, &nodes[R * (node_id(g, gi, gj, gk) + goff)].x);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ G2P + P_op_2 (+ next stress stage)
+// v' = sum w v_g;  C' = 3/dx^2 sum w v_g d^T, factored per row and slab (s: V, then
+// the columns of C' / (3/dx^2), each (x, y), (z, unused)).
+template <int SPLIT, class Nodes>
+__device__ __forceinline__ void g2p_sums(const Nodes& f, const float t[3], float dx, f32x2 (&s)[8]) {
+    float n1[4], d1[4], n2[4], d2[4];
+    axis_stencil(t[1], dx, n1, d1, nullptr);
+    axis_stencil(t[2], dx, n2, d2, nullptr);
+#pragma unroll
+    for (int c = 0; c < 8; c++) s[c] = 0;
+    const int i0 = SPLIT == 4 ? (int)(threadIdx.x & 3) : 0;
+#pragma unroll 1
+    for (int i = i0; i < (SPLIT == 4 ? i0 + 1 : 4); i++) {
+        const float q0 = (float)i - t[0], n0 = bsp(q0), e0 = n0 * (q0 * dx);
+        f32x2 V[2] = {0, 0}, C1[2] = {0, 0}, C2[2] = {0, 0};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const node4<float>* row = f.row(i, j);
+            f32x2 nd[4][2];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                nd[k][0] = nd[k][1] = 0;
+                if (f.in(i, j, k)) load_node(row + k, nd[k]);
+            }
+            f32x2 Vj[2] = {0, 0}, Wj[2] = {0, 0};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float e = n2[k] * d2[k];
+                const f32x2 nn = pk(n2[k], n2[k]), ee = pk(e, e);
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    Vj[c] = fma2(nn, nd[k][c], Vj[c]);
+                    Wj[c] = fma2(ee, nd[k][c], Wj[c]);
+                }
+            }
+            const float e1 = n1[j] * d1[j];
+            const f32x2 nn = pk(n1[j], n1[j]), ee = pk(e1, e1);
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                V[c] = fma2(nn, Vj[c], V[c]);
+                C1[c] = fma2(ee, Vj[c], C1[c]);
+                C2[c] = fma2(nn, Wj[c], C2[c]);
+            }
+        }
+        const f32x2 nn = pk(n0, n0), ee = pk(e0, e0);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            s[c] = fma2(nn, V[c], s[c]);
+            s[2 + c] = fma2(ee, V[c], s[2 + c]);
+            s[4 + c] = fma2(nn, C1[c], s[4 + c]);
+            s[6 + c] = fma2(nn, C2[c], s[6 + c]);
+        }
+    }
+}
+
+// One thread per particle of the sorted order (four below 40k particles), as the
+// adjoint gather.  Per step, with the next stress stage (event times; before: a
+// CTA per brick octant that staged its node tile behind two barriers, 2.1 waves of
+// them): 267k particles 49 against 64 us, 301k at 8 per cell 47 against 87, 2.0M
+// 280 against 490, 8.7k 12.7 against 14; 3 or 5 blocks per SM 51 / 52 us on the
+// first.  F' = (1 - s)(I + dt C')(F + dFc) + s F;  x' = x + dt v'.
+// STRESS: also the next step's stress stage from the strain and C just formed
+// (stress_particle, the arithmetic of k_stress), into a.G_next, for the first
+// a.n_next particles -- one pass over the particles fewer per step.
+#ifndef DMPM_CHUNK_G2P_MINB
+#define DMPM_CHUNK_G2P_MINB 4
+#endif
+template <bool BATCH, bool STRESS, int SPLIT>
+__global__ void __launch_bounds__(DMPM_CHUNK_THREADS, STRESS ? DMPM_CHUNK_G2P_MINB : 6) k_g2p_c(WArgs a) {
+    __shared__ float s_dump[DMPM_CHUNK_THREADS];
+    const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) / SPLIT);
+    if ((q & ~(32 / SPLIT - 1)) >= a.n) return;  // the whole warp
+    const size_t np = a.np, npl = a.npl, npn = a.npn;
+    const int p = (int)a.items.order[min(q, a.n - 1)];
+    const int inst = BATCH ? (int)a.pinst[p] : 0;
+    const GridGeom& geo = chunk_geo<BATCH>(a, inst);
+    const int goff = BATCH ? a.ig[inst].goff : 0;
+    float t[3];
+    int base[3];
+    double xd[3];
+    load_x_base(a.st, npl, p, geo, t, base, a.xlo, xd);
+    warm_stencils<1>(a.grid, geo, goff, base, s_dump + threadIdx.x);
+    async_commit();
+    const m3<float> H = load_m3(a.st + (size_t)PF * npl, npl, p);
+    const m3<float> D = H + load_m3(a.dfc, np, p);
+    const float dx = (float)a.geo.dx, k3 = 3.f / (dx * dx);
+    float s[12];
+    {
+        f32x2 s2[8];
+        if (__all_sync(0xffffffffu, stencil_inside(geo, base)))
+            g2p_sums<SPLIT>(StencilNodes<true, 1>(a.grid, geo, goff, base), t, dx, s2);
+        else
+            g2p_sums<SPLIT>(StencilNodes<false, 1>(a.grid, geo, goff, base), t, dx, s2);
+        float skip;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            unpk(s2[2 * c], s[3 * c], s[3 * c + 1]);
+            unpk(s2[2 * c + 1], s[3 * c + 2], skip);
+        }
+    }
+    if (SPLIT == 4) reduce_slabs<12>(s);
+    async_wait<0>();
+    if (q >= a.n || (SPLIT == 4 && (threadIdx.x & 3) != 0)) return;
+    m3<float> Cn;
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) Cn.a[r][c] = k3 * s[3 + 3 * c + r];
+    bool finite = true;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const float xn = store_x(a.st_next, npn, p, c, xd[c], a.dt, s[c], a.xlo);
+        a.st_next[(size_t)(PV + c) * npn + p] = s[c];
+        finite &= isfinite(xn);
+    }
+    store_m3(a.st_next + (size_t)PC * npn, npn, p, Cn);
+    // strain update H' = (1 - s)(D + dt C' (I + D)) + s H,  D = H + dFc
+    m3<float> Hn;
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            const float u = D.a[r][c] + a.dt * (Cn.a[r][c] + (Cn.a[r][0] * D.a[0][c] + Cn.a[r][1] * D.a[1][c] +
+                                                               Cn.a[r][2] * D.a[2][c]));
+            const float hn = (1.f - a.s) * u + a.s * H.a[r][c];
+            a.st_next[(size_t)(PF + r + 3 * c) * npn + p] = hn;
+            Hn.a[r][c] = hn;
+            finite &= isfinite(hn);
+        }
+    if (!finite) atomicOr(a.status, ST_NONFINITE_FWD);
+    if (STRESS && p < a.n_next)
+        stress_particle(a, p, Hn, load_m3(a.dfc_next, np, p), [&]() { return Cn; }, a.G_next, npn, a.P_next);
 }
 
 // The gather's sums (the algebra of kernels.cuh:k_adj_gather): g = M (9, row-major), X, u, z.
@@ -491,22 +661,7 @@ __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, DMPM_CHUNK_GATHER_MINB) k_
     float t[3];
     int base[3];
     load_x_base(a.st, npl, p, geo, t, base, a.xlo);
-    {  // the stencils of the warp's first and last particle into L1 (s_dump is not read): 102 -> 98 us
-        const int lane = threadIdx.x & 31;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int src = h ? 31 : 0;
-            int o[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) o[c] = __shfl_sync(0xffffffffu, base[c], src);
-#pragma unroll
-            for (int m = 0; m < 2; m++) {
-                const int gi = o[0] + 2 * m + (lane >> 4), gj = o[1] + ((lane >> 2) & 3), gk = o[2] + (lane & 3);
-                if (in_grid(geo, gi, gj, gk))
-                    async4(s_dump + threadIdx.x, &a.gadj2[2 * (node_id(geo, gi, gj, gk) + goff)].x);
-            }
-        }
-    }
+    warm_stencils<2>(a.gadj2, geo, goff, base, s_dump + threadIdx.x);  // 102 -> 98 us
     async_commit();
     const float dx = (float)a.geo.dx, k3 = 3.f / (dx * dx);
     const float mp = a.cst[(size_t)KM * np + p], cd = EXACT ? (1.f - a.dt * a.drag) : 1.f;
@@ -531,6 +686,15 @@ __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, DMPM_CHUNK_GATHER_MINB) k_
 inline int particle_threads(int n) {
     const int blocks = 148 * 2;
     return n >= 128 * blocks ? 128 : n >= 64 * blocks ? 64 : 32;
+}
+// the same for G2P, with the next stress stage where a.G_next is set
+template <bool BATCH> inline void launch_g2p(const WArgs& a, cudaStream_t st) {
+    const int split = a.n < 40000 ? 4 : 1, t = particle_threads(split * a.n);
+    const unsigned b = (unsigned)((split * a.n + t - 1) / t);
+    if (split == 4 && a.G_next) k_g2p_c<BATCH, true, 4><<<b, t, 0, st>>>(a);
+    else if (split == 4) k_g2p_c<BATCH, false, 4><<<b, t, 0, st>>>(a);
+    else if (a.G_next) k_g2p_c<BATCH, true, 1><<<b, t, 0, st>>>(a);
+    else k_g2p_c<BATCH, false, 1><<<b, t, 0, st>>>(a);
 }
 // Four threads per particle below 40k particles (8.7k: 14.7 against 18-21 us per
 // step), one above (79k: 33 against 57 us)

@@ -254,11 +254,7 @@ __device__ __forceinline__ void load_x_base(const float* st, size_t np, int p, c
     }
 }
 // x' = x + dt v of axis c from the position x read by load_x_base, into the
-// next layer's planes (hi and, when xlo, lo); returns the stored hi.  The
-// brick G2P keeps x in registers from its first load (64.6 us per step on the
-// 64^3, 267k-particle workload, against 67.4 us re-reading it before the
-// store); the warp-item G2P re-reads it (advance_x), as holding it there
-// costs 52 bytes of spill at its 64-register budget.
+// next layer's planes (hi and, when xlo, lo); returns the stored hi
 __device__ __forceinline__ float store_x(float* st_next, size_t npn, int p, int c, double x, float dt, float v,
                                          int xlo) {
     if (!xlo) {
@@ -272,12 +268,6 @@ __device__ __forceinline__ float store_x(float* st_next, size_t npn, int p, int 
     st_next[(size_t)(PXL + c) * npn + p] = (float)(xn - (double)hi);
     return hi;
 }
-// the same, re-reading x from layer n's planes
-__device__ __forceinline__ float advance_x(const float* st, float* st_next, size_t npl, size_t npn, int p, int c,
-                                           float dt, float v, int xlo) {
-    return store_x(st_next, npn, p, c, load_xd(st, npl, p, c, xlo), dt, v, xlo);
-}
-
 // ------------------------------------------------------------------ args
 // Minimum resident blocks per SM (the register cap the compiler works to) for
 // k_stress at 256 threads per block (2: 128 registers, no spills; 1 lets it take
@@ -362,11 +352,12 @@ struct WArgs {
     float* dbg_dLdP;
     float* dbg_vnext;
     float* dbg_Cnext;
-    // G2P with the next step's stress stage (kernels_brick.cuh): dFc of layer n + 1,
+    // G2P with the next step's stress stage (kernels_chunk.cuh): dFc of layer n + 1,
     // its G planes and its debug P (or null)
     const float* dfc_next;
     float* G_next;
     float* P_next;
+    int n_next;            // particles that take the next step (a batch's shorter rollouts end)
     // deterministic mode (fixpoint.cuh): integer node sums and their bound slots, or null
     fix4* fix;
     unsigned* fixb;
@@ -401,42 +392,6 @@ template <int MODE> __device__ __forceinline__ void item_grid(const WArgs& a, in
         g = a.geo;
         goff = 0;
     }
-}
-
-// G2P and the adjoint gather over a warp whose 32 lanes share one stencil base
-// (all 8 particles of the item in one cell, the common case after the cell sort)
-// first copies the item's 64 stencil nodes, R consecutive node4 records each,
-// from global memory into the warp's shared-memory slice: 2R independent
-// 16-byte loads per lane, all in flight together, instead of 16 R dependent
-// loads per lane.  Record r of stencil node (s, j, k) lands at
-// dst[stage_index<R>(16 s + 4 j + k, r)]; nodes outside the grid are stored as
-// zeros.  Each slab's 16 R records are followed by one padding record, so the
-// four slabs that a warp's lanes read at the same time fall into different
-// shared-memory banks (without it the reads conflict 4-way; with it the
-// gather takes 86 instead of 116 us and G2P 56 instead of 73 us on the 64^3,
-// 267k-particle workload).  Warp kernels run 256-thread blocks (8 warps), one
-// slice per warp.
-#ifndef DMPM_STAGE_NODES
-#define DMPM_STAGE_NODES 1
-#endif
-template <int R> __device__ __forceinline__ int stage_index(int n, int r) { return R * n + r + (n >> 4); }
-template <int R> struct StageRecords { static constexpr int value = 64 * R + 4; };
-template <int R>
-__device__ __forceinline__ void stage_stencil(const node4<float>* __restrict__ src, const GridGeom& g, int goff,
-                                              const int base[3], node4<float>* dst) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();  // the previous item's readers are done with the slice
-#pragma unroll
-    for (int i = 0; i < 2 * R; i++) {
-        const int t = lane + 32 * i;
-        const int n = t / R, r = t % R;
-        const int gi = base[0] + (n >> 4), gj = base[1] + ((n >> 2) & 3), gk = base[2] + (n & 3);
-        const bool in = (unsigned)gi < (unsigned)g.dim[0] && (unsigned)gj < (unsigned)g.dim[1] &&
-                        (unsigned)gk < (unsigned)g.dim[2];
-        dst[stage_index<R>(n, r)] = in ? src[(size_t)R * (unsigned)((gi * g.dim[1] + gj) * g.dim[2] + gk + goff) + r]
-                                       : node4<float>{0.f, 0.f, 0.f, 0.f};
-    }
-    __syncwarp();
 }
 
 // ------------------------------------------------------------------ forward
@@ -607,135 +562,6 @@ static __global__ void k_gop_inplace(node4<float>* grid, size_t G, float dt, flo
     nd.y = v[1];
     nd.z = v[2];
     grid[g] = nd;
-}
-
-// G2P + P_op_2: v' = sum w v_g;  C' = 3/dx^2 sum w v_g d^T;
-// F' = (1 - s)(I + dt C')(F + dFc) + s F;  x' = x + dt v'
-// G2P keeps 64 registers without spills, so four 256-thread CTAs reside per SM
-#ifndef DMPM_G2P_CTAS
-#define DMPM_G2P_CTAS 4
-#endif
-template <int MODE> __global__ void __launch_bounds__(256, 4) k_g2p_w(WArgs a) {
-    const int nit = item_count(a);
-    const size_t np = a.np, npl = a.npl, npn = a.npn;
-    for (int item = first_warp(); item < nit; item = next_item<MODE>(item, nit)) {
-        GridGeom geo;
-        int goff;
-        item_grid<MODE>(a, item, geo, goff);
-        const ItemLane L = item_lane(a.items, item);
-        float t[3];
-        int base[3];
-        load_x_base(a.st, npl, L.p, geo, t, base, a.xlo);
-        LaneW w;
-        float own1[3];
-        lane_weights_k(t, geo, L.s, w, own1, false);
-        // v = sum w v_g and C = sum w v_g d^T (scaled by 3/dx^2 at the end), with the
-        // weight w = n0 n1[j] n2[k] and d = (d0, d1[j], d2[k]) factored per stencil row:
-        // the node loop accumulates only the k-dependent sums, the row applies n0 n1[j]
-        // and d1[j], and the d0 column is d0 v.
-        float nd2[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) nd2[k] = w.n2[k] * w.d2[k];
-        float V[3] = {0.f, 0.f, 0.f}, C1[3] = {0.f, 0.f, 0.f}, C2[3] = {0.f, 0.f, 0.f};
-        // one stencil row j from its four node records
-        auto row_sum = [&](int j, const node4<float> (&row)[4]) {
-            float Vj[3] = {0.f, 0.f, 0.f}, Wj[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float vg[3] = {row[k].x, row[k].y, row[k].z};
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    Vj[r] += w.n2[k] * vg[r];
-                    Wj[r] += nd2[k] * vg[r];
-                }
-            }
-            float d1, n1, s1;
-            row_weights(own1, j, d1, n1, s1);
-            const float w01 = w.n0 * n1, w01d = w01 * d1;
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                V[r] += w01 * Vj[r];
-                C1[r] += w01d * Vj[r];
-                C2[r] += w01 * Wj[r];
-            }
-        };
-        // a uniform item stages its 64 stencil nodes in shared memory (stage_stencil);
-        // otherwise each lane loads its slab's nodes, a row at a time (the row's four
-        // records before any is used; nodes outside the grid read as zero)
-        __shared__ node4<float> s_nodes[8][StageRecords<1>::value];
-        if (DMPM_STAGE_NODES && warp_uniform_base(base)) {
-            node4<float>* sw = s_nodes[threadIdx.x >> 5];
-            stage_stencil<1>(a.grid, geo, goff, base, sw);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                node4<float> row[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) row[k] = sw[stage_index<1>(16 * L.s + 4 * j + k, 0)];
-                row_sum(j, row);
-            }
-        } else {
-            LaneNodes N = lane_nodes(geo, base, L.s);
-            N.g00 += goff;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                node4<float> row[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    row[k] = ((N.mask >> (4 * j + k)) & 1u) ? a.grid[N.g00 + j * N.sj + k]
-                                                            : node4<float>{0.f, 0.f, 0.f, 0.f};
-                row_sum(j, row);
-            }
-        }
-        float acc[12];  // v (3), C (9) row-major
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            acc[r] = V[r];
-            acc[3 + 3 * r] = w.d0 * V[r];
-            acc[4 + 3 * r] = C1[r];
-            acc[5 + 3 * r] = C2[r];
-        }
-        reduce_slabs<12>(acc);
-        if (!L.valid) continue;
-        const float dx = (float)geo.dx;
-        const float k3 = 3.f / (dx * dx);
-        const int p = L.p;
-        m3<float> Cn;
-#pragma unroll
-        for (int r = 0; r < 3; r++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) Cn.a[r][c] = k3 * acc[3 + 3 * r + c];
-        // lane s = 0 stores x' and v', s = 1 C'; lanes s = 0, 2, 3 each one column
-        // c of F' = (1-s)(I + dt C') Fe[:,c] + s F[:,c]
-        bool finite = true;
-        if (L.s == 0) {
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const float xn = advance_x(a.st, a.st_next, npl, npn, p, c, a.dt, acc[c], a.xlo);
-                a.st_next[(size_t)(PV + c) * npn + p] = acc[c];
-                finite &= isfinite(xn);
-            }
-        }
-        if (L.s == 1) {
-            store_m3(a.st_next + (size_t)PC * npn, npn, p, Cn);
-        } else {
-            // column c of the strain: H' = (1 - s)(D + dt C' (I + D)) + s H,  D = H + dFc
-            const int c = L.s == 0 ? 0 : L.s - 1;
-            float Hc[3], Dc[3];
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                Hc[r] = a.st[(size_t)(PF + r + 3 * c) * npl + p];
-                Dc[r] = Hc[r] + a.dfc[(size_t)(r + 3 * c) * np + p];
-            }
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const float t = Dc[r] + a.dt * (Cn.a[r][c] + (Cn.a[r][0] * Dc[0] + Cn.a[r][1] * Dc[1] + Cn.a[r][2] * Dc[2]));
-                const float hn = (1.f - a.s) * t + a.s * Hc[r];
-                a.st_next[(size_t)(PF + r + 3 * c) * npn + p] = hn;
-                finite &= isfinite(hn);
-            }
-        }
-        if (!finite) atomicOr(a.status, ST_NONFINITE_FWD);
-    }
 }
 
 // ------------------------------------------------------------------ adjoint
