@@ -46,32 +46,34 @@ constexpr int kAux = 24;  // G (9), polar R (9), polar S (6) per particle and st
 constexpr int kDefaultSortEvery = 8;
 constexpr int kDefaultCtasPerSm = 3;
 
-// cell key of each particle of the active prefix: its instance's key offset +
-// the one-scene key of sort.cuh (the stencil base the warp-item kernels form)
-__global__ void k_cell_keys_batch(int n, size_t np, const float* __restrict__ st, const uint16_t* __restrict__ pinst,
-                                  const InstGeo* __restrict__ ig, uint32_t* keys, uint32_t* vals) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
+// cell key of a particle of the active prefix: its instance's key offset + the
+// one-scene key of sort.cuh (the stencil base the chunk kernels form)
+__device__ __forceinline__ uint32_t batch_key(size_t np, const float* __restrict__ st, const uint16_t* __restrict__ pinst,
+                                              const InstGeo* __restrict__ ig, int p) {
     const InstGeo g = ig[pinst[p]];
     int base[3];
 #pragma unroll
     for (int c = 0; c < 3; c++)
         (void)stencil_coord<float>(load_xd(st, np, p, c, 1), g.g.mn[c], 1.0 / g.g.dx, g.g.dim[c], base[c]);
-    keys[p] = g.koff + cell_key(base, g.g.dim);
+    return g.koff + cell_key(base, g.g.dim);
+}
+// keys and particle indices for the radix sort; keys and ranks for the counting sort
+__global__ void k_cell_keys_batch(int n, size_t np, const float* __restrict__ st, const uint16_t* __restrict__ pinst,
+                                  const InstGeo* __restrict__ ig, uint32_t* keys, uint32_t* vals) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    keys[p] = batch_key(np, st, pinst, ig, p);
     vals[p] = (uint32_t)p;
 }
-
-// instance of every warp item, and one past the last item of each instance
-// (items of an instance are contiguous: its keys form one range)
-__global__ void k_item_inst(const uint32_t* __restrict__ order, const uint32_t* __restrict__ items,
-                            const uint32_t* __restrict__ n_items, const uint16_t* __restrict__ pinst, int cap,
-                            uint16_t* item_inst, uint32_t* item_end) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ni = (int)*n_items;
-    if (j >= ni || j >= cap) return;
-    const uint16_t i = pinst[order[items[j]]];
-    item_inst[j] = i;
-    if (j + 1 == ni || pinst[order[items[j + 1]]] != i) item_end[i] = (uint32_t)(j + 1);
+__global__ void k_cell_count_batch(int n, size_t np, const float* __restrict__ st, const uint16_t* __restrict__ pinst,
+                                   const InstGeo* __restrict__ ig, uint32_t* keys, uint32_t* rank, uint32_t* count) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = p < n;
+    const uint32_t key = valid ? batch_key(np, st, pinst, ig, p) : 0xffffffffu;
+    const uint32_t r = count_rank(key, valid, count);
+    if (!valid) return;
+    keys[p] = key;
+    rank[p] = r;
 }
 
 __global__ void k_set_target(const double* __restrict__ src, size_t G, float* dst) {
@@ -95,10 +97,6 @@ struct Inst {
 
 struct BEpoch {
     uint32_t* order = nullptr;
-    uint32_t* items = nullptr;
-    uint16_t* item_inst = nullptr;
-    uint32_t* item_end = nullptr;  // [instances]
-    uint32_t* n_items = nullptr;   // device scalar
 };
 
 }  // namespace
@@ -149,7 +147,8 @@ struct dmpm_batch::Impl {
     double* ctrl_acc = nullptr;
     std::vector<BEpoch> ep;
     int ep_every = 0;
-    uint32_t *sk[2] = {nullptr, nullptr}, *sv[2] = {nullptr, nullptr}, *sh = nullptr, *sf = nullptr;
+    uint32_t *sk[2] = {nullptr, nullptr}, *sv[2] = {nullptr, nullptr};
+    uint32_t *count_keys = nullptr, *count_totals = nullptr;  // counting sort, or null (radix sort)
     uint32_t *counts = nullptr, *tile_tot = nullptr;
     bool ready = false;
     cudaGraphExec_t gexec = nullptr;
@@ -372,12 +371,6 @@ struct dmpm_batch::Impl {
             const size_t n = P[e * se + 1];  // particles stepping at the epoch's first step
             BEpoch x;
             x.order = (uint32_t*)epochs_arena.alloc(n * 4);
-            x.items = (uint32_t*)epochs_arena.alloc((n + 1) * 4);
-            x.item_inst = (uint16_t*)epochs_arena.alloc(n * 2);
-            x.item_end = (uint32_t*)epochs_arena.alloc((size_t)count * 4);
-            x.n_items = (uint32_t*)epochs_arena.alloc(16);
-            DMPM_CK(cudaMemsetAsync(x.item_end, 0, (size_t)count * 4, b->stream));
-            DMPM_CK(cudaMemsetAsync(x.n_items, 0, 16, b->stream));
             ep.push_back(x);
         }
         ep_every = se;
@@ -421,8 +414,12 @@ struct dmpm_batch::Impl {
             sk[i] = (uint32_t*)layers.alloc(np0 * 4);
             sv[i] = (uint32_t*)layers.alloc(np0 * 4);
         }
-        sh = (uint32_t*)layers.alloc(np0 * 4);
-        sf = (uint32_t*)layers.alloc(np0 * 4);
+        count_keys = nullptr;
+        if (counting_sort_fits(keys_total, N)) {
+            const size_t tiles = count_tiles(keys_total);
+            count_keys = (uint32_t*)layers.alloc(tiles * COUNT_TILE * 4);
+            count_totals = (uint32_t*)layers.alloc(tiles * 4);
+        }
         const size_t rs_tiles = (N + RS_TILE - 1) / RS_TILE;
         counts = (uint32_t*)layers.alloc(256 * rs_tiles * 4);
         const size_t mx = std::max(N, 256 * rs_tiles);
@@ -446,9 +443,19 @@ struct dmpm_batch::Impl {
         launched();
     }
 
-    // stable sort of the particles stepping at t (layer t) by instance-prefixed cell key
+    // order of the particles stepping at t (layer t) by instance-prefixed cell key
     void cell_sort(int t, BEpoch& e) {
         const int n = (int)P[t + 1];
+        if (count_keys) {
+            DMPM_CK(cudaMemsetAsync(count_keys, 0, count_tiles(keys_total) * COUNT_TILE * 4, b->stream));
+            k_cell_count_batch<<<(n + 255) / 256, 256, 0, b->stream>>>(n, S[t], st[t], pinst, ig, sk[0], sv[0], count_keys);
+            launched();
+            launch_count_order(sk[0], sv[0], count_keys, count_totals, keys_total, n, e.order, b->stream);
+            launched();
+            launched();
+            launched();
+            return;
+        }
         k_cell_keys_batch<<<(n + 255) / 256, 256, 0, b->stream>>>(n, S[t], st[t], pinst, ig, sk[0], sv[0]);
         launched();
         int bits = 1;
@@ -465,19 +472,6 @@ struct dmpm_batch::Impl {
             cur ^= 1;
         }
         DMPM_CK(cudaMemcpyAsync(e.order, sv[cur], (size_t)n * 4, cudaMemcpyDeviceToDevice, b->stream));
-        k_run_heads<<<(n + 255) / 256, 256, 0, b->stream>>>(sk[cur], n, sh);
-        launched();
-        scan<OpMax>(sh, (size_t)n, nullptr);
-        k_item_flags<<<(n + 255) / 256, 256, 0, b->stream>>>(sk[cur], sh, n, sf);
-        launched();
-        scan<OpSum>(sf, (size_t)n, e.n_items);
-        k_item_starts<<<(n + 255) / 256, 256, 0, b->stream>>>(sk[cur], sh, sf, n, e.items);
-        launched();
-        k_item_sentinel<<<1, 1, 0, b->stream>>>(e.items, e.n_items, n);
-        launched();
-        k_item_inst<<<(n + 255) / 256, 256, 0, b->stream>>>(e.order, e.items, e.n_items, pinst, n, e.item_inst,
-                                                            e.item_end);
-        launched();
     }
 
     WArgs args(int t) const {
@@ -493,10 +487,8 @@ struct dmpm_batch::Impl {
         a.s = (float)prm.smoothing;
         for (int c = 0; c < 3; c++) a.fext[c] = (float)prm.f_ext[c];
         const BEpoch& e = ep[t / ep_every];
-        a.items = WarpItems{e.order, e.items, 0};
-        a.n_items_dev = e.item_end + (A[t + 1] - 1);
+        a.items = WarpItems{e.order, nullptr};
         a.ig = ig;
-        a.item_inst = e.item_inst;
         a.pinst = pinst;
         a.st = st[t];
         a.st_next = st[t + 1];

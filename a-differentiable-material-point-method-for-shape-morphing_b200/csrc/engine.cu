@@ -252,11 +252,13 @@ template <class T> class Engine : public EngineBase {
         uint32_t* unit_items = nullptr;  // first warp item of each unit
         uint32_t* n_units = nullptr;
         int unit_shift = -1;
-        bool valid = false;
+        bool valid = false;    // order holds a cell order of the epoch
+        bool grouped = false;  // and it is the stable one, with items and units (deterministic mode)
     };
 
     explicit Engine(dmpm_ctx* c) : ctx_(c) {
-        for (Arena* a : {&scene_arena_, &scene_arena_grid_, &layer_arena_, &staging_arena_, &misc_arena_, &fix_arena_})
+        for (Arena* a : {&scene_arena_, &scene_arena_grid_, &layer_arena_, &staging_arena_, &misc_arena_, &fix_arena_,
+                         &group_arena_})
             a->set_budget(&ctx_->budget);
     }
 
@@ -322,7 +324,7 @@ template <class T> class Engine : public EngineBase {
             // scratch: the first epoch's order and items (recomputed by the next forward
             // pass) and layer 0's state planes (overwritten from st0_ right after)
             Epoch& e = epochs_[0];
-            cell_sort(st0_, e);  // e.order[i] = index of the i-th particle in cell order
+            cell_sort(st0_, e, false);  // e.order[i] = index of the i-th particle in cell order
             if (!perm_) perm_ = (uint32_t*)scene_arena_.alloc((size_t)n_ * 4);
             DMPM_CK(cudaMemcpyAsync(perm_, e.order, (size_t)n_ * 4, cudaMemcpyDeviceToDevice, ctx_->stream));
             T* buf = layers_[0].st;
@@ -535,17 +537,11 @@ template <class T> class Engine : public EngineBase {
     }
 
     // the deterministic adjoint scatter: through each unit's shared node tile when the epoch has units
-    template <bool EX, bool GEN> void launch_adj_scatter_fix_t(const WArgs& a, int ush, unsigned ws) {
+    template <bool GEN> void launch_adj_scatter_fix(const WArgs& a, int ush, unsigned ws) {
         const unsigned bt = DMPM_BRICK_THREADS;
-        if (ush == 3) k_adj_scatter_fix_b<2, EX, GEN><<<brick_blocks(k_adj_scatter_fix_b<2, EX, GEN>), bt, 0, ctx_->stream>>>(a);
-        else if (ush == 6) k_adj_scatter_fix_b<4, EX, GEN><<<brick_blocks(k_adj_scatter_fix_b<4, EX, GEN>), bt, 0, ctx_->stream>>>(a);
-        else k_adj_scatter_w<EX, GEN, ITEMS_PERSISTENT, true><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, ctx_->stream>>>(a);
-    }
-    void launch_adj_scatter_fix(const WArgs& a, bool ex, bool gen, int ush, unsigned ws) {
-        if (ex && gen) launch_adj_scatter_fix_t<true, true>(a, ush, ws);
-        else if (ex) launch_adj_scatter_fix_t<true, false>(a, ush, ws);
-        else if (gen) launch_adj_scatter_fix_t<false, true>(a, ush, ws);
-        else launch_adj_scatter_fix_t<false, false>(a, ush, ws);
+        if (ush == 3) k_adj_scatter_fix_b<2, GEN><<<brick_blocks(k_adj_scatter_fix_b<2, GEN>), bt, 0, ctx_->stream>>>(a);
+        else if (ush == 6) k_adj_scatter_fix_b<4, GEN><<<brick_blocks(k_adj_scatter_fix_b<4, GEN>), bt, 0, ctx_->stream>>>(a);
+        else k_adj_scatter_w<GEN><<<ws, DMPM_ADJ_SCATTER_THREADS, 0, ctx_->stream>>>(a);
     }
 
     void launched() {
@@ -899,16 +895,12 @@ template <class T> class Engine : public EngineBase {
     void alloc_sort() {
         const int nep = std::max(1, (L_ - 1 + sort_every() - 1) / sort_every());
         epochs_.assign(nep, Epoch{});
-        for (Epoch& e : epochs_) {
-            e.order = (uint32_t*)layer_arena_.alloc((size_t)n_ * sizeof(uint32_t));
-            e.items = (uint32_t*)layer_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
-            e.n_items = (uint32_t*)layer_arena_.alloc(16);
-            if (ctx_->prm.brick_cells) {
-                e.units = (uint32_t*)layer_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
-                e.unit_keys = (uint32_t*)layer_arena_.alloc((size_t)n_ * sizeof(uint32_t));
-                e.unit_items = (uint32_t*)layer_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
-                e.n_units = (uint32_t*)layer_arena_.alloc(16);
-            }
+        for (Epoch& e : epochs_) e.order = (uint32_t*)layer_arena_.alloc((size_t)n_ * sizeof(uint32_t));
+        count_ = nullptr;
+        if (counting_sort_fits(key_span(geo_.dim), (size_t)n_)) {
+            const size_t tiles = count_tiles(key_span(geo_.dim));
+            count_ = (uint32_t*)layer_arena_.alloc(tiles * COUNT_TILE * 4);
+            count_totals_ = (uint32_t*)layer_arena_.alloc(tiles * 4);
         }
         const size_t n = (size_t)n_;
         sk_[0] = (uint32_t*)layer_arena_.alloc(n * 4);
@@ -923,6 +915,53 @@ template <class T> class Engine : public EngineBase {
         tile_tot_ = (uint32_t*)layer_arena_.alloc(((mx + SCAN_TILE - 1) / SCAN_TILE + 1) * 4);
     }
 
+    // items and units of every epoch, which only the deterministic mode reads;
+    // like its integer grid allocated on first use, before any capture
+    void ensure_groups() {
+        if (!det() || epochs_.empty() || epochs_[0].items) return;
+        group_arena_.release();
+        drop_graphs();
+        for (Epoch& e : epochs_) {
+            e.items = (uint32_t*)group_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
+            e.n_items = (uint32_t*)group_arena_.alloc(16);
+            e.units = (uint32_t*)group_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
+            e.unit_keys = (uint32_t*)group_arena_.alloc((size_t)n_ * sizeof(uint32_t));
+            e.unit_items = (uint32_t*)group_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
+            e.n_units = (uint32_t*)group_arena_.alloc(16);
+        }
+    }
+
+    // The order the pass needs: the counting sort where it fits, else (and in the
+    // deterministic mode, which needs stable order, items and units) the radix sort.
+    void cell_order(const T* st, Epoch& e) {
+        if (det() || !count_) {
+            cell_sort(st, e, det());
+            return;
+        }
+        const uint64_t keys = key_span(geo_.dim);
+        DMPM_CK(cudaMemsetAsync(count_, 0, count_tiles(keys) * COUNT_TILE * 4, ctx_->stream));
+        k_cell_count<T><<<(n_ + 255) / 256, 256, 0, ctx_->stream>>>(key_args(st), count_);
+        launched();
+        launch_count_order(sk_[0], sv_[0], count_, count_totals_, keys, n_, e.order, ctx_->stream);
+        launched();
+        launched();
+        launched();
+        e.unit_shift = -1;
+        e.grouped = false;
+        e.valid = true;
+    }
+    KeyArgs<T> key_args(const T* st) const {
+        KeyArgs<T> ka{};
+        ka.n = n_;
+        ka.np = np_;
+        ka.geo = geo_;
+        ka.st = st;
+        ka.xlo = kWarp ? 1 : 0;
+        ka.keys = sk_[0];
+        ka.vals = sv_[0];
+        return ka;
+    }
+
     template <class Op> void device_scan(uint32_t* data, size_t n, uint32_t* grand) {
         const int tiles = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
         k_scan_tiles<Op><<<tiles, SCAN_THREADS, 0, ctx_->stream>>>(data, (int)n, tile_tot_);
@@ -934,18 +973,12 @@ template <class T> class Engine : public EngineBase {
     }
 
     // Stable sort of the particles of a layer state by cell key; fills the
-    // epoch's order and warp items.  Keys stay in sk_[sorted_] for inspection.
-    void cell_sort(const T* st, Epoch& e) {
+    // epoch's order and, with groups, its warp items and units.  Keys stay in
+    // sk_[sorted_] for inspection.
+    void cell_sort(const T* st, Epoch& e, bool groups) {
+        if (groups && !e.items) throw StateError{"internal: the epoch has no item storage"};
         const int n = n_;
-        KeyArgs<T> ka{};
-        ka.n = n;
-        ka.np = np_;
-        ka.geo = geo_;
-        ka.st = st;
-        ka.xlo = kWarp ? 1 : 0;
-        ka.keys = sk_[0];
-        ka.vals = sv_[0];
-        k_cell_keys<T><<<(n + 255) / 256, 256, 0, ctx_->stream>>>(ka);
+        k_cell_keys<T><<<(n + 255) / 256, 256, 0, ctx_->stream>>>(key_args(st));
         launched();
         const uint64_t max_key = key_span(geo_.dim);
         int bits = 1;
@@ -963,6 +996,10 @@ template <class T> class Engine : public EngineBase {
         }
         sorted_ = cur;
         DMPM_CK(cudaMemcpyAsync(e.order, sv_[cur], (size_t)n * 4, cudaMemcpyDeviceToDevice, ctx_->stream));
+        e.unit_shift = -1;
+        e.grouped = groups;
+        e.valid = true;
+        if (!groups) return;
         k_run_heads<<<(n + 255) / 256, 256, 0, ctx_->stream>>>(sk_[cur], n, sh_);
         launched();
         device_scan<OpMax>(sh_, (size_t)n, nullptr);
@@ -973,7 +1010,6 @@ template <class T> class Engine : public EngineBase {
         launched();
         k_item_sentinel<<<1, 1, 0, ctx_->stream>>>(e.items, e.n_items, n);
         launched();
-        e.unit_shift = -1;
         if (ctx_->prm.brick_cells && e.units) {
             const int shift = ctx_->prm.brick_cells == 4 ? 6 : 3;
             k_unit_flags<<<(n + 255) / 256, 256, 0, ctx_->stream>>>(sk_[cur], n, shift, sf_);
@@ -988,15 +1024,14 @@ template <class T> class Engine : public EngineBase {
             launched();
             e.unit_shift = shift;
         }
-        e.valid = true;
     }
 
     Epoch& epoch_for(int l, const T* st, bool allow_sort) {
         Epoch& e = epochs_[std::min((int)epochs_.size() - 1, l / sort_every())];
-        if (allow_sort && (l % sort_every() == 0 || !e.valid)) cell_sort(st, e);
-        if (!e.valid) cell_sort(st, e);
+        if ((allow_sort && l % sort_every() == 0) || !usable(e)) cell_order(st, e);
         return e;
     }
+    bool usable(const Epoch& e) const { return e.valid && (e.grouped || !det()); }
 
     void debug_cell_sort(int l, uint32_t* keys, uint32_t* order, uint32_t* items, int* n_items) {
         if (!kWarp) throw StateError{"the cell sort belongs to the FP32 path"};
@@ -1006,7 +1041,7 @@ template <class T> class Engine : public EngineBase {
         e.order = (uint32_t*)tmp.alloc((size_t)n_ * 4);
         e.items = (uint32_t*)tmp.alloc(((size_t)n_ + 1) * 4);
         e.n_items = (uint32_t*)tmp.alloc(16);
-        cell_sort(materialize_state(l), e);
+        cell_sort(materialize_state(l), e, true);
         uint32_t ni = 0;
         DMPM_CK(cudaMemcpyAsync(&ni, e.n_items, 4, cudaMemcpyDeviceToHost, ctx_->stream));
         DMPM_CK(cudaStreamSynchronize(ctx_->stream));
@@ -1064,10 +1099,11 @@ template <class T> class Engine : public EngineBase {
     bool step(int l, const T* st, T* out, node4<T>* g, T* Gd, bool allow_sort, bool g_ready = false,
               T* Gd_next = nullptr) {
         if constexpr (kWarp) {
-            ensure_fix();  // allocated already (a no-op) on every captured path
+            ensure_fix();  // allocated already (no-ops) on every captured path
+            ensure_groups();
             Epoch& ep = epoch_for(l, st, allow_sort);
             WArgs a = warp_args();
-            a.items = WarpItems{ep.order, ep.items, 0};
+            a.items = WarpItems{ep.order, ep.items};
             a.n_items_dev = ep.n_items;
             a.st = (const float*)st;
             a.st_next = (float*)out;
@@ -1101,8 +1137,8 @@ template <class T> class Engine : public EngineBase {
             } else if (dm && ush == 6) {
                 if (gen) k_p2g_fix_b<4, true><<<brick_blocks(k_p2g_fix_b<4, true>), bt, 0, ctx_->stream>>>(a);
                 else k_p2g_fix_b<4, false><<<brick_blocks(k_p2g_fix_b<4, false>), bt, 0, ctx_->stream>>>(a);
-            } else if (dm && gen) k_p2g_w<true, ITEMS_PERSISTENT, true><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
-            else if (dm) k_p2g_w<false, ITEMS_PERSISTENT, true><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
+            } else if (dm && gen) k_p2g_w<true><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
+            else if (dm) k_p2g_w<false><<<ws, DMPM_P2G_THREADS, 0, ctx_->stream>>>(a);
             else if (gen) k_p2g_c<false, true><<<chunk_blocks(n_, a.chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a);
             else k_p2g_c<false, false><<<chunk_blocks(n_, a.chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a);
             launched();
@@ -1218,7 +1254,8 @@ template <class T> class Engine : public EngineBase {
         if (L_ <= 0) throw StateError{"dmpm_setup has not been called"};
         if (start < 0 || start >= L_) throw ArgError{"start_layer out of range"};
         reset_status();
-        ensure_fix();  // before any capture: a captured launch holds the buffer's address
+        ensure_fix();  // before any capture: a captured launch holds the buffers' addresses
+        ensure_groups();
         if (k_ == 1) {
             auto body = [&]() {
                 bool ready = false;  // layer l's G formed by the previous step
@@ -1229,8 +1266,11 @@ template <class T> class Engine : public EngineBase {
             if (graphs_ok()) {
                 run_graph({0, start}, body);
                 if constexpr (kWarp)  // the replayed sorts refreshed every epoch the pass touches
-                    for (int l = start; l + 1 < L_; l++)
-                        epochs_[std::min((int)epochs_.size() - 1, l / sort_every())].valid = true;
+                    for (int l = start; l + 1 < L_; l++) {
+                        Epoch& e = epochs_[std::min((int)epochs_.size() - 1, l / sort_every())];
+                        e.valid = true;
+                        e.grouped = det() || !count_;
+                    }
             } else {
                 body();
             }
@@ -1325,7 +1365,7 @@ template <class T> class Engine : public EngineBase {
         if constexpr (kWarp) {
             Epoch& ep = epoch_for(i, state_of(i), false);
             WArgs a = warp_args();
-            a.items = WarpItems{ep.order, ep.items, 0};
+            a.items = WarpItems{ep.order, ep.items};
             a.n_items_dev = ep.n_items;
             a.st = (const float*)state_of(i);
             a.st_next = (float*)state_of(i + 1);
@@ -1359,7 +1399,8 @@ template <class T> class Engine : public EngineBase {
                 if (ex) k_adj_sources<true><<<pgrid256(), 256, 0, ctx_->stream>>>(a);
                 else k_adj_sources<false><<<pgrid256(), 256, 0, ctx_->stream>>>(a);
                 launched();
-                launch_adj_scatter_fix(a, ex, P.warp_general != 0, ush, ws);
+                if (P.warp_general) launch_adj_scatter_fix<true>(a, ush, ws);
+                else launch_adj_scatter_fix<false>(a, ush, ws);
                 launched();
                 k_fix_to_node4<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, 1, (node4<float>*)gadj_);
             } else {
@@ -1456,6 +1497,7 @@ template <class T> class Engine : public EngineBase {
     void backward_range(int top, int control) {
         if (!forward_done_ && L_ > 1) throw StateError{"dmpm_forward has not been run"};
         ensure_fix();
+        ensure_groups();
         if (top < 0 || top > L_ - 1) throw ArgError{"top layer out of range"};
         if (control < 0 || control > top) throw ArgError{"control_layer out of range"};
         if (top < L_ - 1 && !layers_[top].adj) throw StateError{"set keep_adjoints to start the adjoint below the last layer"};
@@ -1468,7 +1510,7 @@ template <class T> class Engine : public EngineBase {
             bool sorted = true;  // a captured backward pass must not contain sorts
             if constexpr (kWarp)
                 for (int i = top - 1; i >= control; i--)
-                    sorted &= epochs_[std::min((int)epochs_.size() - 1, i / sort_every())].valid;
+                    sorted &= usable(epochs_[std::min((int)epochs_.size() - 1, i / sort_every())]);
             if (graphs_ok() && sorted) run_graph({1 + (int64_t)top, control}, body);
             else body();
         } else {
@@ -1771,7 +1813,7 @@ template <class T> class Engine : public EngineBase {
     bool grid_set_ = false;
     int n_ = 0;
     size_t np_ = 0;
-    Arena scene_arena_, scene_arena_grid_, layer_arena_, staging_arena_, misc_arena_, fix_arena_;
+    Arena scene_arena_, scene_arena_grid_, layer_arena_, staging_arena_, misc_arena_, fix_arena_, group_arena_;
     T* cst_ = nullptr;
     T* st0_ = nullptr;
     T* dfc0_ = nullptr;
@@ -1815,6 +1857,8 @@ template <class T> class Engine : public EngineBase {
     uint32_t* sf_ = nullptr;
     uint32_t* counts_ = nullptr;
     uint32_t* tile_tot_ = nullptr;
+    uint32_t* count_ = nullptr;  // counting sort: a counter per key and the scan's tile totals, or null
+    uint32_t* count_totals_ = nullptr;
     int sorted_ = 0;
     std::map<int, T*> adam_;  // Adam moment buffers per control set (layer, or -1 for tied controls)
     double* ctrl_acc_ = nullptr;

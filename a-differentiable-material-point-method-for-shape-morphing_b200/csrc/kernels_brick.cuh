@@ -87,13 +87,13 @@ __global__ void __launch_bounds__(DMPM_BRICK_THREADS, DMPM_FIX_P2G_MINB) k_p2g_f
         FixTile ft;
         fix_tile_begin<B>(ft, tile, a.unit_key[u], a.geo);
         for (uint32_t it = a.unit_item[u] + warp; it < a.unit_item[u + 1]; it += nw)
-            p2g_item<GENERAL, ITEMS_PERSISTENT, true, true>(a, (int)it, sp, sm, ft);
+            p2g_item<GENERAL, true>(a, (int)it, sp, sm, ft);
         __syncthreads();
         fix_tile_flush<B>(ft, a.geo, a.fix);
     }
 }
 
-template <int B, bool EXACT, bool GENERAL>
+template <int B, bool GENERAL>
 __global__ void __launch_bounds__(DMPM_BRICK_THREADS, DMPM_FIX_SCATTER_MINB) k_adj_scatter_fix_b(WArgs a) {
     __shared__ long long tile[4 * BrickShape<B>::NT];
     const int nun = (int)*a.n_units_dev;
@@ -102,8 +102,7 @@ __global__ void __launch_bounds__(DMPM_BRICK_THREADS, DMPM_FIX_SCATTER_MINB) k_a
     for (int u = blockIdx.x; u < nun; u += gridDim.x) {
         FixTile ft;
         fix_tile_begin<B>(ft, tile, a.unit_key[u], a.geo);
-        adj_scatter_items<EXACT, GENERAL, ITEMS_PERSISTENT, true, true>(a, (int)a.unit_item[u] + warp,
-                                                                        (int)a.unit_item[u + 1], nw, sa, ft);
+        adj_scatter_items<GENERAL, true>(a, (int)a.unit_item[u] + warp, (int)a.unit_item[u + 1], nw, sa, ft);
         __syncthreads();
         fix_tile_flush<B>(ft, a.geo, a.fix);
     }

@@ -51,7 +51,6 @@ __device__ __forceinline__ m3<double> fe_from_strain_d(const m3<float>& H, const
 struct WarpItems {
     const uint32_t* order;       // sorted particle indices
     const uint32_t* item_start;  // n_items + 1 entries
-    int n_items;
 };
 
 struct ItemLane {
@@ -169,40 +168,9 @@ __device__ __forceinline__ float bsp_slope(float q) {
 }
 
 // The 4 lanes of a particle (equal lane >> 2) each evaluate the weights of
-// stencil node s on all three axes; axis-1 and axis-2 values of the other
-// nodes come from the sibling lanes by shuffles.  Every lane of the warp must
-// call this (full-mask shuffles).
-__device__ __forceinline__ void lane_weights(const float t[3], const GridGeom& g, int s, LaneW& w, bool slopes) {
-    const float dx = (float)g.dx;
-    float d[3], n[3], sl[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const float q = (float)s - t[c];  // node offset in cells (exact for t in [1, 2))
-        d[c] = q * dx;
-        n[c] = bsp(q);
-        sl[c] = slopes ? bsp_slope(q) : 0.f;
-    }
-    w.d0 = d[0];
-    w.n0 = n[0];
-    w.s0 = sl[0];
-    const int grp = (threadIdx.x & 31) & ~3;
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-        w.d1[t] = __shfl_sync(0xffffffffu, d[1], grp + t);
-        w.n1[t] = __shfl_sync(0xffffffffu, n[1], grp + t);
-        w.d2[t] = __shfl_sync(0xffffffffu, d[2], grp + t);
-        w.n2[t] = __shfl_sync(0xffffffffu, n[2], grp + t);
-        if (slopes) {
-            w.s1[t] = __shfl_sync(0xffffffffu, sl[1], grp + t);
-            w.s2[t] = __shfl_sync(0xffffffffu, sl[2], grp + t);
-        } else {
-            w.s1[t] = 0.f;
-            w.s2[t] = 0.f;
-        }
-    }
-}
-
-// As lane_weights, but axis 1 is left to the caller: it gets this lane's own
+// stencil node s on all three axes; axis-2 values of the other nodes come from
+// the sibling lanes by shuffles (every lane of the warp must call this).  Axis 1
+// is left to the caller: it gets this lane's own
 // axis-1 offset, weight and slope in own1 and fetches row j's values with
 // row_weights (three shuffles) when it reaches that row, so only one row's
 // values are live at a time.  Fills d0, n0, s0 and the axis-2 arrays of w,
@@ -328,9 +296,8 @@ struct WArgs {
     GridGeom geo;
     float dt, drag, s, fext[3];
     WarpItems items;
-    const uint32_t* n_items_dev;  // item count on the device (grid-stride launches), or null: items.n_items
-    const InstGeo* ig;            // batch: per-instance grids, indexed by item_inst
-    const uint16_t* item_inst;
+    const uint32_t* n_items_dev;  // warp item count, on the device
+    const InstGeo* ig;            // batch: per-instance grids
     const uint16_t* pinst;        // batch: instance of each particle
     const float* st;       // layer n state
     float* st_next;        // layer n+1 state
@@ -370,29 +337,9 @@ struct WArgs {
     const uint32_t* unit_item;  // first warp item of each unit (n_units + 1 entries), or null
 };
 
-// How a warp-item launch walks its items:
-//   ITEMS_PER_WARP   one warp per item, the grid sized on the host from the item count
-//   ITEMS_PERSISTENT a persistent grid sized to the SMs loops over the items, whose
-//                    count stays on the device (no host read-back, so capturable)
-//   ITEMS_BATCH      persistent, items of several instances, each item's grid looked up
-enum : int { ITEMS_PER_WARP = 0, ITEMS_PERSISTENT = 1, ITEMS_BATCH = 2 };
-__device__ __forceinline__ int item_count(const WArgs& a) {
-    return a.n_items_dev ? (int)*a.n_items_dev : a.items.n_items;
-}
+// Persistent launches over warp items: the item count stays on the device.
 __device__ __forceinline__ int first_warp() { return (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); }
-template <int MODE> __device__ __forceinline__ int next_item(int item, int nit) {
-    return MODE != ITEMS_PER_WARP ? item + (int)((gridDim.x * blockDim.x) >> 5) : nit;
-}
-template <int MODE> __device__ __forceinline__ void item_grid(const WArgs& a, int item, GridGeom& g, int& goff) {
-    if constexpr (MODE == ITEMS_BATCH) {
-        const InstGeo& ig = a.ig[a.item_inst[item]];
-        g = ig.g;
-        goff = ig.goff;
-    } else {
-        g = a.geo;
-        goff = 0;
-    }
-}
+__device__ __forceinline__ int warp_count() { return (int)((gridDim.x * blockDim.x) >> 5); }
 
 // ------------------------------------------------------------------ forward
 // P = PK(F + dFc) in FP64;  G = -3/dx^2 dt vol P Fe^T + m C  (P_op_1 and the
@@ -457,17 +404,15 @@ template <bool DET = false> __global__ void __launch_bounds__(256, DMPM_STRESS_M
 }
 
 // P2G: m_g += w m_p;  p_g += w (m_p v (1 - dt drag) + G (x_g - x_p))
-// One warp item of P2G.  DET: integer node sums (fixpoint.cuh) into a.fix
-// instead of float atomics into a.grid; with a tile (ft.t non-null), the sums
-// of an item whose stencil lies in the tile go to its shared-memory integers.
-template <bool GENERAL, int MODE, bool DET, bool TILE>
+// One warp item of P2G in the deterministic mode: integer node sums
+// (fixpoint.cuh) into a.fix, or with a tile (ft.t non-null) those of an item
+// whose stencil lies in the tile into its shared-memory integers.
+template <bool GENERAL, bool TILE>
 __device__ __forceinline__ void p2g_item(const WArgs& a, int item, const FixScale& sp, const FixScale& sm,
                                          const FixTile& ft) {
     const size_t np = a.np, npl = a.npl;
     {
-        GridGeom geo;
-        int goff;
-        item_grid<MODE>(a, item, geo, goff);
+        const GridGeom& geo = a.geo;
         const ItemLane L = item_lane(a.items, item);
         float t[3];
         int base[3];
@@ -487,8 +432,7 @@ __device__ __forceinline__ void p2g_item(const WArgs& a, int item, const FixScal
             mvd[c] = mp * a.st[(size_t)(PV + c) * npl + L.p] * damp;
             g0[c] = G.a[c][0] * w.d0;
         }
-        LaneNodes N = lane_nodes(geo, base, L.s);
-        N.g00 += goff;
+        const LaneNodes N = lane_nodes(geo, base, L.s);
         // tile offset of node (0, 0, 0) of the item's stencil, or -1 when the stencil is not inside the tile
         const int tile_l = TILE && uniform ? fix_tile_offset(ft, base) : -1;
 #pragma unroll
@@ -517,19 +461,16 @@ __device__ __forceinline__ void p2g_item(const WArgs& a, int item, const FixScal
                 if (((N.mask >> (4 * j + k)) & 1u) && (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f || v[3] != 0.f)) {
                     if (TILE && tile_l >= 0)
                         fix_red4_tile(ft, tile_l + (L.s * ft.E + j) * ft.E + k, v[0], v[1], v[2], v[3], sp.s, sm.s);
-                    else if (DET) fix_red4(a.fix + (N.g00 + j * N.sj + k), v[0], v[1], v[2], v[3], sp.s, sm.s);
-                    else red_add4(a.grid + (N.g00 + j * N.sj + k), v[0], v[1], v[2], v[3]);
+                    else
+                        fix_red4(a.fix + (N.g00 + j * N.sj + k), v[0], v[1], v[2], v[3], sp.s, sm.s);
                 }
             } else if (L.valid) {
 #pragma unroll
                 for (int nd = 0; nd < 8; nd++) {
                     const int j = 2 * half + ((nd >> 2) ^ P.jp), k = (nd & 3) ^ P.kp;
                     if (!((N.mask >> (4 * j + k)) & 1u)) continue;
-                    if (DET)
-                        fix_red4(a.fix + (N.g00 + j * N.sj + k), v[nd * 4], v[nd * 4 + 1], v[nd * 4 + 2], v[nd * 4 + 3],
-                                 sp.s, sm.s);
-                    else
-                        red_add4(a.grid + (N.g00 + j * N.sj + k), v[nd * 4], v[nd * 4 + 1], v[nd * 4 + 2], v[nd * 4 + 3]);
+                    fix_red4(a.fix + (N.g00 + j * N.sj + k), v[nd * 4], v[nd * 4 + 1], v[nd * 4 + 2], v[nd * 4 + 3],
+                             sp.s, sm.s);
                 }
             }
         }
@@ -537,17 +478,11 @@ __device__ __forceinline__ void p2g_item(const WArgs& a, int item, const FixScal
 }
 
 // P2G over warp items (one item per warp, persistent grid-stride)
-template <bool GENERAL, int MODE, bool DET = false>
-__global__ void __launch_bounds__(DMPM_P2G_THREADS, DMPM_SCATTER_MIN_BLOCKS) k_p2g_w(WArgs a) {
-    const int nit = item_count(a);
-    FixScale sp{1.f, 1.f}, sm{1.f, 1.f};
-    if (DET) {
-        sp = fix_scale(a.fixb + FIXB_MOMENTUM, a.n);
-        sm = fix_scale(a.fixb + FIXB_MASS, a.n);
-    }
+template <bool GENERAL> __global__ void __launch_bounds__(DMPM_P2G_THREADS, DMPM_SCATTER_MIN_BLOCKS) k_p2g_w(WArgs a) {
+    const int nit = (int)*a.n_items_dev;
+    const FixScale sp = fix_scale(a.fixb + FIXB_MOMENTUM, a.n), sm = fix_scale(a.fixb + FIXB_MASS, a.n);
     const FixTile none{nullptr, 0, {0, 0, 0}, 0};
-    for (int item = first_warp(); item < nit; item = next_item<MODE>(item, nit))
-        p2g_item<GENERAL, MODE, DET, false>(a, item, sp, sm, none);
+    for (int item = first_warp(); item < nit; item += warp_count()) p2g_item<GENERAL, false>(a, item, sp, sm, none);
 }
 
 // G_op in place: (p, m) -> (v, m), v = p/m + dt f where |m| > FLT_EPSILON, else 0
@@ -608,65 +543,36 @@ template <bool EXACT> __global__ void __launch_bounds__(256) k_adj_sources(WArgs
     fix_bound(a.fixb + FIXB_ADJ, c * 1.001f);
 }
 
-// Warp items first, first + stride, ... below end of the adjoint scatter.
-// DET: the sources come from k_adj_sources (adjn) and the node sums go to
-// a.fix as integers (fixpoint.cuh) instead of float atomics into a.gadj; with a
-// tile, those of an item whose stencil lies in it go to the tile's
-// shared-memory integers.
-template <bool EXACT, bool GENERAL, int MODE, bool DET, bool TILE>
+// Warp items first, first + stride, ... below end of the deterministic mode's
+// adjoint scatter: the sources come from k_adj_sources (adjn), the node sums go
+// to a.fix as integers (fixpoint.cuh) or, with a tile, those of an item whose
+// stencil lies in it to the tile's shared-memory integers.
+template <bool GENERAL, bool TILE>
 __device__ __forceinline__ void adj_scatter_items(const WArgs& a, int first, int end, int stride, const FixScale& sa,
                                                   const FixTile& ft) {
     const size_t np = a.np, npl = a.npl;
     for (int item = first; item < end; item += stride) {
-        GridGeom geo;
-        int goff;
-        item_grid<MODE>(a, item, geo, goff);
+        const GridGeom& geo = a.geo;
         const ItemLane L = item_lane(a.items, item);
         const int p = L.p;
         float t[3];
         int base[3];
         load_x_base(a.st, npl, p, geo, t, base, a.xlo);
         const bool uniform = !GENERAL && warp_uniform_base(base);
-        const ScatterPerm P = scatter_perm();  // as in k_p2g_w
+        const ScatterPerm P = scatter_perm();  // as in p2g_item
         LaneW w;
         float own1[3];
         lane_weights_k(t, geo, L.s, w, own1, false, P.kp);
         float vn[3];
-        m3<float> Cn;
-        if constexpr (DET) {
 #pragma unroll
-            for (int c = 0; c < 3; c++) vn[c] = a.adjn[(size_t)c * np + p];
-            Cn = load_m3(a.adjn + 3 * np, np, p);
-        } else {
-            const size_t npn = a.npn;
-#pragma unroll
-            for (int c = 0; c < 3; c++)
-                vn[c] = a.dt * a.adj_next[(size_t)(PX + c) * npn + p] + a.adj_next[(size_t)(PV + c) * npn + p];
-            const m3<float> Fe = fe_from_strain(load_m3(a.st + (size_t)PF * npl, npl, p), load_m3(a.dfc, np, p));
-            const float cf = EXACT ? (1.f - a.s) * a.dt : a.dt;
-            Cn = (cf * load_m3(a.adj_next + (size_t)PF * npn, npn, p)) * transpose(Fe) +
-                 load_m3(a.adj_next + (size_t)PC * npn, npn, p);
-        }
-        if (!DET && L.valid) {
-            if (L.s == 0) {
-#pragma unroll
-                for (int c = 0; c < 3; c++) a.adjn[(size_t)c * np + p] = vn[c];
-                if (a.dbg_vnext) {
-#pragma unroll
-                    for (int c = 0; c < 3; c++) a.dbg_vnext[(size_t)c * np + p] = vn[c];
-                }
-            } else if (L.s == 1) {
-                store_m3(a.adjn + 3 * np, np, p, Cn);
-                if (a.dbg_Cnext) store_m3(a.dbg_Cnext, np, p, Cn);
-            }
-        }
+        for (int c = 0; c < 3; c++) vn[c] = a.adjn[(size_t)c * np + p];
+        const m3<float> Cn = load_m3(a.adjn + 3 * np, np, p);
         const float dx = (float)geo.dx;
         const float k3 = 3.f / (dx * dx);
         float c0[3];
 #pragma unroll
         for (int r = 0; r < 3; r++) c0[r] = k3 * Cn.a[r][0] * w.d0;
-        LaneNodes N = lane_nodes(geo, base, L.s);
-        N.g00 += goff;
+        const LaneNodes N = lane_nodes(geo, base, L.s);
         const int tile_l = TILE && uniform ? fix_tile_offset(ft, base) : -1;
 #pragma unroll
         for (int half = 0; half < 2; half++) {
@@ -693,19 +599,15 @@ __device__ __forceinline__ void adj_scatter_items(const WArgs& a, int first, int
                 if (((N.mask >> (4 * j + k)) & 1u) && (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f)) {
                     if (TILE && tile_l >= 0)
                         fix_red4_tile(ft, tile_l + (L.s * ft.E + j) * ft.E + k, v[0], v[1], v[2], 0.f, sa.s, sa.s);
-                    else if (DET) fix_red4(a.fix + (N.g00 + j * N.sj + k), v[0], v[1], v[2], 0.f, sa.s, sa.s);
-                    else red_add4(a.gadj + (N.g00 + j * N.sj + k), v[0], v[1], v[2], 0.f);
+                    else
+                        fix_red4(a.fix + (N.g00 + j * N.sj + k), v[0], v[1], v[2], 0.f, sa.s, sa.s);
                 }
             } else if (L.valid) {
 #pragma unroll
                 for (int nd = 0; nd < 8; nd++) {
                     const int j = 2 * half + ((nd >> 2) ^ P.jp), k = (nd & 3) ^ P.kp;
                     if (!((N.mask >> (4 * j + k)) & 1u)) continue;
-                    if (DET)
-                        fix_red4(a.fix + (N.g00 + j * N.sj + k), v[nd * 3], v[nd * 3 + 1], v[nd * 3 + 2], 0.f, sa.s,
-                                 sa.s);
-                    else
-                        red_add4(a.gadj + (N.g00 + j * N.sj + k), v[nd * 3], v[nd * 3 + 1], v[nd * 3 + 2], 0.f);
+                    fix_red4(a.fix + (N.g00 + j * N.sj + k), v[nd * 3], v[nd * 3 + 1], v[nd * 3 + 2], 0.f, sa.s, sa.s);
                 }
             }
         }
@@ -713,14 +615,11 @@ __device__ __forceinline__ void adj_scatter_items(const WArgs& a, int first, int
 }
 
 // adjoint scatter over warp items (one item per warp, persistent grid-stride)
-template <bool EXACT, bool GENERAL, int MODE, bool DET = false>
+template <bool GENERAL>
 __global__ void __launch_bounds__(DMPM_ADJ_SCATTER_THREADS, DMPM_ADJ_SCATTER_MIN_BLOCKS) k_adj_scatter_w(WArgs a) {
-    const int nit = item_count(a);
-    FixScale sa{1.f, 1.f};
-    if (DET) sa = fix_scale(a.fixb + FIXB_ADJ, a.n);
+    const FixScale sa = fix_scale(a.fixb + FIXB_ADJ, a.n);
     const FixTile none{nullptr, 0, {0, 0, 0}, 0};
-    const int stride = MODE != ITEMS_PER_WARP ? (int)((gridDim.x * blockDim.x) >> 5) : nit;  // as next_item
-    adj_scatter_items<EXACT, GENERAL, MODE, DET, false>(a, first_warp(), nit, stride, sa, none);
+    adj_scatter_items<GENERAL, false>(a, first_warp(), (int)*a.n_items_dev, warp_count(), sa, none);
 }
 
 // adjoint G_op per node: (dLdp, dLdm) from dLdv and the layer's (v, m)

@@ -1,5 +1,6 @@
-// sort.cuh -- stable LSD radix sort of (cell key, particle index) pairs, the
-// scans it needs, and the grouping of sorted particles into warp items.
+// sort.cuh -- the cell sort: a counting sort for the order alone, a stable LSD
+// radix sort of (cell key, particle index) pairs with the scans it needs, and the
+// grouping of sorted particles into warp items.
 //
 // Cell key of a particle: the cell holding it, from the reference's
 // floor((x - min) / dx) by division (ForwardSimulation.cpp:19), shifted so that
@@ -12,7 +13,7 @@
 //   morton = (l_0>>1) 32 + (l_1>>1) 16 + (l_2>>1) 8 + (l_0&1) 4 + (l_1&1) 2 + (l_2&1).
 // So the particles of one cell (a run of equal keys), of one 2 x 2 x 2 octant
 // of a brick (equal key >> 3) and of one brick (equal key >> 6) are contiguous
-// in the sorted order.  Sorting is stable, so equal keys keep their index
+// in the sorted order.  The radix sort is stable, so equal keys keep their index
 // order and the permutation equals a CPU std::stable_sort / numpy
 // argsort(kind="stable") of the keys.
 //
@@ -78,9 +79,7 @@ DMPM_HD void unit_first_cell(uint32_t key_hi, int shift, const int dim[3], int c
     c[2] = (int)(4u * b2 + (((m >> 3) & 1u) << 1) + (m & 1u));
 }
 
-template <class T> __global__ void k_cell_keys(KeyArgs<T> a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.n) return;
+template <class T> __device__ __forceinline__ uint32_t particle_key(const KeyArgs<T>& a, int p) {
     int base[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
@@ -89,7 +88,12 @@ template <class T> __global__ void k_cell_keys(KeyArgs<T> a) {
         else
             base[c] = stencil_base<T>(a.st[(size_t)(PX + c) * a.np + p] - (T)a.geo.mn[c], (T)a.geo.dx, a.geo.dim[c]);
     }
-    a.keys[p] = cell_key(base, a.geo.dim);
+    return cell_key(base, a.geo.dim);
+}
+template <class T> __global__ void k_cell_keys(KeyArgs<T> a) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.n) return;
+    a.keys[p] = particle_key(a, p);
     a.vals[p] = (uint32_t)p;
 }
 
@@ -252,6 +256,86 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const uint32
             vals_out[pos] = val[r];
         }
     }
+}
+
+// ------------------------------------------------------------------ counting sort
+// The order alone, without the keys' own order being stable: particles counted
+// per cell (k_cell_count gives each its rank in the cell), the counts scanned,
+// every particle written to its place -- 5 launches, where the radix sort takes 5
+// per digit and the items and units another 14.  Within a cell the particles of
+// one warp keep their order and the warps come as their atomics do, so two runs
+// may order a cell differently; the sums over a cell are float atomics anyway.
+// The deterministic mode and dmpm_cell_sort take the stable radix sort.
+// On 79k particles of a 64 x 60 x 53 grid the radix sort with items and units
+// took 160 us of kernels, 20 us a step when sorting every 8 steps.
+constexpr int COUNT_ITEMS = 16;
+constexpr int COUNT_TILE = SCAN_THREADS * COUNT_ITEMS;
+// The counting sort clears and scans a counter per key, so it serves grids of at
+// most this many keys per particle (beyond, the radix sort's passes over the
+// particles cost less) and below 4M keys (16 MB) any.
+inline bool counting_sort_fits(uint64_t keys, size_t n) {
+    return keys <= (1u << 22) || (keys <= 32ull * n && keys < (1ull << 31));
+}
+inline size_t count_tiles(uint64_t keys) { return (size_t)((keys + COUNT_TILE - 1) / COUNT_TILE); }
+
+// the rank of this lane's particle among those counted under its key so far;
+// every lane of the warp calls it
+__device__ __forceinline__ uint32_t count_rank(uint32_t key, bool valid, uint32_t* count) {
+    const int lane = threadIdx.x & 31;
+    const unsigned vm = __ballot_sync(0xffffffffu, valid);
+    const unsigned m = __match_any_sync(0xffffffffu, key) & vm;
+    const unsigned before = m & ((1u << lane) - 1u);
+    uint32_t base = 0;
+    if (valid && !before) base = atomicAdd(count + key, (uint32_t)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, m ? __ffs(m) - 1 : 0);
+    return base + (uint32_t)__popc(before);
+}
+template <class T> __global__ void k_cell_count(KeyArgs<T> a, uint32_t* count) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = p < a.n;
+    const uint32_t key = valid ? particle_key(a, p) : 0xffffffffu;
+    const uint32_t r = count_rank(key, valid, count);
+    if (!valid) return;
+    a.keys[p] = key;
+    a.vals[p] = r;
+}
+// counts -> exclusive sums within each tile of COUNT_TILE keys (the array is
+// padded to whole tiles), and the tiles' totals
+static __global__ void __launch_bounds__(SCAN_THREADS) k_count_scan(uint32_t* count, uint32_t* totals) {
+    uint4* c4 = reinterpret_cast<uint4*>(count + (size_t)blockIdx.x * COUNT_TILE) + threadIdx.x * (COUNT_ITEMS / 4);
+    uint4 v[COUNT_ITEMS / 4];
+    uint32_t acc = 0;
+#pragma unroll
+    for (int i = 0; i < COUNT_ITEMS / 4; i++) {
+        v[i] = c4[i];
+        acc += v[i].x + v[i].y + v[i].z + v[i].w;
+    }
+    uint32_t total;
+    uint32_t run = block_exclusive_scan<OpSum>(acc, total);
+#pragma unroll
+    for (int i = 0; i < COUNT_ITEMS / 4; i++) {
+        const uint4 o = make_uint4(run, run + v[i].x, run + v[i].x + v[i].y, run + v[i].x + v[i].y + v[i].z);
+        run = o.w + v[i].w;
+        c4[i] = o;
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = total;
+}
+// totals: exclusive sums over the tiles (k_scan_totals)
+static __global__ void k_count_order(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ rank,
+                                     const uint32_t* __restrict__ count, const uint32_t* __restrict__ totals, int n,
+                                     uint32_t* order) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const uint32_t k = keys[p];
+    order[totals[k / COUNT_TILE] + count[k] + rank[p]] = (uint32_t)p;
+}
+// scan and order on st, after the counting kernel
+inline void launch_count_order(const uint32_t* keys, const uint32_t* rank, uint32_t* count, uint32_t* totals,
+                               uint64_t key_count, int n, uint32_t* order, cudaStream_t st) {
+    const int tiles = (int)count_tiles(key_count);
+    k_count_scan<<<tiles, SCAN_THREADS, 0, st>>>(count, totals);
+    k_scan_totals<OpSum><<<1, 1024, 0, st>>>(totals, tiles, nullptr);
+    k_count_order<<<(n + 255) / 256, 256, 0, st>>>(keys, rank, count, totals, n, order);
 }
 
 // ------------------------------------------------------------------ warp items
