@@ -7,11 +7,21 @@
 // (s = 1 - 2 w, S = s |d|; points exactly on the surface are left out here,
 // see the header).
 //
-// One thread per lattice point sums the solid angles of all triangles in
-// FP64 -- each by the formula of Van Oosterom and Strackee (1983),
-// tan(Omega / 2) = a.(b x c) / (|a||b||c| + (a.b)|c| + (b.c)|a| + (c.a)|b|)
-// with a, b, c the triangle's vertices relative to the point -- reading the
-// triangles in tiles staged in shared memory by the whole block.  The lattice
+// One thread per lattice point sums the solid angles of the mesh in FP64 -- a
+// triangle's by the formula of Van Oosterom and Strackee (1983),
+// tan(Omega / 2) = det / den, det = a.(b x c),
+// den = |a||b||c| + (a.b)|c| + (b.c)|a| + (c.a)|b|,
+// with a, b, c its vertices relative to the point.
+//   The half angles are summed as the product of the complex numbers den + i det,
+// with a count of the times it passes the negative real axis: one atan2 per point
+// in place of one per triangle, whose FP64 instructions were the kernel's cost.
+//   The triangles are cut into patches.  A surface's solid angle from a point is
+// that of any surface with the same boundary that the point is not between, so a
+// patch is summed triangle by triangle only for warps with a point in its bounding
+// box; for all others by the fan over its boundary edges from one of its
+// vertices, which lies in the box too (Jacobson, Kavan and Sorkine-Hornung 2013).
+// The fan has about 4 sqrt(triangles) triangles, each with one new vertex.
+//   The kept points are compacted on the GPU in lattice order.  The lattice
 // coordinates are formed in float with the reference's two roundings.
 //
 // dmpm_mesh_jittered_points uses the same inside test for jittered stratified
@@ -20,16 +30,26 @@
 // depend only on the seed and the sub-cell, not on the launch.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <array>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <numeric>
+#include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "dmpm.h"
+#include "sort.cuh"
 
 namespace {
 
-constexpr int kTriTile = 256;
+// triangles per patch, at most: at 1,152 triangles 64 makes 18 patches of about 25
+// boundary edges
+constexpr int kPatchTriangles = 64;
 
 // the lattice point min_point + sampling_dx * (i, j, k): a product and a sum, each rounded to float
 struct LatticePoints {
@@ -65,39 +85,125 @@ struct JitteredPoints {
     }
 };
 
+// One patch: its triangles [t0, t1), its boundary fan's edges [e0, e1) around
+// apex, and its bounding box.  e0 = e1 and far = 0: no cheaper fan.
+struct Patch {
+    float lo[3], hi[3], apex[3];
+    int t0, t1, e0, e1, far;
+};
+
+struct Vec {
+    double x, y, z;
+};
+__device__ __forceinline__ Vec rel(const float* v, const double p[3]) { return Vec{v[0] - p[0], v[1] - p[1], v[2] - p[2]}; }
+__device__ __forceinline__ double dot(const Vec& a, const Vec& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+
+// The sum of half solid angles as arg(re + i im) + 2 pi turns, arg in [-pi, pi]
+// with atan2's signs at the cut.
+struct AngleSum {
+    double re = 1.0, im = 0.0;
+    int turns = 0;
+    // add atan2(det, den)
+    __device__ __forceinline__ void add(double det, double den) {
+        if (det == 0.0 && den == 0.0) return;  // atan2 gives 0 (or -0)
+        const double r = re * den - im * det, i = re * det + im * den;
+        const bool up = !signbit(im) && !signbit(det) && signbit(i), down = signbit(im) && signbit(det) && !signbit(i);
+        turns += (up ? 1 : 0) - (down ? 1 : 0);
+        re = r;
+        im = i;
+        const double m = fabs(re) + fabs(im);
+        if (!(m > 1e-100 && m < 1e100)) {  // rescale; exact, and NaN stays NaN
+            const int e = -ilogb(m);
+            if (m > 0.0 && m < 1e308) {
+                re = scalbn(re, e);
+                im = scalbn(im, e);
+            }
+        }
+    }
+    __device__ __forceinline__ double value() const { return 2.0 * M_PI * turns + atan2(im, re); }
+};
+
+// mask: a bit per point, count: points kept by each block of 256
 template <class Points>
-__global__ void __launch_bounds__(256) k_mesh_winding(const float* __restrict__ tri, int nf, Points pts, int d0, int d1,
-                                                      int d2, uint8_t* __restrict__ inside) {
-    __shared__ float s_tri[kTriTile * 9];
+__global__ void __launch_bounds__(256) k_mesh_winding(const float* __restrict__ tri, const float* __restrict__ edges,
+                                                      const Patch* __restrict__ patches, int np, Points pts, int d0,
+                                                      int d1, int d2, uint32_t* __restrict__ mask,
+                                                      uint32_t* __restrict__ count) {
     const long long total = (long long)d0 * d1 * d2;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = idx < total;
-    const long long q = valid ? idx : 0;
+    const long long q = valid ? idx : total - 1;
     const int i = (int)(q / ((long long)d1 * d2)), j = (int)((q / d2) % d1), k = (int)(q % d2);
-    double P[3];
-    pts(i, j, k, P);
-    const double px = P[0], py = P[1], pz = P[2];
-    double ang = 0.0;
-    for (int t0 = 0; t0 < nf; t0 += kTriTile) {
-        const int cnt = min(kTriTile, nf - t0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < cnt * 9; e += blockDim.x) s_tri[e] = tri[(size_t)t0 * 9 + e];
-        __syncthreads();
-        if (!valid) continue;
-        for (int t = 0; t < cnt; t++) {
-            const float* v = s_tri + 9 * t;
-            const double ax = v[0] - px, ay = v[1] - py, az = v[2] - pz;
-            const double bx = v[3] - px, by = v[4] - py, bz = v[5] - pz;
-            const double cx = v[6] - px, cy = v[7] - py, cz = v[8] - pz;
-            const double la = sqrt(ax * ax + ay * ay + az * az), lb = sqrt(bx * bx + by * by + bz * bz),
-                         lc = sqrt(cx * cx + cy * cy + cz * cz);
-            const double det = ax * (by * cz - bz * cy) - ay * (bx * cz - bz * cx) + az * (bx * cy - by * cx);
-            const double den = la * lb * lc + (ax * bx + ay * by + az * bz) * lc + (bx * cx + by * cy + bz * cz) * la +
-                               (cx * ax + cy * ay + cz * az) * lb;
-            ang += atan2(det, den);  // Omega / 2
+    double p[3];
+    pts(i, j, k, p);
+    AngleSum sum;
+    for (int n = 0; n < np; n++) {
+        const Patch& P = patches[n];
+        bool near = !P.far;
+        if (P.far) {
+            bool in = true;
+#pragma unroll
+            for (int a = 0; a < 3; a++) in &= p[a] >= (double)P.lo[a] && p[a] <= (double)P.hi[a];
+            near = __any_sync(0xffffffffu, in || !(p[0] == p[0]));
+        }
+        if (near) {
+            for (int t = P.t0; t < P.t1; t++) {
+                const float* v = tri + 9 * (size_t)t;
+                const double ax = v[0] - p[0], ay = v[1] - p[1], az = v[2] - p[2];
+                const double bx = v[3] - p[0], by = v[4] - p[1], bz = v[5] - p[2];
+                const double cx = v[6] - p[0], cy = v[7] - p[1], cz = v[8] - p[2];
+                const double la = sqrt(ax * ax + ay * ay + az * az), lb = sqrt(bx * bx + by * by + bz * bz),
+                             lc = sqrt(cx * cx + cy * cy + cz * cz);
+                const double det = ax * (by * cz - bz * cy) - ay * (bx * cz - bz * cx) + az * (bx * cy - by * cx);
+                const double den = la * lb * lc + (ax * bx + ay * by + az * bz) * lc +
+                                   (bx * cx + by * cy + bz * cz) * la + (cx * ax + cy * ay + cz * az) * lb;
+                sum.add(det, den);
+            }
+        } else {
+            const Vec a = rel(P.apex, p);
+            const double la = sqrt(dot(a, a));
+            Vec c{0.0, 0.0, 0.0};
+            double lc = 0.0, ca = 0.0;
+            for (int e = P.e0; e < P.e1; e++) {  // (apex, b, c) with c carried over where the edges chain
+                const float* v = edges + 7 * (size_t)e;
+                Vec b = c;
+                double lb = lc, ab = ca;
+                if (v[6] == 0.f) {
+                    b = rel(v, p);
+                    lb = sqrt(dot(b, b));
+                    ab = dot(a, b);
+                }
+                c = rel(v + 3, p);
+                lc = sqrt(dot(c, c));
+                ca = dot(c, a);
+                const double det = a.x * (b.y * c.z - b.z * c.y) - a.y * (b.x * c.z - b.z * c.x) + a.z * (b.x * c.y - b.y * c.x);
+                sum.add(det, la * lb * lc + ab * lc + dot(b, c) * la + ca * lb);
+            }
         }
     }
-    if (valid) inside[idx] = (ang / (2.0 * M_PI) >= 0.5) ? 1 : 0;  // w = sum Omega / (4 pi)
+    const bool keep = valid && sum.value() / (2.0 * M_PI) >= 0.5;  // w = sum Omega / (4 pi)
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if ((threadIdx.x & 31) == 0) mask[idx >> 5] = m;
+    const int kept = __syncthreads_count(keep);
+    if (threadIdx.x == 0) count[blockIdx.x] = (uint32_t)kept;
+}
+
+// the kept points in lattice order: first[b] = points kept by the blocks before b
+template <class Points>
+__global__ void __launch_bounds__(256) k_mesh_compact(const uint32_t* __restrict__ mask,
+                                                      const uint32_t* __restrict__ first, Points pts, int d0, int d1,
+                                                      int d2, long long capacity, float* __restrict__ out) {
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t m = mask[idx >> 5];
+    long long o = first[blockIdx.x];
+    for (int u = 0; u < w; u++) o += __popc(mask[(idx >> 5) - w + u]);
+    o += __popc(m & ((1u << lane) - 1u));
+    if (!((m >> lane) & 1u) || o >= capacity) return;
+    const int i = (int)(idx / ((long long)d1 * d2)), j = (int)((idx / d2) % d1), k = (int)(idx % d2);
+    double p[3];
+    pts(i, j, k, p);
+    for (int a = 0; a < 3; a++) out[3 * o + a] = (float)p[a];  // a float value: exact
 }
 
 // triangles gathered as 9 floats each, indices checked
@@ -112,33 +218,176 @@ int gather_triangles(const float* V, int nv, const int* F, int nf, std::vector<f
     return DMPM_OK;
 }
 
-// the inside mask of d0 x d1 x d2 generated points on the GPU
+// The triangles in patches of at most kPatchTriangles, split at the median
+// centroid of the longest axis, and each patch's boundary edges: 7 floats each, the
+// two ends and 1 where the first end is the edge before's second (the edges are
+// chained as far as they go).
+struct Mesh {
+    std::vector<float> tri, edges;
+    std::vector<Patch> patches;
+};
+void make_patches(const std::vector<float>& tri, int nf, Mesh& m) {
+    // vertices by position, so that unwelded meshes have inner edges too
+    auto hash = [](const std::array<float, 3>& x) {
+        uint32_t u[3];
+        std::memcpy(u, x.data(), sizeof u);
+        return (size_t)splitmix64(((uint64_t)u[0] << 32 | u[1]) ^ splitmix64(u[2]));
+    };
+    std::unordered_map<std::array<float, 3>, int, decltype(hash)> ids((size_t)nf * 2, hash);
+    std::vector<int> vid((size_t)nf * 3);
+    for (size_t v = 0; v < vid.size(); v++) {
+        const float* x = &tri[3 * v];
+        const std::array<float, 3> key{x[0] + 0.f, x[1] + 0.f, x[2] + 0.f};  // -0 + 0 = 0
+        if (!(std::isfinite(x[0]) && std::isfinite(x[1]) && std::isfinite(x[2]))) {
+            vid[v] = -1 - (int)v;  // its own vertex: NaN has no order
+            continue;
+        }
+        vid[v] = ids.emplace(key, (int)ids.size()).first->second;
+    }
+    std::vector<int> order(nf);
+    std::iota(order.begin(), order.end(), 0);
+    auto centre = [&](int f, int a) { return tri[9 * (size_t)f + a] + tri[9 * (size_t)f + 3 + a] + tri[9 * (size_t)f + 6 + a]; };
+    std::vector<std::pair<int, int>> todo{{0, nf}};
+    while (!todo.empty()) {
+        const auto [b, e] = todo.back();
+        todo.pop_back();
+        Patch P{};
+        for (int a = 0; a < 3; a++) {
+            P.lo[a] = INFINITY;
+            P.hi[a] = -INFINITY;
+        }
+        bool finite = true;
+        for (int i = b; i < e; i++)
+            for (int c = 0; c < 9; c++) {
+                const float x = tri[9 * (size_t)order[i] + c];
+                finite &= std::isfinite(x);
+                P.lo[c % 3] = std::min(P.lo[c % 3], x);
+                P.hi[c % 3] = std::max(P.hi[c % 3], x);
+            }
+        if (finite && e - b > kPatchTriangles) {
+            int axis = 0;
+            for (int a = 1; a < 3; a++)
+                if (P.hi[a] - P.lo[a] > P.hi[axis] - P.lo[axis]) axis = a;
+            const int mid = b + (e - b) / 2;
+            std::nth_element(order.begin() + b, order.begin() + mid, order.begin() + e,
+                             [&](int f, int g) { return centre(f, axis) < centre(g, axis); });
+            todo.push_back({mid, e});
+            todo.push_back({b, mid});
+            continue;
+        }
+        P.t0 = (int)(m.tri.size() / 9);
+        std::map<std::pair<int, int>, int> net;  // directed edges that no opposite one cancels
+        std::map<int, const float*> at;
+        for (int i = b; i < e; i++) {
+            const size_t f = (size_t)order[i];
+            m.tri.insert(m.tri.end(), tri.begin() + 9 * f, tri.begin() + 9 * f + 9);
+            for (int c = 0; c < 3; c++) {
+                const int u = vid[3 * f + c], v = vid[3 * f + (c + 1) % 3];
+                at[u] = &tri[9 * f + 3 * c];
+                if (u == v) continue;
+                const auto back = net.find({v, u});
+                if (back == net.end()) net[{u, v}]++;
+                else if (--back->second == 0) net.erase(back);
+            }
+        }
+        P.t1 = (int)(m.tri.size() / 9);
+        int left = 0;
+        for (const auto& n : net) left += n.second;
+        // a fan triangle costs about half a triangle of its own
+        P.far = finite && left < 2 * (P.t1 - P.t0) ? 1 : 0;
+        P.e0 = (int)(m.edges.size() / 7);
+        if (P.far && left > 0) {
+            const int apex = net.begin()->first.first;
+            std::copy(at[apex], at[apex] + 3, P.apex);
+            int prev = -1;
+            bool chained = false;
+            while (!net.empty()) {
+                auto it = chained ? net.lower_bound({prev, INT_MIN}) : net.begin();
+                if (chained && (it == net.end() || it->first.first != prev)) {
+                    chained = false;
+                    continue;
+                }
+                const auto [u, v] = it->first;
+                if (--it->second == 0) net.erase(it);
+                if (u != apex && v != apex) {  // an edge at the apex spans no triangle
+                    const bool follows = chained && m.edges.size() / 7 > (size_t)P.e0 &&
+                                         std::equal(at[u], at[u] + 3, &m.edges[m.edges.size() - 4]);
+                    m.edges.insert(m.edges.end(), at[u], at[u] + 3);
+                    m.edges.insert(m.edges.end(), at[v], at[v] + 3);
+                    m.edges.push_back(follows ? 1.f : 0.f);
+                }
+                prev = v;
+                chained = true;
+            }
+        }
+        P.e1 = (int)(m.edges.size() / 7);
+        m.patches.push_back(P);
+    }
+}
+
+// device memory of one call
+struct DeviceMem {
+    std::vector<void*> ptrs;
+    ~DeviceMem() {
+        for (void* p : ptrs) cudaFree(p);
+    }
+    template <class T> T* alloc(size_t count) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, std::max<size_t>(1, count) * sizeof(T)) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        ptrs.push_back(p);
+        return (T*)p;
+    }
+};
+int cuda_failed() {
+    cudaGetLastError();
+    return DMPM_ERR_CUDA;
+}
+
+// the points of the d0 x d1 x d2 generated ones that lie inside, in order: all
+// counted, the first `capacity` of them written to out
 template <class Points>
-int inside_mask(const std::vector<float>& tri, int nf, const Points& pts, const int dims[3], std::vector<uint8_t>& mask) {
+int inside_points(const std::vector<float>& tri, int nf, const Points& pts, const int dims[3], float* out,
+                  int64_t capacity, int64_t* count) {
+    using namespace dmpm;
     const long long total = (long long)dims[0] * dims[1] * dims[2];
-    float* dtri = nullptr;
-    uint8_t* dmask = nullptr;
-    if (cudaMalloc(&dtri, tri.size() * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&dmask, (size_t)total) != cudaSuccess) {
-        cudaFree(dtri);
-        cudaGetLastError();
-        return DMPM_ERR_OOM;
-    }
-    mask.resize((size_t)total);
-    int rc = DMPM_OK;
-    if (cudaMemcpy(dtri, tri.data(), tri.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
-        rc = DMPM_ERR_CUDA;
-    } else {
-        const unsigned blocks = (unsigned)((total + 255) / 256);
-        k_mesh_winding<Points><<<blocks, 256>>>(dtri, nf, pts, dims[0], dims[1], dims[2], dmask);
+    Mesh m;
+    make_patches(tri, nf, m);
+    const unsigned blocks = (unsigned)((total + 255) / 256);
+    const int tiles = (int)((blocks + SCAN_TILE - 1) / SCAN_TILE);
+    DeviceMem mem;
+    float* dtri = mem.alloc<float>(m.tri.size() + m.edges.size());
+    Patch* dpat = mem.alloc<Patch>(m.patches.size());
+    uint32_t* dmask = mem.alloc<uint32_t>((size_t)blocks * 9 + tiles + 2);
+    if (!dtri || !dpat || !dmask) return DMPM_ERR_OOM;
+    float* dedge = dtri + m.tri.size();
+    uint32_t *dcount = dmask + (size_t)blocks * 8, *dtot = dcount + blocks, *dgrand = dtot + tiles;
+    if (cudaMemcpy(dtri, m.tri.data(), m.tri.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
+        (!m.edges.empty() &&
+         cudaMemcpy(dedge, m.edges.data(), m.edges.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) ||
+        cudaMemcpy(dpat, m.patches.data(), m.patches.size() * sizeof(Patch), cudaMemcpyHostToDevice) != cudaSuccess)
+        return cuda_failed();
+    k_mesh_winding<Points><<<blocks, 256>>>(dtri, dedge, dpat, (int)m.patches.size(), pts, dims[0], dims[1], dims[2],
+                                            dmask, dcount);
+    k_scan_tiles<OpSum><<<tiles, SCAN_THREADS>>>(dcount, (int)blocks, dtot);
+    k_scan_totals<OpSum><<<1, 1024>>>(dtot, tiles, dgrand);
+    k_scan_add<OpSum><<<tiles, SCAN_THREADS>>>(dcount, (int)blocks, dtot);
+    uint32_t n = 0;
+    if (cudaGetLastError() != cudaSuccess || cudaMemcpy(&n, dgrand, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+        return cuda_failed();
+    *count = n;
+    const int64_t write = std::min<int64_t>(n, capacity);
+    if (write > 0) {
+        float* dout = mem.alloc<float>((size_t)write * 3);
+        if (!dout) return DMPM_ERR_OOM;
+        k_mesh_compact<Points><<<blocks, 256>>>(dmask, dcount, pts, dims[0], dims[1], dims[2], write, dout);
         if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpy(mask.data(), dmask, (size_t)total, cudaMemcpyDeviceToHost) != cudaSuccess)
-            rc = DMPM_ERR_CUDA;
+            cudaMemcpy(out, dout, (size_t)write * 12, cudaMemcpyDeviceToHost) != cudaSuccess)
+            return cuda_failed();
     }
-    cudaFree(dtri);
-    cudaFree(dmask);
-    if (rc != DMPM_OK) cudaGetLastError();
-    return rc;
+    return (int64_t)n > capacity ? DMPM_ERR_TOO_LARGE : DMPM_OK;
 }
 
 }  // namespace
@@ -166,24 +415,7 @@ extern "C" int dmpm_mesh_lattice_points(const float* V, int nv, const int* F, in
     std::vector<float> tri;
     if ((st = gather_triangles(V, nv, F, nf, tri)) != DMPM_OK) return st;
     LatticePoints pts{{min_point[0], min_point[1], min_point[2]}, sampling_dx};
-    std::vector<uint8_t> mask;
-    if ((st = inside_mask(tri, nf, pts, dims, mask)) != DMPM_OK) return st;
-    // kept points in the reference's lattice order, coordinates rounded as it rounds them
-    int64_t n = 0;
-    for (long long q = 0; q < total; q++) {
-        if (!mask[(size_t)q]) continue;
-        if (n < capacity) {
-            const int i = (int)(q / ((long long)dims[1] * dims[2])), j = (int)((q / dims[2]) % dims[1]),
-                      k = (int)(q % dims[2]);
-            volatile float t0 = sampling_dx * (float)i, t1 = sampling_dx * (float)j, t2 = sampling_dx * (float)k;
-            out[3 * n] = min_point[0] + t0;
-            out[3 * n + 1] = min_point[1] + t1;
-            out[3 * n + 2] = min_point[2] + t2;
-        }
-        n++;
-    }
-    *count = n;
-    return n > capacity ? DMPM_ERR_TOO_LARGE : DMPM_OK;
+    return inside_points(tri, nf, pts, dims, out, capacity, count);
 }
 
 extern "C" int dmpm_mesh_jittered_points(const float* V, int nv, const int* F, int nf, const float* min_point,
@@ -205,22 +437,5 @@ extern "C" int dmpm_mesh_jittered_points(const float* V, int nv, const int* F, i
     if (st != DMPM_OK) return st;
     const float sdx = cell_dx / (float)per_axis;
     JitteredPoints pts{{min_point[0], min_point[1], min_point[2]}, sdx, dims[1], dims[2], seed};
-    std::vector<uint8_t> mask;
-    if ((st = inside_mask(tri, nf, pts, dims, mask)) != DMPM_OK) return st;
-    int64_t n = 0;
-    for (long long q = 0; q < total; q++) {
-        if (!mask[(size_t)q]) continue;
-        if (n < capacity) {
-            const long long id[3] = {q / ((long long)dims[1] * dims[2]), (q / dims[2]) % dims[1], q % dims[2]};
-            for (int a = 0; a < 3; a++) {
-                const float u = (float)(splitmix64(seed + 3 * (uint64_t)q + a) >> 40) * (1.f / 16777216.f);
-                volatile float s = (float)id[a] + u;
-                volatile float t = s * sdx;
-                out[3 * n + a] = min_point[a] + t;
-            }
-        }
-        n++;
-    }
-    *count = n;
-    return n > capacity ? DMPM_ERR_TOO_LARGE : DMPM_OK;
+    return inside_points(tri, nf, pts, dims, out, capacity, count);
 }
