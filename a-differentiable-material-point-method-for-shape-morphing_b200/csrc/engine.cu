@@ -21,6 +21,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <thread>
 #include <type_traits>
 #include <vector>
 
@@ -66,6 +67,38 @@ __global__ void k_unpack_ref(const float* __restrict__ pts, int n, size_t np, T*
     cst[(size_t)KLAM * np + p] = (T)m[35];
     cst[(size_t)KMU * np + p] = (T)m[36];
     for (int q = 0; q < 9; q++) dfc[(size_t)q * np + p] = (T)m[37 + q];
+}
+// The fields that the engine fills of one layer's reference MaterialPoints, W floats
+// per point in the caller's order: x v F C (24), m vol lam mu dFc (13) and, with adj,
+// dLdx dLdv dLdF dLdC (24) -- the floats 0-23 and 33-45 (-69) of the struct.
+constexpr int kRefState = 24, kRefFixed = 13, kRefFixedAt = 33, kRefFloats = 118;
+template <class T, bool STRAIN>
+__global__ void k_pack_ref(const T* __restrict__ st, const T* __restrict__ cst, const T* __restrict__ dfc,
+                           const T* __restrict__ adj, size_t np, int n, const uint32_t* __restrict__ perm, int W,
+                           float* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float* o = out + caller_index(perm, i) * W;
+    for (int c = 0; c < 3; c++) o[c] = (float)load_xd(st, np, i, c, STRAIN ? 1 : 0);
+    for (int q = 3; q < kRefState; q++) {
+        double v = (double)st[(size_t)q * np + i];
+        if (STRAIN && q >= PF && q < PC && (q - PF) % 4 == 0) v += 1.0;  // F = I + H
+        o[q] = (float)v;
+    }
+    o += kRefState;
+    for (int q = 0; q < NCONST; q++) o[q] = (float)cst[(size_t)q * np + i];
+    for (int q = 0; q < 9; q++) o[NCONST + q] = (float)dfc[(size_t)q * np + i];
+    if (adj)
+        for (int q = 0; q < NSTATE; q++) o[kRefFixed + q] = (float)adj[(size_t)q * np + i];
+}
+// rows [a, b) of W packed floats into the caller's structs
+inline void unpack_ref_rows(const float* rows, int W, size_t a, size_t b, float* pts) {
+    for (size_t p = a; p < b; p++) {
+        const float* r = rows + (p - a) * W;
+        float* d = pts + p * kRefFloats;
+        std::memcpy(d, r, kRefState * sizeof(float));
+        std::memcpy(d + kRefFixedAt, r + kRefState, (size_t)(W - kRefState) * sizeof(float));
+    }
 }
 // Grid fields of one layer.  The stored node holds (p, m), or, where the
 // FP32 path's grid update has overwritten p in place (stored_v), (v, m): then
@@ -1747,30 +1780,66 @@ template <class T> class Engine : public EngineBase {
         DMPM_CK(cudaStreamSynchronize(ctx_->stream));
     }
 
+    // One kernel packs the filled fields of every point, and the packed rows come
+    // through two pinned buffers, the next one's copy running while the host writes
+    // the last one's rows into the structs (on a few threads, as one core's stores
+    // are slower than the copy).  Field by field through double arrays, 79k points
+    // took 10.3 ms; 2 buffers of 4 MB serve any cloud.
     void get_points_ref(int l, void* pts) {
         if (!pts) throw ArgError{"points is NULL"};
-        float* mp = (float*)pts;
-        std::vector<double> buf((size_t)n_ * 9);
-        auto put = [&](int field, int off, int width) {
-            get_particles(l, field, buf.data());
-            for (int p = 0; p < n_; p++)
-                for (int q = 0; q < width; q++) mp[(size_t)p * 118 + off + q] = (float)buf[(size_t)p * width + q];
+        if (l < 0 || l >= L_) throw ArgError{"layer out of range"};
+        const T* adj = nullptr;
+        if (layers_[l].adj || l == backward_lo_ || (l == L_ - 1 && loss_done_)) adj = adj_of(l, false);
+        const int W = kRefState + kRefFixed + (adj ? (int)NSTATE : 0);
+        const T* st = materialize_state(l);
+        float* dev = (float*)staging(((size_t)n_ * W + 1) / 2);
+        k_pack_ref<T, kStrain><<<(unsigned)((n_ + 127) / 128), 128, 0, ctx_->stream>>>(st, cst_, layers_[l].dfc, adj, np_,
+                                                                                      n_, perm(), W, dev);
+        launched();
+        const size_t rows = std::min<size_t>((size_t)n_, ((size_t)4 << 20) / (W * sizeof(float)));
+        ensure_pinned(rows * W * sizeof(float));
+        auto copy = [&](size_t a, int b) {
+            const size_t cnt = std::min(rows, (size_t)n_ - a);
+            DMPM_CK(cudaMemcpyAsync(pin_[b], dev + a * W, cnt * W * sizeof(float), cudaMemcpyDeviceToHost, ctx_->stream));
+            DMPM_CK(cudaEventRecord(pin_ev_[b], ctx_->stream));
         };
-        put(DMPM_F_X, 0, 3);
-        put(DMPM_F_V, 3, 3);
-        put(DMPM_F_F, 6, 9);
-        put(DMPM_F_C, 15, 9);
-        put(DMPM_F_M, 33, 1);
-        put(DMPM_F_VOL, 34, 1);
-        put(DMPM_F_LAM, 35, 1);
-        put(DMPM_F_MU, 36, 1);
-        put(DMPM_F_DFC, 37, 9);
-        if (layers_[l].adj || l == backward_lo_ || (l == L_ - 1 && loss_done_)) {
-            put(DMPM_F_DLDX, 46, 3);
-            put(DMPM_F_DLDV, 49, 3);
-            put(DMPM_F_DLDF, 52, 9);
-            put(DMPM_F_DLDC, 61, 9);
+        int b = 0;
+        copy(0, 0);
+        for (size_t a = 0; a < (size_t)n_; a += rows, b ^= 1) {
+            if (a + rows < (size_t)n_) copy(a + rows, b ^ 1);
+            DMPM_CK(cudaEventSynchronize(pin_ev_[b]));
+            const size_t end = std::min((size_t)n_, a + rows);
+            const float* src = (const float*)pin_[b];
+            // threads for chunks above 1 MB: below, starting them costs more than it saves
+            const size_t bytes = (end - a) * W * sizeof(float);
+            const int extra = bytes > (1u << 20) ? (int)std::min<unsigned>(3, std::max(1u, std::thread::hardware_concurrency()) - 1) : 0;
+            const size_t part = (end - a + extra) / (extra + 1);
+            std::vector<std::thread> th;
+            th.reserve(3);
+            size_t done = std::min(end, a + part);  // this thread's share: the first part and what no thread took
+            try {
+                for (int t = 0; t < extra && done < end; t++) {
+                    const size_t to = std::min(end, done + part);
+                    th.emplace_back(unpack_ref_rows, src + (done - a) * W, W, done, to, (float*)pts);
+                    done = to;
+                }
+            } catch (...) {  // no more threads to be had
+            }
+            unpack_ref_rows(src, W, a, std::min(end, a + part), (float*)pts);
+            if (done < end) unpack_ref_rows(src + (done - a) * W, W, done, end, (float*)pts);
+            for (std::thread& t : th) t.join();
         }
+    }
+    void ensure_pinned(size_t bytes) {
+        if (bytes <= pin_bytes_) return;
+        for (int b = 0; b < 2; b++) {
+            if (pin_[b]) cudaFreeHost(pin_[b]);
+            pin_[b] = nullptr;
+            pin_bytes_ = 0;
+            if (!pin_ev_[b]) DMPM_CK(cudaEventCreateWithFlags(&pin_ev_[b], cudaEventDisableTiming));
+        }
+        for (int b = 0; b < 2; b++) DMPM_CK(cudaMallocHost(&pin_[b], bytes));
+        pin_bytes_ = bytes;
     }
 
     void info(int64_t* out, int count) const {
@@ -1789,6 +1858,10 @@ template <class T> class Engine : public EngineBase {
         harvest();
         for (cudaEvent_t e : event_pool_) cudaEventDestroy(e);
         if (host_misc_) cudaFreeHost(host_misc_);
+        for (int b = 0; b < 2; b++) {
+            if (pin_[b]) cudaFreeHost(pin_[b]);
+            if (pin_ev_[b]) cudaEventDestroy(pin_ev_[b]);
+        }
     }
 
    private:
@@ -1835,6 +1908,9 @@ template <class T> class Engine : public EngineBase {
     unsigned* fixb_ = nullptr;
     size_t fix_G_ = 0;
     void* host_misc_ = nullptr;
+    void* pin_[2] = {nullptr, nullptr};  // pinned buffers of get_points_ref
+    size_t pin_bytes_ = 0;
+    cudaEvent_t pin_ev_[2] = {nullptr, nullptr};
     int L_ = 0, k_ = 1;
     std::vector<LayerSlots> layers_;
     T* ring_[2] = {nullptr, nullptr};
