@@ -324,6 +324,7 @@ template <class T> class Engine : public EngineBase {
     void alloc_particles(int n) {
         if (n <= 0) throw ArgError{"particle count must be positive"};
         permuted_ = false;  // a new cloud arrives in the caller's order
+        boxes_fresh_ = false;
         if (n == n_ && cst_) {
             // same cloud size: overwrite in place and keep the layer storage
             DMPM_CK(cudaMemsetAsync(cst_, 0, NCONST * np_ * sizeof(T), ctx_->stream));
@@ -820,6 +821,7 @@ template <class T> class Engine : public EngineBase {
             node4<T>* gbase = (node4<T>*)layer_arena_.alloc((size_t)L_ * gr_bytes);
             for (int l = 0; l < L_; l++) layers_[l].grid = gbase + (size_t)l * G_;
         }
+        if (kWarp) alloc_boxes();
         // controls
         if (per_layer) {
             // control frames own a dFc copy and a gradient; the other layers read
@@ -898,12 +900,40 @@ template <class T> class Engine : public EngineBase {
         }
     }
 
+    // node boxes (kernels_warp.cuh): one per layer grid, then the whole grid's
+    void alloc_boxes() {
+        boxes_ = (int*)layer_arena_.alloc((size_t)(num_grids() + 1) * 6 * sizeof(int));
+        box_full_ = boxes_ + 6 * num_grids();
+        boxes_fresh_ = false;
+    }
+    int num_grids() const { return k_ == 1 ? L_ : k_; }
+    // all grids zero, all boxes empty
+    void reset_boxes() {
+        k_box_reset<<<(unsigned)((num_grids() + 1) * 6 + 255) / 256, 256, 0, ctx_->stream>>>(boxes_, num_grids(), geo_);
+        launched();
+        if (k_ == 1) DMPM_CK(cudaMemsetAsync(layers_[0].grid, 0, (size_t)L_ * G_ * sizeof(node4<T>), ctx_->stream));
+        else for (node4<T>* g : seg_grid_) DMPM_CK(cudaMemsetAsync(g, 0, G_ * sizeof(node4<T>), ctx_->stream));
+        boxes_fresh_ = true;
+    }
+    int* box_of(const node4<T>* g) const {
+        if (k_ == 1) return boxes_ + 6 * ((g - layers_[0].grid) / (ptrdiff_t)G_);
+        for (size_t i = 0; i < seg_grid_.size(); i++)
+            if (seg_grid_[i] == g) return boxes_ + 6 * i;
+        throw StateError{"internal: grid without a box"};
+    }
+    // blocks of a node-box kernel: a warp per row of the grid, at most 8 blocks of 256 per SM
+    unsigned box_blocks() {
+        if (sms_ == 0) warp_blocks();
+        return (unsigned)std::min<size_t>((size_t)sms_ * 8, ((size_t)geo_.dim[0] * geo_.dim[1] + 7) / 8);
+    }
+
     // SetUpCompGraph semantics on allocated storage: layer 0 = the uploaded
     // cloud, every layer's dFc = the uploaded dFc, gradients cleared.  Layer
     // states other than 0 are not copied: each is written by the forward pass
     // before anything reads it.
     void reset_layers() {
         if (ctx_->prm.reorder_particles && !permuted_) reorder_scene();
+        if (kWarp && !boxes_fresh_) reset_boxes();
         const size_t st_bytes = kNst * np_ * sizeof(T);
         DMPM_CK(cudaMemcpyAsync(layers_[0].st, st0_, st_bytes, cudaMemcpyDeviceToDevice, ctx_->stream));
         if (ctx_->prm.control_mode == DMPM_CTRL_PER_LAYER) {
@@ -1150,7 +1180,11 @@ template <class T> class Engine : public EngineBase {
                 a.fixb = fixb_;
                 clear_fix(-1);
             } else {
-                DMPM_CK(cudaMemsetAsync(g, 0, G_ * sizeof(node4<T>), ctx_->stream));
+                int* box = box_of(g);
+                k_box_clear<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, box, box > boxes_ ? box - 6 : nullptr,
+                                                                    geo_);
+                launched();
+                a.box = box;
             }
             const unsigned ws = warp_blocks(DMPM_SCATTER_CTAS, DMPM_P2G_THREADS);
             const int ush = set_units(a, ep);
@@ -1181,7 +1215,8 @@ template <class T> class Engine : public EngineBase {
             }
             pend();
             pbeg(K_GOP);
-            k_gop_inplace<<<ggrid(), 256, 0, ctx_->stream>>>((node4<float>*)g, G_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
+            k_box_gop<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, dm ? box_full_ : a.box,
+                                                              dm ? box_of(g) : nullptr, geo_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
             launched();
             pend();
             // the deterministic mode keeps the standalone stress stage: it also raises the
@@ -1422,9 +1457,7 @@ template <class T> class Engine : public EngineBase {
                 a.fix = fix_;
                 a.fixb = fixb_;
                 clear_fix(FIXB_ADJ);
-            } else {
-                DMPM_CK(cudaMemsetAsync(gadj_, 0, G_ * sizeof(node4<T>), ctx_->stream));
-            }
+            }  // else gadj_ is zero: cleared when the pass began and by each adjoint grid update
             const unsigned ws = warp_blocks(DMPM_ADJ_SCATTER_CTAS, DMPM_ADJ_SCATTER_THREADS);
             const int ush = set_units(a, ep);
             pbeg(K_ADJ_SCATTER);
@@ -1449,15 +1482,17 @@ template <class T> class Engine : public EngineBase {
             launched();
             pend();
             pbeg(K_ADJ_GOP);
-            if (ex) k_adj_gop_w<true><<<ggrid(), 256, 0, ctx_->stream>>>(a.grid, a.gadj, a.gadj2, G_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
-            else k_adj_gop_w<false><<<ggrid(), 256, 0, ctx_->stream>>>(a.grid, a.gadj, a.gadj2, G_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
+            if (P.keep_intermediates)
+                DMPM_CK(cudaMemcpyAsync(layers_[i].dbggdv, gadj_, G_ * sizeof(node4<T>), cudaMemcpyDeviceToDevice, ctx_->stream));
+            // kept intermediates show every node of the grid
+            const int* box = P.keep_intermediates ? box_full_ : box_of(grid_of(i));
+            if (ex) k_box_adj_gop<true><<<box_blocks(), 256, 0, ctx_->stream>>>(a.grid, a.gadj, a.gadj2, box, geo_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
+            else k_box_adj_gop<false><<<box_blocks(), 256, 0, ctx_->stream>>>(a.grid, a.gadj, a.gadj2, box, geo_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
             launched();
             pend();
-            if (P.keep_intermediates) {
-                DMPM_CK(cudaMemcpyAsync(layers_[i].dbggdv, gadj_, G_ * sizeof(node4<T>), cudaMemcpyDeviceToDevice, ctx_->stream));
+            if (P.keep_intermediates)
                 DMPM_CK(cudaMemcpy2DAsync(layers_[i].dbggdp, sizeof(node4<T>), gadj2_, 2 * sizeof(node4<T>),
                                           sizeof(node4<T>), G_, cudaMemcpyDeviceToDevice, ctx_->stream));
-            }
             pbeg(K_ADJ_GATHER);
             launch_gather<false>(a, ex, ctx_->stream);
             launched();
@@ -1536,6 +1571,7 @@ template <class T> class Engine : public EngineBase {
         if (top < L_ - 1 && !layers_[top].adj) throw StateError{"set keep_adjoints to start the adjoint below the last layer"};
         reset_status();
         if (ctrl_acc_) DMPM_CK(cudaMemsetAsync(ctrl_acc_, 0, 9 * np_ * sizeof(double), ctx_->stream));
+        if (kWarp) DMPM_CK(cudaMemsetAsync(gadj_, 0, G_ * sizeof(node4<T>), ctx_->stream));
         if (k_ == 1) {
             auto body = [&]() {
                 for (int i = top - 1; i >= control; i--) adjoint_step(i);
@@ -1624,6 +1660,10 @@ template <class T> class Engine : public EngineBase {
                 if (!layers_[l].st) throw StateError{"layer state is not stored (checkpointing)"};
                 if (field == DMPM_F_X) {
                     upload_x(in, layers_[l].st);
+                    // the stencils no longer are those that the layer's node box holds
+                    if (kWarp && k_ == 1)
+                        DMPM_CK(cudaMemcpyAsync(box_of(layers_[l].grid), box_full_, 6 * sizeof(int),
+                                                cudaMemcpyDeviceToDevice, ctx_->stream));
                     break;
                 }
                 const int off = field == DMPM_F_V ? PV : field == DMPM_F_F ? PF : PC;
@@ -1920,6 +1960,8 @@ template <class T> class Engine : public EngineBase {
     T* adj_pp_[2] = {nullptr, nullptr};
     node4<T>* gadj_ = nullptr;
     node4<T>* gadj2_ = nullptr;
+    int *boxes_ = nullptr, *box_full_ = nullptr;  // FP32 path: node boxes
+    bool boxes_fresh_ = false;                    // the boxes began empty with this cloud
     T* gridv_ = nullptr;
     T* pscratch_ = nullptr;
     // FP32 path

@@ -207,11 +207,13 @@ __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, DMPM_CHUNK_P2G_MINB) k_p2g
     __shared__ __align__(16) float s_rec[DMPM_CHUNK_THREADS * kRecFloats];
     const ChunkLane L = chunk_lane<BATCH>(a);
     if (L.cnt <= 0) return;
+    const int have = !BATCH && a.box && (threadIdx.x & 31) < 6 ? *(volatile int*)(a.box + (threadIdx.x & 31)) : 0;
     float* rec = s_rec + (threadIdx.x & ~31) * kRecFloats;
     float t[3];
     int base[3];
     load_x_base(a.st, a.npl, L.p, chunk_geo<BATCH>(a, L.inst), t, base, a.xlo);
     const ChunkGroups grp = chunk_groups<GENERAL>(chunk_key<BATCH>(a, L.inst, base), L.valid);
+    if (!BATCH && a.box) widen_box(a.box, have, a.geo, base, L.valid);
     {
         const float mp = a.cst[(size_t)KM * a.np + L.p], damp = 1.f - a.dt * a.drag;
         float b[4];

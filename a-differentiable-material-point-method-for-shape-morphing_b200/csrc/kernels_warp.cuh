@@ -305,7 +305,8 @@ struct WArgs {
     const float* cst;      // constants
     const float* dfc;      // dFc of layer n
     float* G;              // [24][npl] per layer: G (9), polar R (9), polar S (6: s00 s01 s02 s11 s12 s22)
-    node4<float>* grid;    // layer n grid: (p, m) after P2G, (v, m) after k_gop_inplace
+    node4<float>* grid;    // layer n grid: (p, m) after P2G, (v, m) after the grid update
+    int* box;              // node box that P2G widens to the stencils it adds to (NodeBox), or null
     float* P;              // debug: stress of layer n (or null)
     unsigned* status;
     // adjoint
@@ -486,17 +487,96 @@ template <bool GENERAL> __global__ void __launch_bounds__(DMPM_P2G_THREADS, DMPM
 }
 
 // G_op in place: (p, m) -> (v, m), v = p/m + dt f where |m| > FLT_EPSILON, else 0
-static __global__ void k_gop_inplace(node4<float>* grid, size_t G, float dt, float f0, float f1, float f2) {
-    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    node4<float> nd = grid[g];
-    const float f[3] = {f0, f1, f2};
+__device__ __forceinline__ void gop_node(node4<float>* n, float dt, const float f[3]) {
+    node4<float> nd = *n;
     float v[3];
     node_velocity(nd, dt, f, v);
     nd.x = v[0];
     nd.y = v[1];
     nd.z = v[2];
-    grid[g] = nd;
+    *n = nd;
+}
+static __global__ void k_gop_inplace(node4<float>* grid, size_t G, float dt, float f0, float f1, float f2) {
+    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= G) return;
+    const float f[3] = {f0, f1, f2};
+    gop_node(grid + g, dt, f);
+}
+
+// Node boxes.  A cloud fills a part of its grid: 8 % of the 64^3 headline scene's
+// nodes, 3 % of a 256^3 grid with a sphere of 79 cells.  Each layer's grid has a box
+// of nodes (first and last per axis, 6 ints) outside which it is zero, and the
+// node passes of the layer -- clearing its grid before P2G, the grid update, the
+// adjoint grid update -- walk the box instead of the grid.  P2G widens the box to
+// the stencils it adds to; boxes only grow (until a new cloud is set up), and a
+// layer's takes in the layer's before it first, so that P2G finds it wide enough
+// nearly always and few warps reach the atomics (starting empty at every step,
+// P2G took 55 instead of 29 us per step on the 64^3, 267k-particle scene).
+// One warp walks a row of the box along the last axis.
+struct NodeRange {
+    int lo[3], n[3];
+    __device__ __forceinline__ NodeRange(const int* box) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            lo[c] = box[c];
+            n[c] = box[3 + c] - box[c] + 1;  // <= 0: empty
+        }
+    }
+    __device__ __forceinline__ int rows() const { return n[0] > 0 && n[1] > 0 && n[2] > 0 ? n[0] * n[1] : 0; }
+    __device__ __forceinline__ size_t first(int row, const GridGeom& g) const {
+        const int i = row / n[1];
+        return node_id(g, lo[0] + i, lo[1] + (row - i * n[1]), lo[2]);
+    }
+};
+constexpr int kEmptyLo = 0x7fffffff;
+// boxes [0, grids) empty, box `grids` the whole grid
+static __global__ void k_box_reset(int* boxes, int grids, GridGeom g) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, b = t / 6, c = t % 6;
+    if (b > grids) return;
+    boxes[t] = b == grids ? (c < 3 ? 0 : g.dim[c - 3] - 1) : (c < 3 ? kEmptyLo : -1);
+}
+// every lane of the warp: widen the box to the stencils of the valid lanes; have:
+// lanes 0..5 the box's ints as read when the kernel began
+__device__ __forceinline__ void widen_box(int* box, int have, const GridGeom& g, const int base[3], bool valid) {
+    const int lane = threadIdx.x & 31;
+    int lo = kEmptyLo, hi = -1;  // of axis lane (lo) and lane - 3 (hi)
+    bool some = true;            // the warp has a node inside the grid
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const int l = max(0, __reduce_min_sync(0xffffffffu, valid ? base[c] : kEmptyLo));
+        const int h = min(g.dim[c] - 1, __reduce_max_sync(0xffffffffu, valid ? base[c] + 3 : -1));
+        some &= l <= h;
+        lo = lane == c ? l : lo;
+        hi = lane == 3 + c ? h : hi;
+    }
+    if (!some) return;
+    if (lane < 3 && lo < have) atomicMin(box + lane, lo);
+    if (lane >= 3 && lane < 6 && hi > have) atomicMax(box + lane, hi);
+}
+// zero the nodes of the layer's box, then take in the box `prev` (or null).  A block
+// may read the box while it grows: it then clears more, which is zero already.
+static __global__ void __launch_bounds__(256) k_box_clear(node4<float>* grid, int* box, const int* prev, GridGeom g) {
+    const NodeRange r(box);
+    for (int row = first_warp(); row < r.rows(); row += warp_count()) {
+        node4<float>* p = grid + r.first(row, g);
+        for (int k = threadIdx.x & 31; k < r.n[2]; k += 32) p[k] = node4<float>{0.f, 0.f, 0.f, 0.f};
+    }
+    if (prev && blockIdx.x == 0 && threadIdx.x < 6) {
+        const int a = box[threadIdx.x], b = prev[threadIdx.x];
+        box[threadIdx.x] = threadIdx.x < 3 ? min(a, b) : max(a, b);
+    }
+}
+// the grid update over the box; mark: the box to set to it (the deterministic mode
+// fills its grids whole), or null
+static __global__ void __launch_bounds__(256)
+    k_box_gop(node4<float>* grid, const int* __restrict__ box, int* mark, GridGeom g, float dt, float f0, float f1, float f2) {
+    const NodeRange r(box);
+    const float f[3] = {f0, f1, f2};
+    if (mark && blockIdx.x == 0 && threadIdx.x < 6) mark[threadIdx.x] = box[threadIdx.x];
+    for (int row = first_warp(); row < r.rows(); row += warp_count()) {
+        node4<float>* p = grid + r.first(row, g);
+        for (int k = threadIdx.x & 31; k < r.n[2]; k += 32) gop_node(p + k, dt, f);
+    }
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -626,23 +706,42 @@ __global__ void __launch_bounds__(DMPM_ADJ_SCATTER_THREADS, DMPM_ADJ_SCATTER_MIN
 // The record pair (dLdp, dLdm), (v, m) of a node is stored contiguously (32 B)
 // so the gather reads one sector per node.
 template <bool EXACT>
-__global__ void k_adj_gop_w(const node4<float>* __restrict__ grid, const node4<float>* __restrict__ gadj,
-                            node4<float>* gadj2, size_t G, float dt, float f0, float f1, float f2) {
-    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    const node4<float> nd = grid[g];
-    const node4<float> dv = gadj[g];
+__device__ __forceinline__ void adj_gop_node(const node4<float>& nd, const node4<float>& dv, node4<float>* out, float dt,
+                                             const float f[3]) {
     node4<float> o{0.f, 0.f, 0.f, 0.f};
     if (fabsf(nd.w) > (float)kFltEps) {
         float v[3] = {nd.x, nd.y, nd.z};
-        if (EXACT) { v[0] -= dt * f0; v[1] -= dt * f1; v[2] -= dt * f2; }
+        if (EXACT) { v[0] -= dt * f[0]; v[1] -= dt * f[1]; v[2] -= dt * f[2]; }
         o.x = dv.x / nd.w;
         o.y = dv.y / nd.w;
         o.z = dv.z / nd.w;
         o.w = -1.f / nd.w * (v[0] * dv.x + v[1] * dv.y + v[2] * dv.z);
     }
-    gadj2[2 * g] = o;
-    gadj2[2 * g + 1] = nd;
+    out[0] = o;
+    out[1] = nd;
+}
+template <bool EXACT>
+__global__ void k_adj_gop_w(const node4<float>* __restrict__ grid, const node4<float>* __restrict__ gadj,
+                            node4<float>* gadj2, size_t G, float dt, float f0, float f1, float f2) {
+    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= G) return;
+    const float f[3] = {f0, f1, f2};
+    adj_gop_node<EXACT>(grid[g], gadj[g], gadj2 + 2 * g, dt, f);
+}
+// the same over the layer's box, clearing dLdv behind it for the next scatter
+template <bool EXACT>
+__global__ void __launch_bounds__(256)
+    k_box_adj_gop(const node4<float>* __restrict__ grid, node4<float>* gadj, node4<float>* gadj2,
+                  const int* __restrict__ box, GridGeom g, float dt, float f0, float f1, float f2) {
+    const NodeRange r(box);
+    const float f[3] = {f0, f1, f2};
+    for (int row = first_warp(); row < r.rows(); row += warp_count()) {
+        const size_t n0 = r.first(row, g);
+        for (int k = threadIdx.x & 31; k < r.n[2]; k += 32) {
+            adj_gop_node<EXACT>(grid[n0 + k], gadj[n0 + k], gadj2 + 2 * (n0 + k), dt, f);
+            gadj[n0 + k] = node4<float>{0.f, 0.f, 0.f, 0.f};
+        }
+    }
 }
 
 // ------------------------------------------------------------------ finalize
