@@ -874,8 +874,8 @@ template <class T> class Engine : public EngineBase {
                 for (int i = 0; i < k_; i++) seg_G_[i] = (T*)layer_arena_.alloc(g_bytes);
             }
             adjn_ = (T*)layer_arena_.alloc(12 * np_ * sizeof(T));
-            alloc_sort();
         }
+        alloc_sort();
         if (P.keep_intermediates) {
             T* b1 = (T*)layer_arena_.alloc((size_t)L_ * 9 * np_ * sizeof(T));   // P
             T* b2 = (T*)layer_arena_.alloc((size_t)L_ * 9 * np_ * sizeof(T));   // dLdP
@@ -1242,17 +1242,16 @@ template <class T> class Engine : public EngineBase {
         a.gridv = gridv_;
         a.P = ctx_->prm.keep_intermediates ? layers_[l].dbgP : (kTiled ? nullptr : pscratch_);
         DMPM_CK(cudaMemsetAsync(g, 0, G_ * sizeof(node4<T>), ctx_->stream));
-        const size_t tile_b = (size_t)tile_cap() * sizeof(node4<T>);
-        (void)tile_b;
         (void)Gd;
-        (void)allow_sort;
-        {
+        if constexpr (!kWarp) {
+            const uint32_t* order = epoch_for(l, st, allow_sort).order;
             pbeg(K_P_OP1);
             k_p_op1<T><<<pgrid(), block(), 0, ctx_->stream>>>(a);
             launched();
             pend();
             pbeg(K_P2G);
-            k_p2g<T, false, false><<<pgrid(), block(), 0, ctx_->stream>>>(a);
+            const int chunk = scatter_chunk(n_);
+            k_p2g_c64<<<chunk_blocks(n_, chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a, order, chunk);
             launched();
             pend();
             pbeg(K_GOP);
@@ -1260,7 +1259,7 @@ template <class T> class Engine : public EngineBase {
             launched();
             pend();
             pbeg(K_G2P);
-            k_g2p<T, false><<<pgrid(), block(), 0, ctx_->stream>>>(a);
+            k_g2p<T><<<pgrid(), block(), 0, ctx_->stream>>>(a);
             launched();
             pend();
         }
@@ -1526,21 +1525,25 @@ template <class T> class Engine : public EngineBase {
         if (!a.st || !a.st_next || !a.grid) throw StateError{"internal: layer not materialised"};
         DMPM_CK(cudaMemsetAsync(gadj_, 0, G_ * sizeof(node4<T>), ctx_->stream));
         const bool ex = P.adjoint_mode == DMPM_ADJ_EXACT;
-        {
+        if constexpr (!kWarp) {
+            const uint32_t* order = epoch_for(i, state_of(i), false).order;
+            const int chunk = scatter_chunk(n_);
+            const unsigned cb = chunk_blocks(n_, chunk);
             pbeg(K_ADJ_SCATTER);
-            if (ex) k_adj_scatter<T, false, true><<<pgrid(), block(), 0, ctx_->stream>>>(a);
-            else k_adj_scatter<T, false, false><<<pgrid(), block(), 0, ctx_->stream>>>(a);
+            if (ex) k_adj_scatter_c64<true><<<cb, DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a, order, chunk);
+            else k_adj_scatter_c64<false><<<cb, DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a, order, chunk);
             launched();
             pend();
             pbeg(K_ADJ_GOP);
-            if (ex) k_adj_gop<T, true><<<ggrid(), 256, 0, ctx_->stream>>>(a, G_);
-            else k_adj_gop<T, false><<<ggrid(), 256, 0, ctx_->stream>>>(a, G_);
+            if (ex) k_adj_gop<T, true, true><<<ggrid(), 256, 0, ctx_->stream>>>(a, G_);
+            else k_adj_gop<T, false, true><<<ggrid(), 256, 0, ctx_->stream>>>(a, G_);
             launched();
             pend();
             if (P.keep_intermediates) debug_grid_adjoint(i, a, ex);
             pbeg(K_ADJ_GATHER);
-            if (ex) k_adj_gather<T, false, true><<<pgrid(), block(), 0, ctx_->stream>>>(a);
-            else k_adj_gather<T, false, false><<<pgrid(), block(), 0, ctx_->stream>>>(a);
+            const unsigned gt = (unsigned)std::min(block(), 128), gb = (unsigned)((n_ + gt - 1) / gt);
+            if (ex) k_adj_gather<T, true><<<gb, gt, 0, ctx_->stream>>>(a);
+            else k_adj_gather<T, false><<<gb, gt, 0, ctx_->stream>>>(a);
             launched();
             pend();
         }
@@ -1550,8 +1553,8 @@ template <class T> class Engine : public EngineBase {
         DMPM_CK(cudaMemcpyAsync(layers_[i].dbggdv, gadj_, G_ * sizeof(node4<T>), cudaMemcpyDeviceToDevice, ctx_->stream));
         AdjArgs<T> b = a;
         b.gadj2 = layers_[i].dbggdp;
-        if (ex) k_adj_gop<T, true><<<ggrid(), 256, 0, ctx_->stream>>>(b, G_);
-        else k_adj_gop<T, false><<<ggrid(), 256, 0, ctx_->stream>>>(b, G_);
+        if (ex) k_adj_gop<T, true, false><<<ggrid(), 256, 0, ctx_->stream>>>(b, G_);
+        else k_adj_gop<T, false, false><<<ggrid(), 256, 0, ctx_->stream>>>(b, G_);
         launched();
     }
 

@@ -11,14 +11,14 @@
 // The stencil of a particle is the 4x4x4 node block at floor((x-min)/dx) - 1
 // (reference: ForwardSimulation.cpp:17-36); nodes outside the grid are skipped.
 //
-// Two execution strategies share the arithmetic:
-//   TILED (FP32 path): each CTA takes a contiguous chunk of particles, reduces
-//     the bounding box of their stencils and, when it fits the shared-memory
-//     capacity, scatters into / gathers from a shared-memory node tile; tiles
-//     are flushed with one vector red.global.add per touched node.  Chunks whose
-//     box does not fit use the global path.
-//   plain (FP64 path): one thread per particle, global atomics and gathers,
-//     one kernel per reference stage.
+// These are the FP64 path's kernels, one per reference stage and one thread per
+// particle, and the loss and volume kernels that both paths use; the FP64 path's
+// P2G and adjoint scatter walk chunks of the cell-sorted order
+// (kernels_chunk.cuh).  The mass raster of the FP32 path is TILED: each CTA takes
+// a contiguous chunk of particles, reduces the bounding box of their stencils and,
+// when it fits the shared-memory capacity, adds into a shared-memory node tile
+// that is flushed once per touched node; chunks whose box does not fit add to
+// global memory.
 #pragma once
 #include <cstdint>
 #include "elasticity.cuh"
@@ -193,99 +193,10 @@ template <class T> __global__ void k_p_op1(FwdArgs<T> a) {
     if (p >= a.n) return;
     m3<double> Fe = m3_cast<double>(load_m3(a.st + (size_t)PF * a.np, a.np, p)) + m3_cast<double>(load_m3(a.dfc, a.np, p));
     if (a.strain) Fe = Fe + m3_eye<double>();  // the F planes hold H = F - I
-    const m3<double> P = pk_stress<double>(Fe, (double)a.cst[(size_t)KLAM * a.np + p], (double)a.cst[(size_t)KMU * a.np + p]);
+    m3<double> R, S;
+    polar(Fe, R, S);
+    const m3<double> P = pk_from_polar(Fe, R, (double)a.cst[(size_t)KLAM * a.np + p], (double)a.cst[(size_t)KMU * a.np + p]);
     store_m3(a.P, a.np, p, m3_cast<T>(P));
-}
-
-// ------------------------------------------------------------------ P2G
-// m_g += w m_p;  p_g += w (m_p v (1 - dt drag) + (-3/dx^2 dt vol P Fe^T + m_p C) (x_g - x_p))
-// (SingleParticle_to_grid, ForwardSimulation.cpp:11-51).  FUSED_P computes P
-// here (FP64 polar) instead of reading the P_op_1 output.
-template <class T, bool TILED, bool FUSED_P> __global__ void __launch_bounds__(256) k_p2g(FwdArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = p < a.n;
-    const T dx = (T)a.geo.dx;
-    T x[3] = {0, 0, 0};
-    int base[3] = {0, 0, 0};
-    m3<T> G = m3_zero<T>();
-    T mvd[3] = {0, 0, 0}, mp = 0;
-    if (valid) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            x[c] = a.st[(size_t)(PX + c) * a.np + p];
-            base[c] = stencil_base<T>(x[c] - (T)a.geo.mn[c], dx, a.geo.dim[c]);
-        }
-        const m3<T> F = load_m3(a.st + (size_t)PF * a.np, a.np, p);
-        const m3<T> Fe = F + load_m3(a.dfc, a.np, p);
-        mp = a.cst[(size_t)KM * a.np + p];
-        const T vol = a.cst[(size_t)KVOL * a.np + p];
-        m3<T> P;
-        if (FUSED_P) {
-            const m3<double> Pd = pk_stress<double>(m3_cast<double>(Fe), (double)a.cst[(size_t)KLAM * a.np + p],
-                                                    (double)a.cst[(size_t)KMU * a.np + p]);
-            P = m3_cast<T>(Pd);
-            if (a.P) store_m3(a.P, a.np, p, P);
-        } else {
-            P = load_m3(a.P, a.np, p);
-        }
-        const T k = -T(3) / (dx * dx) * a.dt * vol;
-        G = (k * P) * transpose(Fe) + mp * load_m3(a.st + (size_t)PC * a.np, a.np, p);
-        const T damp = T(1) - a.dt * a.drag;
-#pragma unroll
-        for (int c = 0; c < 3; c++) mvd[c] = mp * a.st[(size_t)(PV + c) * a.np + p] * damp;
-    }
-    axis_w<T> w[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) axis_weights(x[c], (T)a.geo.mn[c], dx, base[c], w[c], false);
-
-    TileBox tb;
-    tb.ok = false;
-    node4<T>* tile = reinterpret_cast<node4<T>*>(smem_raw);
-    if (TILED) {
-        tb = block_tile_box(valid, base, a.tile_cap);
-        if (tb.ok) {
-            for (int t = threadIdx.x; t < tb.n; t += blockDim.x) tile[t] = node4<T>{0, 0, 0, 0};
-            __syncthreads();
-        }
-    }
-    if (valid) {
-        const int rot = TILED ? (threadIdx.x & 63) : 0;
-#pragma unroll 4
-        for (int it = 0; it < 64; it++) {
-            const int idx = (it + rot) & 63;
-            const int di = idx >> 4, dj = (idx >> 2) & 3, dk = idx & 3;
-            const int gi = base[0] + di, gj = base[1] + dj, gk = base[2] + dk;
-            if (gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2]) continue;
-            const T d[3] = {pick4(w[0].d, di), pick4(w[1].d, dj), pick4(w[2].d, dk)};
-            const T wt = pick4(w[0].n, di) * pick4(w[1].n, dj) * pick4(w[2].n, dk);
-            T gd[3];
-            mv(G, d, gd);
-            const T q0 = wt * (mvd[0] + gd[0]), q1 = wt * (mvd[1] + gd[1]), q2 = wt * (mvd[2] + gd[2]);
-            const T qm = wt * mp;
-            if (TILED && tb.ok) {
-                node4<T>* nd = tile + tile_index(tb, gi, gj, gk);
-                atomicAdd(&nd->w, qm);
-                atomicAdd(&nd->x, q0);
-                atomicAdd(&nd->y, q1);
-                atomicAdd(&nd->z, q2);
-            } else {
-                const size_t g = ((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk;
-                red_add4(a.grid + g, q0, q1, q2, qm);
-            }
-        }
-    }
-    if (TILED && tb.ok) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < tb.n; t += blockDim.x) {
-            const node4<T> v = tile[t];
-            if (v.w == T(0) && v.x == T(0) && v.y == T(0) && v.z == T(0)) continue;
-            const int k = t % tb.e[2], j = (t / tb.e[2]) % tb.e[1], i = t / (tb.e[2] * tb.e[1]);
-            const int gi = tb.o[0] + i, gj = tb.o[1] + j, gk = tb.o[2] + k;
-            if (gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2]) continue;
-            red_add4(a.grid + ((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk, v.x, v.y, v.z, v.w);
-        }
-    }
 }
 
 // ------------------------------------------------------------------ G_op
@@ -313,69 +224,55 @@ template <class T> __global__ void k_gop(FwdArgs<T> a, size_t G) {
 // ------------------------------------------------------------------ G2P + P_op_2
 // v' = sum w v_g;  C' = 3/dx^2 sum w v_g (x_g - x_p)^T  (ForwardSimulation.cpp:60-106)
 // F' = (1 - s)(I + dt C')(F + dFc) + s F;  x' = x + dt v'  (:108-124)
-// TILED fuses G_op into the tile load.
-template <class T, bool TILED> __global__ void __launch_bounds__(256) k_g2p(FwdArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+template <class T> __global__ void __launch_bounds__(256) k_g2p(FwdArgs<T> a) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = p < a.n;
+    if (p >= a.n) return;
     const T dx = (T)a.geo.dx;
     const size_t G = (size_t)a.geo.dim[0] * a.geo.dim[1] * a.geo.dim[2];
-    T x[3] = {0, 0, 0};
-    int base[3] = {0, 0, 0};
-    if (valid) {
+    T x[3];
+    int base[3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            x[c] = a.st[(size_t)(PX + c) * a.np + p];
-            base[c] = stencil_base<T>(x[c] - (T)a.geo.mn[c], dx, a.geo.dim[c]);
-        }
+    for (int c = 0; c < 3; c++) {
+        x[c] = a.st[(size_t)(PX + c) * a.np + p];
+        base[c] = stencil_base<T>(x[c] - (T)a.geo.mn[c], dx, a.geo.dim[c]);
     }
-    TileBox tb;
-    tb.ok = false;
-    node4<T>* tile = reinterpret_cast<node4<T>*>(smem_raw);
-    if (TILED) {
-        tb = block_tile_box(valid, base, a.tile_cap);
-        if (tb.ok) {
-            for (int t = threadIdx.x; t < tb.n; t += blockDim.x) {
-                const int k = t % tb.e[2], j = (t / tb.e[2]) % tb.e[1], i = t / (tb.e[2] * tb.e[1]);
-                const int gi = tb.o[0] + i, gj = tb.o[1] + j, gk = tb.o[2] + k;
-                T v[3] = {0, 0, 0};
-                if (!(gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2]))
-                    node_velocity(a.grid[((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk], a.dt, a.fext, v);
-                tile[t] = node4<T>{v[0], v[1], v[2], T(0)};
-            }
-            __syncthreads();
-        }
-    }
-    if (!valid) return;
     axis_w<T> w[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) axis_weights(x[c], (T)a.geo.mn[c], dx, base[c], w[c], false);
+    // factored per stencil row: the k sums of n2 v and n2 d2 v
     T vn[3] = {0, 0, 0};
     m3<T> Cn = m3_zero<T>();
     const T k3 = T(3) / (dx * dx);
-#pragma unroll 2
-    for (int idx = 0; idx < 64; idx++) {
-        const int di = idx >> 4, dj = (idx >> 2) & 3, dk = idx & 3;
-        const int gi = base[0] + di, gj = base[1] + dj, gk = base[2] + dk;
-        if (gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2]) continue;
-        const T d[3] = {w[0].d[di], w[1].d[dj], w[2].d[dk]};
-        const T wt = w[0].n[di] * w[1].n[dj] * w[2].n[dk];
-        T vg[3];
-        if (TILED && tb.ok) {
-            const node4<T> nd = tile[tile_index(tb, gi, gj, gk)];
-            vg[0] = nd.x; vg[1] = nd.y; vg[2] = nd.z;
-        } else if (TILED) {
-            node_velocity(a.grid[((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk], a.dt, a.fext, vg);
-        } else {
-            const size_t g = ((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk;
-            vg[0] = a.gridv[g]; vg[1] = a.gridv[G + g]; vg[2] = a.gridv[2 * G + g];
-        }
+#pragma unroll 1
+    for (int di = 0; di < 4; di++) {
+        const int gi = base[0] + di;
+        if (gi < 0 || gi >= a.geo.dim[0]) continue;
+#pragma unroll 1
+        for (int dj = 0; dj < 4; dj++) {
+            const int gj = base[1] + dj;
+            if (gj < 0 || gj >= a.geo.dim[1]) continue;
+            const ptrdiff_t row = ((ptrdiff_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + base[2];
+            T R[3] = {0, 0, 0}, D[3] = {0, 0, 0};
 #pragma unroll
-        for (int r = 0; r < 3; r++) {
-            vn[r] += wt * vg[r];
-            const T kv = k3 * wt * vg[r];
+            for (int dk = 0; dk < 4; dk++) {
+                const int gk = base[2] + dk;
+                if (gk < 0 || gk >= a.geo.dim[2]) continue;
+                const T n2 = w[2].n[dk], nd = n2 * w[2].d[dk];
 #pragma unroll
-            for (int c = 0; c < 3; c++) Cn.a[r][c] += kv * d[c];
+                for (int r = 0; r < 3; r++) {
+                    const T vg = a.gridv[(ptrdiff_t)(r * G) + row + dk];
+                    R[r] += n2 * vg;
+                    D[r] += nd * vg;
+                }
+            }
+            const T w01 = w[0].n[di] * w[1].n[dj], c0 = k3 * w01 * w[0].d[di], c1 = k3 * w01 * w[1].d[dj], c2 = k3 * w01;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                vn[r] += w01 * R[r];
+                Cn.a[r][0] += c0 * R[r];
+                Cn.a[r][1] += c1 * R[r];
+                Cn.a[r][2] += c2 * D[r];
+            }
         }
     }
     const m3<T> F = load_m3(a.st + (size_t)PF * a.np, a.np, p);
@@ -572,7 +469,7 @@ template <class T> struct AdjArgs {
     const T* adj_next;    // adjoint of layer n+1
     T* adj;               // adjoint of layer n (output)
     node4<T>* gadj;       // grid scratch: (dLdv.xyz, unused)
-    node4<T>* gadj2;      // plain path: (dLdp.xyz, dLdm)
+    node4<T>* gadj2;      // per node (dLdp.xyz, dLdm), (v.xyz, m)
     T* ctrl_grad;         // per-layer dL/d dFc of layer n [9][np] (or null)
     double* ctrl_acc;     // tied controls: FP64 accumulator [9][np] (or null)
     // debug copies of intermediates (may be null)
@@ -595,83 +492,6 @@ __device__ __forceinline__ void adj_next_terms(const AdjArgs<T>& a, int p, const
     Cn = (c * dFn) * transpose(Fe) + load_m3(a.adj_next + (size_t)PC * a.np, a.np, p);
 }
 
-// Adjoint G2P: dLdv_g += w dLdv_next + 3/dx^2 w dLdC_next (x_g - x_p)
-// (BackPropagation.cpp:27-44).
-template <class T, bool TILED, bool EXACT> __global__ void __launch_bounds__(256) k_adj_scatter(AdjArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = p < a.n;
-    const T dx = (T)a.geo.dx;
-    T x[3] = {0, 0, 0};
-    int base[3] = {0, 0, 0};
-    T vn[3] = {0, 0, 0};
-    m3<T> Cn = m3_zero<T>();
-    if (valid) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            x[c] = a.st[(size_t)(PX + c) * a.np + p];
-            base[c] = stencil_base<T>(x[c] - (T)a.geo.mn[c], dx, a.geo.dim[c]);
-        }
-        const m3<T> Fe = load_m3(a.st + (size_t)PF * a.np, a.np, p) + load_m3(a.dfc, a.np, p);
-        adj_next_terms<T, EXACT>(a, p, Fe, vn, Cn);
-        if (a.dbg_vnext) {
-#pragma unroll
-            for (int c = 0; c < 3; c++) a.dbg_vnext[(size_t)c * a.np + p] = vn[c];
-            store_m3(a.dbg_Cnext, a.np, p, Cn);
-        }
-    }
-    axis_w<T> w[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) axis_weights(x[c], (T)a.geo.mn[c], dx, base[c], w[c], false);
-    TileBox tb;
-    tb.ok = false;
-    node4<T>* tile = reinterpret_cast<node4<T>*>(smem_raw);
-    if (TILED) {
-        tb = block_tile_box(valid, base, a.tile_cap);
-        if (tb.ok) {
-            for (int t = threadIdx.x; t < tb.n; t += blockDim.x) tile[t] = node4<T>{0, 0, 0, 0};
-            __syncthreads();
-        }
-    }
-    const T k3 = T(3) / (dx * dx);
-    if (valid) {
-        const int rot = TILED ? (threadIdx.x & 63) : 0;
-#pragma unroll 4
-        for (int it = 0; it < 64; it++) {
-            const int idx = (it + rot) & 63;
-            const int di = idx >> 4, dj = (idx >> 2) & 3, dk = idx & 3;
-            const int gi = base[0] + di, gj = base[1] + dj, gk = base[2] + dk;
-            if (gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2]) continue;
-            const T d[3] = {pick4(w[0].d, di), pick4(w[1].d, dj), pick4(w[2].d, dk)};
-            const T wt = pick4(w[0].n, di) * pick4(w[1].n, dj) * pick4(w[2].n, dk);
-            T cd[3];
-            mv(Cn, d, cd);
-            const T q0 = vn[0] * wt + k3 * wt * cd[0];
-            const T q1 = vn[1] * wt + k3 * wt * cd[1];
-            const T q2 = vn[2] * wt + k3 * wt * cd[2];
-            if (TILED && tb.ok) {
-                node4<T>* nd = tile + tile_index(tb, gi, gj, gk);
-                atomicAdd(&nd->x, q0);
-                atomicAdd(&nd->y, q1);
-                atomicAdd(&nd->z, q2);
-            } else {
-                red_add4(a.gadj + ((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk, q0, q1, q2, T(0));
-            }
-        }
-    }
-    if (TILED && tb.ok) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < tb.n; t += blockDim.x) {
-            const node4<T> v = tile[t];
-            if (v.x == T(0) && v.y == T(0) && v.z == T(0)) continue;
-            const int k = t % tb.e[2], j = (t / tb.e[2]) % tb.e[1], i = t / (tb.e[2] * tb.e[1]);
-            const int gi = tb.o[0] + i, gj = tb.o[1] + j, gk = tb.o[2] + k;
-            if (gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2]) continue;
-            red_add4(a.gadj + ((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk, v.x, v.y, v.z, T(0));
-        }
-    }
-}
-
 // Adjoint G_op: dLdp = dLdv / m; dLdm = -(1/m) v_m . dLdv where |m| > FLT_EPS
 // (BackPropagation.cpp:46-59).  v_m is the node velocity v (reference) or
 // p/m = v - dt f_ext (EXACT).
@@ -690,12 +510,21 @@ DMPM_HD void node_adjoint(const node4<T>& nd, const node4<T>& gdv, T dt, const T
     }
 }
 
-template <class T, bool EXACT> __global__ void k_adj_gop(AdjArgs<T> a, size_t G) {
+// PAIR: a node's (dLdp, dLdm) and (v, m) side by side in gadj2, so that the gather
+// reads the velocity instead of dividing the momentum at every node of every
+// particle; otherwise (dLdp, dLdm) alone.
+template <class T, bool EXACT, bool PAIR> __global__ void k_adj_gop(AdjArgs<T> a, size_t G) {
     const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G) return;
+    const node4<T> nd = a.grid[g];
     T o[4];
-    node_adjoint<T, EXACT>(a.grid[g], a.gadj[g], a.dt, a.fext, o);
-    a.gadj2[g] = node4<T>{o[0], o[1], o[2], o[3]};
+    node_adjoint<T, EXACT>(nd, a.gadj[g], a.dt, a.fext, o);
+    a.gadj2[PAIR ? 2 * g : g] = node4<T>{o[0], o[1], o[2], o[3]};
+    if (PAIR) {
+        T v[3];
+        node_velocity(nd, a.dt, a.fext, v);
+        a.gadj2[2 * g + 1] = node4<T>{v[0], v[1], v[2], nd.w};
+    }
 }
 
 // Adjoint P2G + P_op_1 (BackPropagation.cpp:61-124), as a per-particle gather.
@@ -709,43 +538,21 @@ template <class T, bool EXACT> __global__ void k_adj_gop(AdjArgs<T> a, size_t G)
 //   REFCOMPAT: dLdF += (I + dt C')^T dLdF' + dP/dF:dLdP     (the transport term twice)
 //   EXACT:     dLdFe = (1-s)(I + dt C')^T dLdF' + stress + dP/dF:dLdP;  dLdF = dLdFe + s dLdF'
 // The polar factors, P and dP/dF:dLdP are evaluated in FP64.
-template <class T, bool TILED, bool EXACT> __global__ void __launch_bounds__(256) k_adj_gather(AdjArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+// Blocks of 128, 4 per SM: the FP64 chains want the warps more than the registers
+// (57.7k particles: 62 us per step at 4, 69 at 2, 70 in blocks of 256 at the
+// compiler's 218 registers).  Sums factored per stencil row, which the other
+// gathers gain from, keep 22 more values live here: 70-83 us.
+template <class T, bool EXACT> __global__ void __launch_bounds__(128, EXACT ? 4 : 2) k_adj_gather(AdjArgs<T> a) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = p < a.n;
+    if (p >= a.n) return;
     const T dx = (T)a.geo.dx;
-    T x[3] = {0, 0, 0};
-    int base[3] = {0, 0, 0};
-    if (valid) {
+    T x[3];
+    int base[3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            x[c] = a.st[(size_t)(PX + c) * a.np + p];
-            base[c] = stencil_base<T>(x[c] - (T)a.geo.mn[c], dx, a.geo.dim[c]);
-        }
+    for (int c = 0; c < 3; c++) {
+        x[c] = a.st[(size_t)(PX + c) * a.np + p];
+        base[c] = stencil_base<T>(x[c] - (T)a.geo.mn[c], dx, a.geo.dim[c]);
     }
-    TileBox tb;
-    tb.ok = false;
-    node4<T>* tile = reinterpret_cast<node4<T>*>(smem_raw);  // [2*n]: (dLdp, dLdm), (v_g, 0)
-    if (TILED) {
-        tb = block_tile_box(valid, base, a.tile_cap);
-        if (tb.ok) {
-            for (int t = threadIdx.x; t < tb.n; t += blockDim.x) {
-                const int k = t % tb.e[2], j = (t / tb.e[2]) % tb.e[1], i = t / (tb.e[2] * tb.e[1]);
-                const int gi = tb.o[0] + i, gj = tb.o[1] + j, gk = tb.o[2] + k;
-                T o[4] = {0, 0, 0, 0}, v[3] = {0, 0, 0};
-                if (!(gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2])) {
-                    const size_t g = ((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk;
-                    const node4<T> nd = a.grid[g];
-                    node_adjoint<T, EXACT>(nd, a.gadj[g], a.dt, a.fext, o);
-                    node_velocity(nd, a.dt, a.fext, v);
-                }
-                tile[2 * t] = node4<T>{o[0], o[1], o[2], o[3]};
-                tile[2 * t + 1] = node4<T>{v[0], v[1], v[2], T(0)};
-            }
-            __syncthreads();
-        }
-    }
-    if (!valid) return;
     const size_t np = a.np;
     const T mp = a.cst[(size_t)KM * np + p], vol = a.cst[(size_t)KVOL * np + p];
     const m3<T> F = load_m3(a.st + (size_t)PF * np, np, p);
@@ -753,7 +560,7 @@ template <class T, bool TILED, bool EXACT> __global__ void __launch_bounds__(256
     // polar factors and stress in FP64
     const m3<double> Fed = m3_cast<double>(Fe);
     m3<double> Rd, Sd;
-    polar3(Fed, Rd, Sd);
+    polar(Fed, Rd, Sd);
     const double lam = (double)a.cst[(size_t)KLAM * np + p], mu = (double)a.cst[(size_t)KMU * np + p];
     const m3<T> P = m3_cast<T>(pk_from_polar(Fed, Rd, lam, mu));
     const T k3 = T(3) / (dx * dx);
@@ -772,30 +579,14 @@ template <class T, bool TILED, bool EXACT> __global__ void __launch_bounds__(256
     m3<T> M = m3_zero<T>();
     T X[3] = {0, 0, 0}, u[3] = {0, 0, 0}, z[3] = {0, 0, 0};
     const T ndx = -T(1) / dx;
-    const size_t G_ = (size_t)a.geo.dim[0] * a.geo.dim[1] * a.geo.dim[2];
-    (void)G_;
 #pragma unroll 2
     for (int idx = 0; idx < 64; idx++) {
         const int di = idx >> 4, dj = (idx >> 2) & 3, dk = idx & 3;
         const int gi = base[0] + di, gj = base[1] + dj, gk = base[2] + dk;
         if (gi < 0 || gi >= a.geo.dim[0] || gj < 0 || gj >= a.geo.dim[1] || gk < 0 || gk >= a.geo.dim[2]) continue;
-        T o[4], vg[3];
-        if (TILED && tb.ok) {
-            const int t = tile_index(tb, gi, gj, gk);
-            const node4<T> q = tile[2 * t], r = tile[2 * t + 1];
-            o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
-            vg[0] = r.x; vg[1] = r.y; vg[2] = r.z;
-        } else {
-            const size_t g = ((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk;
-            const node4<T> nd = a.grid[g];
-            if (TILED) {
-                node_adjoint<T, EXACT>(nd, a.gadj[g], a.dt, a.fext, o);
-            } else {
-                const node4<T> q = a.gadj2[g];
-                o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
-            }
-            node_velocity(nd, a.dt, a.fext, vg);
-        }
+        const node4<T>* pair = a.gadj2 + 2 * (((size_t)gi * a.geo.dim[1] + gj) * a.geo.dim[2] + gk);
+        const node4<T> q = pair[0], nv = pair[1];
+        const T o[4] = {q.x, q.y, q.z, q.w}, vg[3] = {nv.x, nv.y, nv.z};
         const T d[3] = {w[0].d[di], w[1].d[dj], w[2].d[dk]};
         const T nx = w[0].n[di], ny = w[1].n[dj], nz = w[2].n[dk];
         const T wt = nx * ny * nz;

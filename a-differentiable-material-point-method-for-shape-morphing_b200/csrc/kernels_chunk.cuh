@@ -709,4 +709,153 @@ template <bool BATCH> inline void launch_gather(const WArgs& a, bool exact, cuda
     else k_adj_gather_c<false, BATCH, 1><<<b, t, 0, st>>>(a);
 }
 
+// ------------------------------------------------------------------ FP64 path
+// P2G and the adjoint scatter of the FP64 path, as above in double.  One thread
+// per particle adding each of its 64 nodes with 4 FP64 atomics took 146 and 155 us
+// per step on 57.7k particles at 8 per cell; here a cell's particles reach a node
+// in one round of atomics: 35 and 30 us.
+// Record (doubles, 16-byte pairs): (n0, n0 d0)[4], (n1, n1 d1)[4], n2 and n2 d2 in
+// pairs of nodes (2h, 2h + 1), b (4), A (9, column-major); 38 apart.
+constexpr int kRec64 = 38;
+__device__ __forceinline__ void chunk_record64(double* rec, const axis_w<double> (&w)[3], const double b[4],
+                                               const m3<double>& A) {
+    double2* r = reinterpret_cast<double2*>(rec);
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) r[4 * c + k] = make_double2(w[c].n[k], w[c].n[k] * w[c].d[k]);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        r[8 + 2 * h] = make_double2(w[2].n[2 * h], w[2].n[2 * h + 1]);
+        r[9 + 2 * h] = make_double2(w[2].n[2 * h] * w[2].d[2 * h], w[2].n[2 * h + 1] * w[2].d[2 * h + 1]);
+    }
+    r[12] = make_double2(b[0], b[1]);
+    r[13] = make_double2(b[2], b[3]);
+    r[14] = make_double2(A.a[0][0], A.a[1][0]);
+    r[15] = make_double2(A.a[2][0], A.a[0][1]);
+    r[16] = make_double2(A.a[1][1], A.a[2][1]);
+    r[17] = make_double2(A.a[0][2], A.a[1][2]);
+    rec[36] = A.a[2][2];
+}
+template <int NC>
+__device__ __forceinline__ void chunk_scatter64(const double* rec, const int base[3], const ChunkGroups& grp,
+                                                const GridGeom& g, node4<double>* dst) {
+    const int lane = threadIdx.x & 31, hf = lane >> 4, i = (lane >> 2) & 3, j = lane & 3;
+    for (unsigned left = grp.leaders; left; left &= left - 1) {
+        const int lead = __ffs(left) - 1;
+        const int s = __shfl_sync(0xffffffffu, grp.first, lead), e = s + __shfl_sync(0xffffffffu, grp.size, lead);
+        double acc[4][NC];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) acc[k][c] = 0.0;
+#pragma unroll 1
+        for (int q = s; q < e; q += 2) {
+            const bool in = q + hf < e;
+            const double* p = rec + (in ? q + hf : s) * kRec64;
+            const double2* r = reinterpret_cast<const double2*>(p);
+            double2 w0 = r[i];
+            const double2 w1 = r[4 + j], na = r[8 + 2 * hf], ea = r[9 + 2 * hf], nb = r[10 - 2 * hf], eb = r[11 - 2 * hf];
+            const double2 b01 = r[12], b23 = r[13], A0 = r[14], A1 = r[15], A2 = r[16], A3 = r[17];
+            if (!in) w0 = make_double2(0.0, 0.0);
+            const double a0 = w0.x * w1.x, a1 = w0.y * w1.x, a2 = w0.x * w1.y;
+            const double h[3] = {a0 * b01.x + a1 * A0.x + a2 * A1.y, a0 * b01.y + a1 * A0.y + a2 * A2.x,
+                                 a0 * b23.x + a1 * A1.x + a2 * A2.y};
+            const double gg[3] = {a0 * A3.x, a0 * A3.y, a0 * p[36]};
+            const double n2[4] = {na.x, na.y, nb.x, nb.y}, e2[4] = {ea.x, ea.y, eb.x, eb.y}, am = a0 * b23.y;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) acc[k][c] += n2[k] * h[c] + e2[k] * gg[c];
+                if (NC == 4) acc[k][NC - 1] += n2[k] * am;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) acc[k][c] += __shfl_xor_sync(0xffffffffu, acc[k + 2][c], 16);
+        const int gi = __shfl_sync(0xffffffffu, base[0], lead) + i, gj = __shfl_sync(0xffffffffu, base[1], lead) + j,
+                  gk = __shfl_sync(0xffffffffu, base[2], lead) + 2 * hf;
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+            if (in_grid(g, gi, gj, gk + k)) {
+                double* n = &dst[node_id(g, gi, gj, gk + k)].x;
+#pragma unroll
+                for (int c = 0; c < NC; c++)
+                    if (acc[k][c] != 0.0) atomicAdd(n + c, acc[k][c]);
+            }
+    }
+}
+// the lane's particle, stencil base and weights, as the FP64 path forms them
+struct ChunkLane64 {
+    int p, cnt, base[3];
+    bool valid;
+    axis_w<double> w[3];
+    ChunkGroups grp;
+};
+__device__ __forceinline__ bool chunk_lane64(ChunkLane64& L, const uint32_t* order, int n, int chunk, const double* st,
+                                             size_t np, const GridGeom& g) {
+    const int lane = threadIdx.x & 31, q0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * chunk;
+    L.cnt = min(chunk, n - q0);
+    if (L.cnt <= 0) return false;  // the whole warp
+    L.valid = lane < L.cnt;
+    L.p = (int)order[q0 + (L.valid ? lane : 0)];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const double x = st[(size_t)(PX + c) * np + L.p];
+        L.base[c] = stencil_base<double>(x - g.mn[c], g.dx, g.dim[c]);
+        axis_weights<double>(x, g.mn[c], g.dx, L.base[c], L.w[c], false);
+    }
+    L.grp = chunk_groups<false>(cell_key(L.base, g.dim), L.valid);
+    return true;
+}
+
+// m_g += w m_p;  p_g += w (m_p v (1 - dt drag) + (-3/dx^2 dt vol P Fe^T + m_p C) (x_g - x_p))
+// (SingleParticle_to_grid, ForwardSimulation.cpp:11-51)
+static __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, 4) k_p2g_c64(FwdArgs<double> a, const uint32_t* order, int chunk) {
+    __shared__ __align__(16) double s_rec[DMPM_CHUNK_THREADS * kRec64];
+    ChunkLane64 L;
+    if (!chunk_lane64(L, order, a.n, chunk, a.st, a.np, a.geo)) return;
+    double* rec = s_rec + (threadIdx.x & ~31) * kRec64;
+    if (L.valid) {
+        const int p = L.p;
+        const double dx = a.geo.dx, mp = a.cst[(size_t)KM * a.np + p], damp = 1.0 - a.dt * a.drag;
+        const m3<double> Fe = load_m3(a.st + (size_t)PF * a.np, a.np, p) + load_m3(a.dfc, a.np, p);
+        const double k = -3.0 / (dx * dx) * a.dt * a.cst[(size_t)KVOL * a.np + p];
+        const m3<double> G = (k * load_m3((const double*)a.P, a.np, p)) * transpose(Fe) +
+                             mp * load_m3(a.st + (size_t)PC * a.np, a.np, p);
+        double b[4];
+#pragma unroll
+        for (int c = 0; c < 3; c++) b[c] = mp * a.st[(size_t)(PV + c) * a.np + p] * damp;
+        b[3] = mp;
+        chunk_record64(rec + L.grp.slot * kRec64, L.w, b, G);
+    }
+    __syncwarp();
+    chunk_scatter64<4>(rec, L.base, L.grp, a.geo, a.grid);
+}
+// dLdv_g += w dLdv_next + 3/dx^2 w dLdC_next (x_g - x_p)   (BackPropagation.cpp:27-44)
+template <bool EXACT>
+__global__ void __launch_bounds__(DMPM_CHUNK_THREADS, 4) k_adj_scatter_c64(AdjArgs<double> a, const uint32_t* order, int chunk) {
+    __shared__ __align__(16) double s_rec[DMPM_CHUNK_THREADS * kRec64];
+    ChunkLane64 L;
+    if (!chunk_lane64(L, order, a.n, chunk, a.st, a.np, a.geo)) return;
+    double* rec = s_rec + (threadIdx.x & ~31) * kRec64;
+    if (L.valid) {
+        const int p = L.p;
+        const m3<double> Fe = load_m3(a.st + (size_t)PF * a.np, a.np, p) + load_m3(a.dfc, a.np, p);
+        double b[4];
+        m3<double> Cn;
+        adj_next_terms<double, EXACT>(a, p, Fe, b, Cn);
+        b[3] = 0.0;
+        if (a.dbg_vnext) {
+#pragma unroll
+            for (int c = 0; c < 3; c++) a.dbg_vnext[(size_t)c * a.np + p] = b[c];
+            store_m3(a.dbg_Cnext, a.np, p, Cn);
+        }
+        chunk_record64(rec + L.grp.slot * kRec64, L.w, b, (3.0 / (a.geo.dx * a.geo.dx)) * Cn);
+    }
+    __syncwarp();
+    chunk_scatter64<3>(rec, L.base, L.grp, a.geo, a.gadj);
+}
+
 }  // namespace dmpm

@@ -318,4 +318,9 @@ template <class T> DMPM_HD bool polar_newton(const m3<T>& F, m3<T>& R, m3<T>& S)
     return true;
 }
 
+// polar factors: the Newton iteration where it applies, else the SVD
+template <class T> DMPM_HD void polar(const m3<T>& F, m3<T>& R, m3<T>& S) {
+    if (!polar_newton(F, R, S)) polar3(F, R, S);
+}
+
 }  // namespace dmpm

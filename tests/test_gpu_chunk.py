@@ -61,3 +61,28 @@ def test_chunks_match_fp64_oracle(gpu_ready, n, general, adjoint):
             if f == "dLdFe" and adjoint != "exact":
                 continue
             assert normrel(c.get(0, f), o.get(0, f)) < 1e-3, f
+
+
+@pytest.mark.parametrize("n,adjoint", [(1, "exact"), (31, "exact"), (33, "refcompat"), (128, "exact"), (129, "exact"),
+                                       (421, "refcompat"), (421, "exact")])
+def test_fp64_chunks_match_fp64_oracle(gpu_ready, n, adjoint):
+    """The FP64 path's P2G and adjoint scatter over chunks: the bars of the other
+    FP64 tests, as the sums differ from the oracle's by their order alone."""
+    sc = _cloud(n, 300 + n)
+    o = OracleGraph(sc, "f64")
+    o.setup(L, sc.dt, sc.drag, sc.f_ext, sc.smoothing)
+    o.forward(0)
+    loss = o.loss()
+    o.backward(0, 1 if adjoint == "exact" else 0)
+    with make_ctx(sc, "fp64", o.target, adjoint=adjoint, keep_adjoints=True, sort_every=50) as c:
+        c.setup(L)
+        c.forward(0)
+        assert abs(c.loss() - loss) <= 1e-10 * abs(loss)
+        c.backward(0)
+        for l in (0, L - 2):
+            assert relerr(c.get_grid(l, "grid_m"), o.get(l, "grid_m")) < 1e-10
+            assert relerr(c.get_grid(l, "grid_p"), o.get(l, "grid_p")) < 1e-10
+        for f in ("x", "F", "v", "C"):
+            assert relerr(c.get(L - 1, f), o.get(L - 1, f)) < 1e-10, f
+        for f in ("dLdx", "dLdv", "dLdF", "dLdC"):
+            assert normrel(c.get(0, f), o.get(0, f)) < 1e-8, f
