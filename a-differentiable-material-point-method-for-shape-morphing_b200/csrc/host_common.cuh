@@ -8,6 +8,8 @@
 #include <string>
 #include <vector>
 
+#include "scratch.cuh"
+
 namespace dmpm_host {
 
 struct CudaError {
@@ -56,6 +58,11 @@ class Arena {
                                                            std::to_string(budget_->cap)};
         void* p = nullptr;
         cudaError_t e = cudaMalloc(&p, want);
+        if (e == cudaErrorMemoryAllocation) {  // take back what the scratch pool keeps, and try once more
+            cudaGetLastError();
+            scratch_trim();
+            e = cudaMalloc(&p, want);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             throw CudaError{e, "cudaMalloc(" + std::to_string(bytes) + " bytes): " + cudaGetErrorString(e)};

@@ -43,6 +43,7 @@
 #include <vector>
 
 #include "dmpm.h"
+#include "scratch.cuh"
 #include "sort.cuh"
 
 namespace {
@@ -325,22 +326,6 @@ void make_patches(const std::vector<float>& tri, int nf, Mesh& m) {
     }
 }
 
-// device memory of one call
-struct DeviceMem {
-    std::vector<void*> ptrs;
-    ~DeviceMem() {
-        for (void* p : ptrs) cudaFree(p);
-    }
-    template <class T> T* alloc(size_t count) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(1, count) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        ptrs.push_back(p);
-        return (T*)p;
-    }
-};
 int cuda_failed() {
     cudaGetLastError();
     return DMPM_ERR_CUDA;
@@ -357,7 +342,7 @@ int inside_points(const std::vector<float>& tri, int nf, const Points& pts, cons
     make_patches(tri, nf, m);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     const int tiles = (int)((blocks + SCAN_TILE - 1) / SCAN_TILE);
-    DeviceMem mem;
+    dmpm_host::Scratch mem;
     float* dtri = mem.alloc<float>(m.tri.size() + m.edges.size());
     Patch* dpat = mem.alloc<Patch>(m.patches.size());
     uint32_t* dmask = mem.alloc<uint32_t>((size_t)blocks * 9 + tiles + 2);

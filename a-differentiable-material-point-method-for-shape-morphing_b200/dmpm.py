@@ -679,16 +679,19 @@ def extract_surface(field, dims, dx: float, min_point, iso: float):
     f = _f32(field)
     d, mn = _dims(dims), _f32(min_point)
     nv, nf = ctypes.c_int64(), ctypes.c_int64()
-    st = lib.dmpm_surface_extract(f.ctypes.data, d.ctypes.data, float(dx), mn.ctypes.data, float(iso), None, 0, None,
-                                  0, ctypes.byref(nv), ctypes.byref(nf))
-    if st not in (OK, ERR_TOO_LARGE):
-        raise DmpmError(st, "extract_surface")
-    V = np.empty((nv.value, 3), dtype=np.float32)
-    F = np.empty((nf.value, 3), dtype=np.int32)
-    _surf_ck(lib.dmpm_surface_extract(f.ctypes.data, d.ctypes.data, float(dx), mn.ctypes.data, float(iso),
-                                      V.ctypes.data, nv.value, F.ctypes.data, nf.value, ctypes.byref(nv),
-                                      ctypes.byref(nf)), "extract_surface")
-    return V, F
+    # room for a surface of about one crossing per node of 8 grid faces; a larger one is asked for again
+    cv = 4096 + int(min(4e6, 8.0 * max(0.0, float(np.prod(d.astype(np.float64)))) ** (2.0 / 3.0)))
+    cf = 2 * cv
+    for _ in range(2):
+        V = np.empty((cv, 3), dtype=np.float32)
+        F = np.empty((cf, 3), dtype=np.int32)
+        st = lib.dmpm_surface_extract(f.ctypes.data, d.ctypes.data, float(dx), mn.ctypes.data, float(iso),
+                                      V.ctypes.data, cv, F.ctypes.data, cf, ctypes.byref(nv), ctypes.byref(nf))
+        if st != ERR_TOO_LARGE or (nv.value <= cv and nf.value <= cf):
+            break
+        cv, cf = nv.value, nf.value
+    _surf_ck(st, "extract_surface")
+    return V[: nv.value].copy(), F[: nf.value].copy()
 
 
 def marching_cubes_point_cloud(points, iso_mass: float, grid_dx: float, quality: float, min_point, max_point):
