@@ -15,12 +15,15 @@
 //   The half angles are summed as the product of the complex numbers den + i det,
 // with a count of the times it passes the negative real axis: one atan2 per point
 // in place of one per triangle, whose FP64 instructions were the kernel's cost.
-//   The triangles are cut into patches.  A surface's solid angle from a point is
-// that of any surface with the same boundary that the point is not between, so a
-// patch is summed triangle by triangle only for warps with a point in its bounding
-// box; for all others by the fan over its boundary edges from one of its
-// vertices, which lies in the box too (Jacobson, Kavan and Sorkine-Hornung 2013).
-// The fan has about 4 sqrt(triangles) triangles, each with one new vertex.
+//   The triangles are cut into a tree of patches.  A surface's solid angle from a
+// point is that of any surface with the same boundary that the point is not
+// between, so a warp with a point in a patch's bounding box goes on to its two
+// halves (a leaf is summed triangle by triangle), and any other takes the fan over
+// the patch's boundary edges from one of its vertices, which lies in the box too
+// (Jacobson, Kavan and Sorkine-Hornung 2013).  A fan has about 4 sqrt(triangles)
+// triangles, each with one new vertex.  2.7M points inside 4.4M candidates and
+// 1,152 triangles, kernel ms: 29.8 triangle by triangle with an atan2 each, 9.3
+// with one level of patches of up to 64, 3.33 with the tree.
 //   The kept points are compacted on the GPU in lattice order.  The lattice
 // coordinates are formed in float with the reference's two roundings.
 //
@@ -48,9 +51,9 @@
 
 namespace {
 
-// triangles per patch, at most: at 1,152 triangles 64 makes 18 patches of about 25
-// boundary edges
-constexpr int kPatchTriangles = 64;
+// triangles of a leaf patch, at most.  Wall ms at 1,152 / 144 / 24,000 triangles: 16: 8.7 /
+// 2.3 / 27.1; 24: 7.8 / 2.5 / 24.5; 40: 7.9 / 2.9 / 24.1; 72: 9.2 / 3.0 / 21.8.
+constexpr int kPatchTriangles = 40;
 
 // the lattice point min_point + sampling_dx * (i, j, k): a product and a sum, each rounded to float
 struct LatticePoints {
@@ -86,11 +89,12 @@ struct JitteredPoints {
     }
 };
 
-// One patch: its triangles [t0, t1), its boundary fan's edges [e0, e1) around
-// apex, and its bounding box.  e0 = e1 and far = 0: no cheaper fan.
+// One patch, the tree in depth-first order: its bounding box, its boundary fan's
+// edges [e0, e1) around apex (far = 0: no fan that costs less than the triangles),
+// the patch after its subtree, and a leaf's triangles [t0, t1).
 struct Patch {
     float lo[3], hi[3], apex[3];
-    int t0, t1, e0, e1, far;
+    int t0, t1, e0, e1, far, skip;
 };
 
 struct Vec {
@@ -138,7 +142,7 @@ __global__ void __launch_bounds__(256) k_mesh_winding(const float* __restrict__ 
     double p[3];
     pts(i, j, k, p);
     AngleSum sum;
-    for (int n = 0; n < np; n++) {
+    for (int n = 0; n < np;) {
         const Patch& P = patches[n];
         bool near = !P.far;
         if (P.far) {
@@ -147,6 +151,7 @@ __global__ void __launch_bounds__(256) k_mesh_winding(const float* __restrict__ 
             for (int a = 0; a < 3; a++) in &= p[a] >= (double)P.lo[a] && p[a] <= (double)P.hi[a];
             near = __any_sync(0xffffffffu, in || !(p[0] == p[0]));
         }
+        n = near ? n + 1 : P.skip;  // an inner patch's halves follow it
         if (near) {
             for (int t = P.t0; t < P.t1; t++) {
                 const float* v = tri + 9 * (size_t)t;
@@ -219,39 +224,57 @@ int gather_triangles(const float* V, int nv, const int* F, int nf, std::vector<f
     return DMPM_OK;
 }
 
-// The triangles in patches of at most kPatchTriangles, split at the median
-// centroid of the longest axis, and each patch's boundary edges: 7 floats each, the
-// two ends and 1 where the first end is the edge before's second (the edges are
-// chained as far as they go).
+// The triangles in a tree of patches, split at the median centroid of the longest
+// axis, and each patch's boundary edges: 7 floats each, the two ends and 1 where the
+// first end is the edge before's second (the edges are chained as far as they go).
 struct Mesh {
     std::vector<float> tri, edges;
     std::vector<Patch> patches;
 };
-void make_patches(const std::vector<float>& tri, int nf, Mesh& m) {
-    // vertices by position, so that unwelded meshes have inner edges too
-    auto hash = [](const std::array<float, 3>& x) {
-        uint32_t u[3];
-        std::memcpy(u, x.data(), sizeof u);
-        return (size_t)splitmix64(((uint64_t)u[0] << 32 | u[1]) ^ splitmix64(u[2]));
-    };
-    std::unordered_map<std::array<float, 3>, int, decltype(hash)> ids((size_t)nf * 2, hash);
-    std::vector<int> vid((size_t)nf * 3);
-    for (size_t v = 0; v < vid.size(); v++) {
-        const float* x = &tri[3 * v];
-        const std::array<float, 3> key{x[0] + 0.f, x[1] + 0.f, x[2] + 0.f};  // -0 + 0 = 0
-        if (!(std::isfinite(x[0]) && std::isfinite(x[1]) && std::isfinite(x[2]))) {
-            vid[v] = -1 - (int)v;  // its own vertex: NaN has no order
-            continue;
+class PatchTree {
+   public:
+    PatchTree(const std::vector<float>& tri, int nf, Mesh& m) : tri_(tri), m_(m), order_((size_t)nf), vid_((size_t)nf * 3) {
+        // vertices by position, so that unwelded meshes have inner edges too
+        auto hash = [](const std::array<float, 3>& x) {
+            uint32_t u[3];
+            std::memcpy(u, x.data(), sizeof u);
+            return (size_t)splitmix64(((uint64_t)u[0] << 32 | u[1]) ^ splitmix64(u[2]));
+        };
+        std::unordered_map<std::array<float, 3>, int, decltype(hash)> ids((size_t)nf * 2, hash);
+        for (size_t v = 0; v < vid_.size(); v++) {
+            const float* x = &tri[3 * v];
+            if (!(std::isfinite(x[0]) && std::isfinite(x[1]) && std::isfinite(x[2]))) {
+                vid_[v] = -1;  // its patches have no fan
+                continue;
+            }
+            const std::array<float, 3> key{x[0] + 0.f, x[1] + 0.f, x[2] + 0.f};  // -0 + 0 = 0
+            const auto it = ids.emplace(key, (int)at_.size());
+            if (it.second) at_.push_back(x);
+            vid_[v] = it.first->second;
         }
-        vid[v] = ids.emplace(key, (int)ids.size()).first->second;
+        std::iota(order_.begin(), order_.end(), 0);
+        Edges net;
+        build(0, nf, net);
     }
-    std::vector<int> order(nf);
-    std::iota(order.begin(), order.end(), 0);
-    auto centre = [&](int f, int a) { return tri[9 * (size_t)f + a] + tri[9 * (size_t)f + 3 + a] + tri[9 * (size_t)f + 6 + a]; };
-    std::vector<std::pair<int, int>> todo{{0, nf}};
-    while (!todo.empty()) {
-        const auto [b, e] = todo.back();
-        todo.pop_back();
+
+   private:
+    using Edges = std::map<std::pair<int, int>, int>;  // directed edges that no opposite one cancels
+    static void add_edge(Edges& net, int u, int v, int times) {
+        const auto back = net.find({v, u});
+        if (back != net.end()) {
+            const int gone = std::min(times, back->second);
+            if ((back->second -= gone) == 0) net.erase(back);
+            times -= gone;
+        }
+        if (times > 0) net[{u, v}] += times;
+    }
+    float centre(int f, int a) const {
+        return tri_[9 * (size_t)f + a] + tri_[9 * (size_t)f + 3 + a] + tri_[9 * (size_t)f + 6 + a];
+    }
+    // the patch of order_[b, e) and its subtree; its boundary into net
+    void build(int b, int e, Edges& net) {
+        const size_t self = m_.patches.size();
+        m_.patches.push_back(Patch{});
         Patch P{};
         for (int a = 0; a < 3; a++) {
             P.lo[a] = INFINITY;
@@ -260,71 +283,69 @@ void make_patches(const std::vector<float>& tri, int nf, Mesh& m) {
         bool finite = true;
         for (int i = b; i < e; i++)
             for (int c = 0; c < 9; c++) {
-                const float x = tri[9 * (size_t)order[i] + c];
+                const float x = tri_[9 * (size_t)order_[i] + c];
                 finite &= std::isfinite(x);
                 P.lo[c % 3] = std::min(P.lo[c % 3], x);
                 P.hi[c % 3] = std::max(P.hi[c % 3], x);
             }
+        P.t0 = P.t1 = (int)(m_.tri.size() / 9);
         if (finite && e - b > kPatchTriangles) {
             int axis = 0;
             for (int a = 1; a < 3; a++)
                 if (P.hi[a] - P.lo[a] > P.hi[axis] - P.lo[axis]) axis = a;
             const int mid = b + (e - b) / 2;
-            std::nth_element(order.begin() + b, order.begin() + mid, order.begin() + e,
+            std::nth_element(order_.begin() + b, order_.begin() + mid, order_.begin() + e,
                              [&](int f, int g) { return centre(f, axis) < centre(g, axis); });
-            todo.push_back({mid, e});
-            todo.push_back({b, mid});
-            continue;
-        }
-        P.t0 = (int)(m.tri.size() / 9);
-        std::map<std::pair<int, int>, int> net;  // directed edges that no opposite one cancels
-        std::map<int, const float*> at;
-        for (int i = b; i < e; i++) {
-            const size_t f = (size_t)order[i];
-            m.tri.insert(m.tri.end(), tri.begin() + 9 * f, tri.begin() + 9 * f + 9);
-            for (int c = 0; c < 3; c++) {
-                const int u = vid[3 * f + c], v = vid[3 * f + (c + 1) % 3];
-                at[u] = &tri[9 * f + 3 * c];
-                if (u == v) continue;
-                const auto back = net.find({v, u});
-                if (back == net.end()) net[{u, v}]++;
-                else if (--back->second == 0) net.erase(back);
+            Edges right;
+            build(b, mid, net);
+            build(mid, e, right);
+            for (const auto& n : right) add_edge(net, n.first.first, n.first.second, n.second);
+        } else {
+            for (int i = b; i < e; i++) {
+                const size_t f = (size_t)order_[i];
+                m_.tri.insert(m_.tri.end(), tri_.begin() + 9 * f, tri_.begin() + 9 * f + 9);
+                for (int c = 0; c < 3 && finite; c++) {
+                    const int u = vid_[3 * f + c], v = vid_[3 * f + (c + 1) % 3];
+                    if (u != v) add_edge(net, u, v, 1);
+                }
             }
+            P.t1 = (int)(m_.tri.size() / 9);
         }
-        P.t1 = (int)(m.tri.size() / 9);
         int left = 0;
         for (const auto& n : net) left += n.second;
-        // a fan triangle costs about half a triangle of its own
-        P.far = finite && left < 2 * (P.t1 - P.t0) ? 1 : 0;
-        P.e0 = (int)(m.edges.size() / 7);
-        if (P.far && left > 0) {
-            const int apex = net.begin()->first.first;
-            std::copy(at[apex], at[apex] + 3, P.apex);
-            int prev = -1;
-            bool chained = false;
-            while (!net.empty()) {
-                auto it = chained ? net.lower_bound({prev, INT_MIN}) : net.begin();
-                if (chained && (it == net.end() || it->first.first != prev)) {
-                    chained = false;
-                    continue;
-                }
-                const auto [u, v] = it->first;
-                if (--it->second == 0) net.erase(it);
-                if (u != apex && v != apex) {  // an edge at the apex spans no triangle
-                    const bool follows = chained && m.edges.size() / 7 > (size_t)P.e0 &&
-                                         std::equal(at[u], at[u] + 3, &m.edges[m.edges.size() - 4]);
-                    m.edges.insert(m.edges.end(), at[u], at[u] + 3);
-                    m.edges.insert(m.edges.end(), at[v], at[v] + 3);
-                    m.edges.push_back(follows ? 1.f : 0.f);
-                }
-                prev = v;
-                chained = true;
-            }
-        }
-        P.e1 = (int)(m.edges.size() / 7);
-        m.patches.push_back(P);
+        // a fan triangle costs about half of one of the patch's
+        P.far = finite && left < 2 * (e - b) ? 1 : 0;
+        P.e0 = (int)(m_.edges.size() / 7);
+        if (P.far && left > 0) fan(net, P);
+        P.e1 = (int)(m_.edges.size() / 7);
+        P.skip = (int)m_.patches.size();
+        m_.patches[self] = P;
     }
-}
+    void fan(Edges net, Patch& P) {
+        const int apex = net.begin()->first.first;
+        std::copy(at_[apex], at_[apex] + 3, P.apex);
+        const size_t first = m_.edges.size();
+        int prev = -1, last = -1;  // the chain's end, and the last stored edge's
+        while (!net.empty()) {
+            auto it = prev >= 0 ? net.lower_bound({prev, INT_MIN}) : net.begin();
+            if (it == net.end() || (prev >= 0 && it->first.first != prev)) it = net.begin();
+            const auto [u, v] = it->first;
+            if (--it->second == 0) net.erase(it);
+            prev = v;
+            if (u == apex || v == apex) continue;  // an edge at the apex spans no triangle
+            const bool follows = m_.edges.size() > first && last == u;
+            m_.edges.insert(m_.edges.end(), at_[u], at_[u] + 3);
+            m_.edges.insert(m_.edges.end(), at_[v], at_[v] + 3);
+            m_.edges.push_back(follows ? 1.f : 0.f);
+            last = v;
+        }
+    }
+
+    const std::vector<float>& tri_;
+    Mesh& m_;
+    std::vector<int> order_, vid_;
+    std::vector<const float*> at_;  // a vertex's position
+};
 
 int cuda_failed() {
     cudaGetLastError();
@@ -339,7 +360,7 @@ int inside_points(const std::vector<float>& tri, int nf, const Points& pts, cons
     using namespace dmpm;
     const long long total = (long long)dims[0] * dims[1] * dims[2];
     Mesh m;
-    make_patches(tri, nf, m);
+    PatchTree(tri, nf, m);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     const int tiles = (int)((blocks + SCAN_TILE - 1) / SCAN_TILE);
     dmpm_host::Scratch mem;
