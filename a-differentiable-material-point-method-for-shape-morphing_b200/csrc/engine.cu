@@ -1156,11 +1156,15 @@ template <class T> class Engine : public EngineBase {
     }
 
     // One ForwardTimeStep: layer l -> out (state of l+1), grid g, G of layer l
-    // in Gd.  FP32 path: g_ready = Gd already holds layer l's G (the previous
-    // step's G2P formed it), so the stress stage is skipped; Gd_next non-null =
-    // the G2P also forms layer l+1's G there.  Returns whether it did.
-    bool step(int l, const T* st, T* out, node4<T>* g, T* Gd, bool allow_sort, bool g_ready = false,
-              T* Gd_next = nullptr) {
+    // in Gd.  FP32 path: done says what the step before left for this one, and is
+    // set to what this one leaves; Gd_next non-null = the G2P also forms layer l+1's
+    // G there, g_next non-null = the grid update also clears layer l+1's grid.
+    struct StepDone {
+        bool stress = false;   // Gd holds layer l's G
+        bool cleared = false;  // g is zero
+    };
+    void step(int l, const T* st, T* out, node4<T>* g, T* Gd, bool allow_sort, StepDone& done, T* Gd_next = nullptr,
+              node4<T>* g_next = nullptr) {
         if constexpr (kWarp) {
             ensure_fix();  // allocated already (no-ops) on every captured path
             ensure_groups();
@@ -1180,15 +1184,16 @@ template <class T> class Engine : public EngineBase {
                 a.fixb = fixb_;
                 clear_fix(-1);
             } else {
-                int* box = box_of(g);
-                k_box_clear<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, box, box > boxes_ ? box - 6 : nullptr,
-                                                                    geo_);
-                launched();
-                a.box = box;
+                a.box = box_of(g);
+                if (!done.cleared) {
+                    k_box_clear<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, a.box,
+                                                                        a.box > boxes_ ? a.box - 6 : nullptr, geo_);
+                    launched();
+                }
             }
             const unsigned ws = warp_blocks(DMPM_SCATTER_CTAS, DMPM_P2G_THREADS);
             const int ush = set_units(a, ep);
-            if (dm || !g_ready) {
+            if (dm || !done.stress) {
                 pbeg(K_P_OP1);
                 if (dm) k_stress<true><<<pgrid256(), 256, 0, ctx_->stream>>>(a);
                 else k_stress<false><<<pgrid256(), 256, 0, ctx_->stream>>>(a);
@@ -1215,8 +1220,11 @@ template <class T> class Engine : public EngineBase {
             }
             pend();
             pbeg(K_GOP);
-            k_box_gop<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, dm ? box_full_ : a.box,
-                                                              dm ? box_of(g) : nullptr, geo_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
+            const bool clear_next = g_next && !dm;
+            k_box_gop<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, dm ? box_full_ : a.box, dm ? box_of(g) : nullptr,
+                                                              clear_next ? (node4<float>*)g_next : nullptr,
+                                                              clear_next ? box_of(g_next) : nullptr, geo_, a.dt, a.fext[0],
+                                                              a.fext[1], a.fext[2]);
             launched();
             pend();
             // the deterministic mode keeps the standalone stress stage: it also raises the
@@ -1232,7 +1240,8 @@ template <class T> class Engine : public EngineBase {
             launch_g2p<false>(a, ctx_->stream);
             launched();
             pend();
-            return fuse;
+            done = StepDone{fuse, clear_next};
+            return;
         }
         FwdArgs<T> a = fwd_args();
         a.st = st;
@@ -1263,9 +1272,9 @@ template <class T> class Engine : public EngineBase {
             launched();
             pend();
         }
-        (void)g_ready;
+        (void)done;
         (void)Gd_next;
-        return false;
+        (void)g_next;
     }
 
     void reset_status() {
@@ -1325,10 +1334,10 @@ template <class T> class Engine : public EngineBase {
         ensure_groups();
         if (k_ == 1) {
             auto body = [&]() {
-                bool ready = false;  // layer l's G formed by the previous step
+                StepDone done;
                 for (int l = start; l + 1 < L_; l++)
-                    ready = step(l, layers_[l].st, layers_[l + 1].st, layers_[l].grid, layers_[l].G, true, ready,
-                                 l + 2 < L_ ? layers_[l + 1].G : nullptr);
+                    step(l, layers_[l].st, layers_[l + 1].st, layers_[l].grid, layers_[l].G, true, done,
+                         l + 2 < L_ ? layers_[l + 1].G : nullptr, l + 2 < L_ ? layers_[l + 1].grid : nullptr);
             };
             if (graphs_ok()) {
                 run_graph({0, start}, body);
@@ -1344,13 +1353,14 @@ template <class T> class Engine : public EngineBase {
         } else {
             const T* cur = materialize_state(start);
             int r = 0;
-            bool ready = false;
+            StepDone done;
             for (int l = start; l + 1 < L_; l++) {
                 T* out = layers_[l + 1].st ? layers_[l + 1].st : ring_[r];
                 if (!layers_[l + 1].st) r ^= 1;
                 // the current state may live in ring_[r] already (ping-pong); layer l's G in
                 // gscratch_ is read by P2G before G2P writes layer l+1's there
-                ready = step(l, cur, out, seg_grid_[0], gscratch_, true, ready, l + 2 < L_ ? gscratch_ : nullptr);
+                step(l, cur, out, seg_grid_[l & 1], gscratch_, true, done, l + 2 < L_ ? gscratch_ : nullptr,
+                     l + 2 < L_ ? seg_grid_[(l & 1) ^ 1] : nullptr);
                 cur = out;
             }
             seg_lo_ = seg_hi_ = -1;  // segment scratch no longer matches
@@ -1371,18 +1381,18 @@ template <class T> class Engine : public EngineBase {
     void materialize_segment(int c) {
         const int e = std::min(c + k_, L_ - 1);
         const T* cur = layers_[c].st;
-        bool ready = false;
+        StepDone done;
         for (int l = c; l < e; l++) {
             T* out = (l + 1 == e) ? nullptr : seg_st_[l - c];
             T* Gd = seg_G_.empty() ? nullptr : seg_G_[l - c];
             if (out) {
-                ready = step(l, cur, out, seg_grid_[l - c], Gd, false, ready,
-                             seg_G_.empty() ? nullptr : seg_G_[l + 1 - c]);
+                step(l, cur, out, seg_grid_[l - c], Gd, false, done, seg_G_.empty() ? nullptr : seg_G_[l + 1 - c],
+                     seg_grid_[l + 1 - c]);
                 cur = out;
             } else {
                 // last step of the segment: only its grid is needed; the output
                 // (layer e) is a stored layer already, write it to scratch ring
-                step(l, cur, ring_[0], seg_grid_[l - c], Gd, false, ready);
+                step(l, cur, ring_[0], seg_grid_[l - c], Gd, false, done);
             }
         }
         seg_lo_ = c;

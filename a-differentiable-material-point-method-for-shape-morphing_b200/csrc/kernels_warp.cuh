@@ -555,7 +555,7 @@ __device__ __forceinline__ void widen_box(int* box, int have, const GridGeom& g,
 }
 // zero the nodes of the layer's box, then take in the box `prev` (or null).  A block
 // may read the box while it grows: it then clears more, which is zero already.
-static __global__ void __launch_bounds__(256) k_box_clear(node4<float>* grid, int* box, const int* prev, GridGeom g) {
+__device__ __forceinline__ void box_clear(node4<float>* grid, int* box, const int* prev, const GridGeom& g) {
     const NodeRange r(box);
     for (int row = first_warp(); row < r.rows(); row += warp_count()) {
         node4<float>* p = grid + r.first(row, g);
@@ -566,11 +566,18 @@ static __global__ void __launch_bounds__(256) k_box_clear(node4<float>* grid, in
         box[threadIdx.x] = threadIdx.x < 3 ? min(a, b) : max(a, b);
     }
 }
+static __global__ void __launch_bounds__(256) k_box_clear(node4<float>* grid, int* box, const int* prev, GridGeom g) {
+    box_clear(grid, box, prev, g);
+}
 // the grid update over the box; mark: the box to set to it (the deterministic mode
-// fills its grids whole), or null
+// fills its grids whole), or null; next: the next layer's grid, cleared as by
+// k_box_clear for a launch less per step (8.7k particles: 39.9 -> 38.7 us a step
+// forward and back), or null
 static __global__ void __launch_bounds__(256)
-    k_box_gop(node4<float>* grid, const int* __restrict__ box, int* mark, GridGeom g, float dt, float f0, float f1, float f2) {
+    k_box_gop(node4<float>* grid, const int* box, int* mark, node4<float>* next, int* next_box, GridGeom g, float dt,
+              float f0, float f1, float f2) {
     const NodeRange r(box);
+    if (next) box_clear(next, next_box, box, g);
     const float f[3] = {f0, f1, f2};
     if (mark && blockIdx.x == 0 && threadIdx.x < 6) mark[threadIdx.x] = box[threadIdx.x];
     for (int row = first_warp(); row < r.rows(); row += warp_count()) {
