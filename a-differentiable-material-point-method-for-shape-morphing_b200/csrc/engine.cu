@@ -263,7 +263,9 @@ namespace {
 
 template <class T> class Engine : public EngineBase {
    public:
-    // FP32 path: cell-sorted warp items (kernels_warp.cuh); FP64 path: plain kernels (kernels.cuh)
+    // FP32 path: chunks of the cell-sorted order (kernels_chunk.cuh), in the deterministic
+    // mode P2G and the adjoint scatter over warp items and units (kernels_warp.cuh,
+    // kernels_brick.cuh); FP64 path: kernels.cuh, its scatters in kernels_chunk.cuh
     static constexpr bool kTiled = std::is_same<T, float>::value;
     static constexpr bool kWarp = kTiled;
     // the FP32 path stores each layer's strain H = F - I in the F planes (kernels_warp.cuh)
@@ -271,7 +273,7 @@ template <class T> class Engine : public EngineBase {
     // state planes per layer: the FP32 path adds the low parts of its
     // compensated positions (PXL); adjoint layers keep NSTATE planes
     static constexpr int kNst = kWarp ? (int)NSTATE_X : (int)NSTATE;
-    // one cell sort: the stable order and warp items used for steps
+    // one cell sort: the order (deterministic mode: and warp items) used for steps
     // [e * sort_every, (e + 1) * sort_every)
     struct Epoch {
         uint32_t* order = nullptr;
@@ -767,6 +769,7 @@ template <class T> class Engine : public EngineBase {
         drop_graphs();
         try {
             allocate_layers(num_layers);
+            ensure_groups();
         } catch (...) {
             // out of device memory (or over the context's device byte limit):
             // drop the partial storage so the context reads as not set up, and
@@ -979,18 +982,22 @@ template <class T> class Engine : public EngineBase {
     }
 
     // items and units of every epoch, which only the deterministic mode reads;
-    // like its integer grid allocated on first use, before any capture
+    // allocated by dmpm_setup, or before any capture when the mode is set later
     void ensure_groups() {
         if (!det() || epochs_.empty() || epochs_[0].items) return;
         group_arena_.release();
         drop_graphs();
+        // one allocation: the six buffers of each epoch apart took a first pass 15 ms
+        const size_t len = ((size_t)n_ + 1 + 63) / 64 * 64, per_epoch = 4 * len + 64;
+        uint32_t* p = (uint32_t*)group_arena_.alloc(epochs_.size() * per_epoch * sizeof(uint32_t));
         for (Epoch& e : epochs_) {
-            e.items = (uint32_t*)group_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
-            e.n_items = (uint32_t*)group_arena_.alloc(16);
-            e.units = (uint32_t*)group_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
-            e.unit_keys = (uint32_t*)group_arena_.alloc((size_t)n_ * sizeof(uint32_t));
-            e.unit_items = (uint32_t*)group_arena_.alloc(((size_t)n_ + 1) * sizeof(uint32_t));
-            e.n_units = (uint32_t*)group_arena_.alloc(16);
+            e.items = p;
+            e.units = p + len;
+            e.unit_keys = p + 2 * len;
+            e.unit_items = p + 3 * len;
+            e.n_items = p + 4 * len;
+            e.n_units = p + 4 * len + 32;
+            p += per_epoch;
         }
     }
 
@@ -2073,7 +2080,7 @@ void dmpm_default_params(dmpm_params* p) {
     p->adjoint_mode = DMPM_ADJ_REFCOMPAT;
     p->control_mode = DMPM_CTRL_PER_LAYER;
     p->loss_kind = DMPM_LOSS_REF_LOGMASS;
-    p->brick_cells = 2;  // G2P over 2^3-cell bricks (36.7 against 48.1 us per step on 64^3, 267k particles)
+    p->brick_cells = 2;  // the deterministic mode's tiles
 }
 
 int dmpm_create(int device, int precision, dmpm_ctx** out) {
