@@ -8,15 +8,13 @@
 // of that order, stored with its own plane stride S_t.  Time step t advances
 // the instances with steps > t, again a prefix: P_t particles, G_t nodes.
 //
-// Launches.  Every stage of a time step is one launch over the prefix: the
-// per-particle kernels (k_stress, k_adj_finalize) over P_t particles, the node
-// kernels over G_t nodes, and the warp-item kernels (P2G, G2P, adjoint
-// scatter and gather) as persistent grids of ctas_per_sm CTAs per SM looping
-// over the warp items of the active instances.  Items never mix instances
-// (cell keys carry the instance's key offset); each warp looks up its item's
-// grid.  The item count lives on the device -- the cell sort writes the end
-// of every instance's items -- so no result is read back inside a gradient
-// evaluation and the whole evaluation can be captured once as a CUDA graph.
+// Launches.  Every stage of a time step is one launch over the prefix: P2G, G2P
+// with the next step's stress stage, the adjoint scatter and the gather with the
+// finalize (kernels_chunk.cuh) over P_t particles in cell order, the node kernels
+// over G_t nodes.  A cell's particles never mix instances (cell keys carry the
+// instance's key offset); each lane looks up its particle's grid.  No result is
+// read back inside a gradient evaluation, so the whole evaluation can be
+// captured once as a CUDA graph.
 //
 // Losses.  EndLayerMassLoss (CompGraph.cpp:110-244) of instance i is
 // evaluated on its last layer when the backward sweep reaches that layer; its

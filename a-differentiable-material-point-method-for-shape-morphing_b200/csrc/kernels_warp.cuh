@@ -1,4 +1,7 @@
-// kernels_warp.cuh -- FP32 path kernels organised around cell-sorted warp items.
+// kernels_warp.cuh -- FP32 path: what its kernels share (WArgs, the stress and
+// finalize arithmetic, node passes and node boxes) and the deterministic mode's P2G
+// and adjoint scatter over cell-sorted warp items.  The float mode's stencil kernels
+// are in kernels_chunk.cuh.
 //
 // GENERAL (a test switch) forces the per-lane reductions everywhere.
 //
@@ -12,9 +15,8 @@
 // owning one node's complete sum and issues a single vector
 // red.global.add.v4.f32 per 8 nodes x 4 values; otherwise every lane issues
 // its own reductions.  Gathers sum the 16-node partial results of the 4 slab
-// lanes with two xor-shuffles.  The FP64 polar decomposition lives in the
-// per-particle kernels k_stress (forward) and k_adj_finalize (adjoint), so
-// the node loops keep a small register footprint.
+// lanes with two xor-shuffles.  The FP64 polar decomposition is stress_particle's
+// (k_stress, or G2P for the next step) and finalize_particle's (the gather).
 //
 // Math per stage is that of kernels.cuh (which cites the reference).
 //

@@ -179,8 +179,8 @@ def build_scene(instance: int, ppc_root: int):
     return sc
 
 
-# G2P kernel of the FP32 path: None = the library default (bricks of 2^3 cells), 0 = warp
-# items, 2 or 4 = bricks of that many cells per axis
+# node tiles of the deterministic mode's P2G and adjoint scatter: None = the library default
+# (bricks of 2^3 cells), 0 = none, 2 or 4 = bricks of that many cells per axis
 BRICK_CELLS = None
 # cell-sort interval of the FP32 path (None = the library default, 8 steps)
 SORT_EVERY = None
@@ -246,11 +246,11 @@ def timed_steps(torch, c, steps, fn):
     return e0.elapsed_time(e1)
 
 
-# Algorithmic bytes per launch of each kernel of the FP32 path: every particle
+# Algorithmic bytes of each stage of the FP32 path taken by itself: every particle
 # plane it must read or write once (4 B per FP32 value, the FP64 tied-control
-# accumulator 8 B), the sorted-order index of the warp-item kernels (4 B per
-# particle), and its grid records: per touched node for the particle-parallel
-# kernels, per grid node for the node-parallel ones.
+# accumulator 8 B), the sorted-order index (4 B per particle), and its grid records:
+# per touched node for the particle-parallel stages, per grid node for the
+# node-parallel ones.  The kernels as they are launched: launch_bytes.
 # (positions are compensated float pairs, hi + lo: 6 floats per particle)
 PER_PARTICLE_BYTES = {
     "p_op1": (9 + 9 + 4 + 9) * 4 + 24 * 4,                  # F, dFc, m/vol/lam/mu, C -> G, R, S
@@ -258,7 +258,7 @@ PER_PARTICLE_BYTES = {
     "g2p_p_op2": (6 + 9 + 9 + 1) * 4 + 27 * 4,              # x, F, dFc, order -> x, v, C, F
     "adj_g2p_scatter": (6 + 24 + 9 + 9 + 1) * 4 + 12 * 4,   # x, adjoint', F, dFc, order -> dLdv', dLdC'
     "adj_p2g_gather": (6 + 1 + 3 + 12 + 9 + 1) * 4 + 18 * 4,  # x, m, v, dLdv'/dLdC', G, order -> M, X, u, z
-    # the finalize runs as two launches (both read M): the FP64 part and the FP32 transport part
+    # the finalize's FP64 part and FP32 transport part (both read M)
     "adj_finalize": (9 + 9 + 9 + 9 + 6 + 3 + 9 + 9) * 4 + 9 * 4 + 9 * 8 * 2,  # M, F, dFc, R, S, vol/lam/mu,
                                                                                  # C', dLdF' -> dLdF, FP64 acc
     "adj_finalize_transport": (18 + 9 + 9 + 3 + 1) * 4 + 15 * 4,  # M/X/u/z, G, dLdC', dLdx', m -> dLdx, dLdv, dLdC
@@ -269,10 +269,10 @@ PER_TOUCHED_NODE_BYTES = {"p2g": 16, "g2p_p_op2": 16, "adj_g2p_scatter": 16, "ad
 PER_GRID_NODE_BYTES = {"g_op": 32, "adj_g_op": 64}
 
 # Executed flop per particle-step of the hot kernels (add + mul + 2 fma over the predicated-on
-# thread instructions), counted by ncu on the 64^3, 266,868-particle workload
-# (profiles/flops_atomics_hot_kernels_64cubed_267k.txt); it includes the warp-item layout's redundant
-# weight evaluations.  Nominal vector peaks: 148 SMs x 128 FP32 / 64 FP64 lanes x 2 at 1965 MHz.
-FLOP_PER_PARTICLE_STEP = {"fp32": 11375, "fp64": 1192}
+# thread instructions, packed ones counted twice), counted by ncu on the 64^3, 267k-particle scene
+# (profiles/chunk_kernels_64cubed_267k.txt).  Nominal vector peaks: 148 SMs x 128 FP32 / 64 FP64
+# lanes x 2 at 1965 MHz.
+FLOP_PER_PARTICLE_STEP = {"fp32": 10529, "fp64": 937}
 NOMINAL_VECTOR_TFLOPS = {"fp32": 148 * 128 * 2 * 1.965e-3, "fp64": 148 * 64 * 2 * 1.965e-3}
 
 
@@ -288,6 +288,19 @@ def compute_rates(particle_steps_per_s: float) -> dict:
 def algorithmic_bytes(kernel: str, n: int, touched: int, nodes: int) -> float:
     return (PER_PARTICLE_BYTES.get(kernel, 0) * n + PER_TOUCHED_NODE_BYTES.get(kernel, 0) * touched
             + PER_GRID_NODE_BYTES.get(kernel, 0) * nodes)
+
+
+def launch_bytes(kernel: str, n: int, touched: int) -> float:
+    """The same per launch of the kernels as they run: G2P forms the next step's G, R and S from the
+    F and C it holds, the gather goes on to the finalize with its sums in registers, and the node
+    passes walk the box around the cloud (its touched nodes are a lower bound): the grid update also
+    clears the next layer's node, the adjoint one the node it has read."""
+    particle = {"g2p_p_op2": PER_PARTICLE_BYTES["g2p_p_op2"] + (9 + 4 + 24) * 4,
+                "adj_p2g_gather": (6 + 1 + 3 + 12 + 9 + 1) * 4 + (9 + 9 + 9 + 6 + 3 + 9 + 9 + 3) * 4 + 24 * 4 + 9 * 8 * 2}
+    node = {"g_op": 48, "adj_g_op": 80}
+    if kernel in node:
+        return node[kernel] * touched
+    return particle.get(kernel, PER_PARTICLE_BYTES.get(kernel, 0)) * n + PER_TOUCHED_NODE_BYTES.get(kernel, 0) * touched
 
 
 def committed_traffic(kernel: str):
@@ -385,7 +398,7 @@ def workload_config(sc, dt_sub, ckpt):
             "particles": sc.n, "grid": list(sc.dims), "layers": sc.steps + 1, "dt": sc.dt,
             "dt_substituted_from": dt_sub, "checkpoint_every": ckpt, "loss": "reference log-mass + min-mass penalty",
             "l2_policy": "inputs larger than L2 (per-rollout layer state > 5 GB, 126 MB L2)",
-            "g2p_kernel": "warp items" if BRICK_CELLS == 0 else "bricks of %d^3 cells" % (BRICK_CELLS or 2),
+            "g2p_kernel": "one thread per particle in cell order",
             "particle_order": "seeded random permutation" if SHUFFLE else "lattice",
             "reorder_particles": REORDER,
             "parallelism": "replicas: one independent instance per GPU"}
@@ -547,14 +560,14 @@ def run_ours(args):
     top = max(kern, key=lambda k: kern[k]["total_ms"]) if kern else None
     roof = None
     if top:
-        alg = algorithmic_bytes(top, sc.n, touched, nodes)
+        alg = launch_bytes(top, sc.n, touched)
         achieved = alg / (kern[top]["avg_us"] * 1e-6) / 1e9
         roof = {"kernel": top, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": committed_traffic(top), "algorithmic_bytes_per_launch": alg,
                 "avg_launch_us": kern[top]["avg_us"]}
         for k in kern:
-            b = algorithmic_bytes(k, sc.n, touched, nodes)
+            b = launch_bytes(k, sc.n, touched)
             if b:
                 kern[k]["hbm_frac"] = b / (kern[k]["avg_us"] * 1e-6) / 1e9 / peak
 

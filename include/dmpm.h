@@ -67,7 +67,7 @@ typedef struct dmpm_ctx dmpm_ctx;
 
 /* precision paths */
 #define DMPM_FP64 0       /* plain FP64 path: one kernel per reference stage, global atomics */
-#define DMPM_FP32_MIXED 1 /* FP32 state and grid, cell-sorted warp items; FP64 polar/SVD, stress
+#define DMPM_FP32_MIXED 1 /* FP32 state and grid, cell-sorted chunks; FP64 polar/SVD, stress
                              derivative, loss and control-gradient sums */
 
 /* adjoint modes */
@@ -138,9 +138,9 @@ typedef struct {
     int eager;               /* FP32 path with every layer kept: 0 = capture dmpm_forward / dmpm_backward
                                 once per start (top, control) layer and replay them as CUDA graphs;
                                 1 = launch kernel by kernel (per-kernel profiling also does) */
-    int brick_cells;         /* FP32 path, G2P: 2 (default) or 4 = a CTA stages the node tile of a brick
-                                of brick_cells^3 cells in shared memory and each thread handles one
-                                particle of it; 0 = warp items (8 particles of a cell per warp).
+    int brick_cells;         /* deterministic mode, P2G and the adjoint scatter: 2 (default) or 4 = a CTA
+                                adds up a brick of brick_cells^3 cells in a node tile in shared memory;
+                                0 = every sum straight to global memory.  The bits are the same.
                                 Takes effect at the next cell sort. */
     int deterministic;       /* FP32 path: 1 = node sums (P2G, the adjoint scatter, the mass rasters) as
                                 64-bit integer multiples of a power of two fixed per pass, added with
@@ -287,13 +287,12 @@ int dmpm_compute_volumes_noalloc(int n, const float* x, const float* m, int dim_
                                  const float* min_point, float* vol, void* stream);
 
 /* Per-kernel device time.  With profiling on, every hot-path launch is
- * bracketed by CUDA events on the context's stream (the adjoint finalize's two
- * parts, which otherwise run side by side on two streams, then run one after
- * the other); dmpm_kernel_stats returns the summed milliseconds and the launch
- * count of one kernel since profiling was (re)enabled.  Kernel ids run from 0
- * to DMPM_NUM_KERNEL_IDS - 1; dmpm_kernel_name gives their names (p2g,
- * g2p_p_op2, adj_p2g_gather, adj_finalize, adj_finalize_transport, ...) and
- * NULL for any other id. */
+ * bracketed by CUDA events on the context's stream; dmpm_kernel_stats returns
+ * the summed milliseconds and the launch count of one kernel since profiling was
+ * (re)enabled.  Kernel ids run from 0 to DMPM_NUM_KERNEL_IDS - 1;
+ * dmpm_kernel_name gives their names (p2g, g2p_p_op2, adj_p2g_gather, ...) and
+ * NULL for any other id.  adj_finalize and adj_finalize_transport count nothing:
+ * the adjoint finalize is part of adj_p2g_gather. */
 #define DMPM_NUM_KERNEL_IDS 12
 int dmpm_set_profiling(dmpm_ctx* ctx, int on);
 int dmpm_kernel_stats(dmpm_ctx* ctx, int kernel_id, double* total_ms, int64_t* launches);
@@ -322,8 +321,8 @@ typedef struct {
 } dmpm_instance;
 typedef struct {
     int sort_every;     /* re-sort particles by cell every this many steps; 0 = 8 */
-    int ctas_per_sm;    /* persistent grid of the warp-item kernels, CTAs per SM (1..8); 0 = 3 */
-    int particle_block; /* threads per block of the per-particle kernels: 128 or 256; 0 = 256 */
+    int ctas_per_sm;    /* 0 to 8; kept for callers that set it: no kernel has a persistent grid */
+    int particle_block; /* threads per block of the first step's stress kernel: 128 or 256; 0 = 256 */
     int use_graph;      /* 1 = capture the gradient evaluation once, replay it as a CUDA graph */
 } dmpm_batch_launch;
 int dmpm_batch_create(int device, int count, const dmpm_instance* instances, dmpm_batch** out);
