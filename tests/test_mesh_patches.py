@@ -1,5 +1,5 @@
-"""The mesh sampler's patches: triangles are cut into patches of 64 that far
-points see as their boundary's fan, so meshes just below and above one patch,
+"""The mesh sampler's tree of patches: triangles are cut into leaves of 40, far
+points see a patch as its boundary's fan, so meshes of one leaf, of two and more,
 split vertices, an open surface and a second, closed component inside the box are
 where a wrong boundary would show.  The oracle sums every triangle's solid angle
 in FP64; its winding numbers are compared with 1/2 away from rounding (no
@@ -26,6 +26,8 @@ def _torus(nu, nv, R=0.5, r=0.21):
 
 
 def _mesh(kind):
+    if kind == "one_leaf":
+        return _torus(6, 3)
     if kind == "one_patch":
         return _torus(8, 4)
     if kind == "two_patches":
@@ -41,7 +43,7 @@ def _mesh(kind):
     return V, F
 
 
-@pytest.mark.parametrize("kind", ["one_patch", "two_patches", "many", "split_vertices", "open", "two_components"])
+@pytest.mark.parametrize("kind", ["one_leaf", "one_patch", "two_patches", "many", "split_vertices", "open", "two_components"])
 def test_sampler_matches_the_sum_over_all_triangles(gpu_ready, kind):
     V, F = _mesh(kind)
     dx = 0.037
