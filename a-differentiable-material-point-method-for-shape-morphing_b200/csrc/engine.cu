@@ -514,16 +514,28 @@ template <class T> class Engine : public EngineBase {
     // deterministic mode of the FP32 path: order-independent node sums (fixpoint.cuh)
     bool det() const { return kWarp && ctx_->prm.deterministic != 0; }
     void ensure_fix() {
-        if (!det() || (fix_ && fix_G_ == G_)) return;
+        if (!det()) return;
+        if (fix_ && fix_G_ == G_) {
+            if (fix_dirty_) zero_fix();
+            return;
+        }
         fix_arena_.release();
         fix_ = nullptr;
         fixb_ = nullptr;
         fix_ = (fix4*)fix_arena_.alloc(G_ * sizeof(fix4));
         fixb_ = (unsigned*)fix_arena_.alloc(FIXB_SLOTS * sizeof(unsigned));
         fix_G_ = G_;
+        zero_fix();
     }
-    void clear_fix(int slot) {  // zero the integer sums and one bound slot (-1: all) before a pass
+    // The integer sums are zero between passes: reading them back zeroes them.  Only a
+    // pass that failed in between leaves them dirty, for ensure_fix of the next call
+    // (before any capture or replay, which take them as zero).
+    void zero_fix() {
         DMPM_CK(cudaMemsetAsync(fix_, 0, G_ * sizeof(fix4), ctx_->stream));
+        fix_dirty_ = false;
+    }
+    void clear_fix(int slot) {  // zero one bound slot (-1: all) before a pass
+        fix_dirty_ = true;
         if (slot < 0) DMPM_CK(cudaMemsetAsync(fixb_, 0, FIXB_SLOTS * sizeof(unsigned), ctx_->stream));
         else DMPM_CK(cudaMemsetAsync(fixb_ + slot, 0, sizeof(unsigned), ctx_->stream));
     }
@@ -672,6 +684,7 @@ template <class T> class Engine : public EngineBase {
                 launched();
                 k_fix_to_node4<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, a.n, G_, 2, a.grid);
                 launched();
+                fix_dirty_ = false;
                 return;
             }
         }
@@ -1221,18 +1234,19 @@ template <class T> class Engine : public EngineBase {
             else if (gen) k_p2g_c<false, true><<<chunk_blocks(n_, a.chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a);
             else k_p2g_c<false, false><<<chunk_blocks(n_, a.chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a);
             launched();
-            if (dm) {
-                k_fix_to_node4<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, 0, (node4<float>*)g);
-                launched();
-            }
             pend();
             pbeg(K_GOP);
             const bool clear_next = g_next && !dm;
-            k_box_gop<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, dm ? box_full_ : a.box, dm ? box_of(g) : nullptr,
-                                                              clear_next ? (node4<float>*)g_next : nullptr,
-                                                              clear_next ? box_of(g_next) : nullptr, geo_, a.dt, a.fext[0],
-                                                              a.fext[1], a.fext[2]);
+            if (dm)
+                k_fix_gop<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, (node4<float>*)g, box_full_, box_of(g), a.dt,
+                                                             a.fext[0], a.fext[1], a.fext[2]);
+            else
+                k_box_gop<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, a.box,
+                                                                  clear_next ? (node4<float>*)g_next : nullptr,
+                                                                  clear_next ? box_of(g_next) : nullptr, geo_, a.dt,
+                                                                  a.fext[0], a.fext[1], a.fext[2]);
             launched();
+            if (dm) fix_dirty_ = false;
             pend();
             // the deterministic mode keeps the standalone stress stage: it also raises the
             // next P2G's bounds, which that step clears first
@@ -1483,8 +1497,6 @@ template <class T> class Engine : public EngineBase {
                 launched();
                 if (P.warp_general) launch_adj_scatter_fix<true>(a, ush, ws);
                 else launch_adj_scatter_fix<false>(a, ush, ws);
-                launched();
-                k_fix_to_node4<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, 1, (node4<float>*)gadj_);
             } else {
                 const unsigned cb = chunk_blocks(n_, a.chunk), ct = DMPM_CHUNK_THREADS;
                 if (P.warp_general) {
@@ -1498,13 +1510,21 @@ template <class T> class Engine : public EngineBase {
             launched();
             pend();
             pbeg(K_ADJ_GOP);
+            const bool fix_fused = dm && !P.keep_intermediates;
+            if (dm && !fix_fused) {
+                k_fix_to_node4<<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, 1, (node4<float>*)gadj_);
+                launched();
+            }
             if (P.keep_intermediates)
                 DMPM_CK(cudaMemcpyAsync(layers_[i].dbggdv, gadj_, G_ * sizeof(node4<T>), cudaMemcpyDeviceToDevice, ctx_->stream));
             // kept intermediates show every node of the grid
             const int* box = P.keep_intermediates ? box_full_ : box_of(grid_of(i));
-            if (ex) k_box_adj_gop<true><<<box_blocks(), 256, 0, ctx_->stream>>>(a.grid, a.gadj, a.gadj2, box, geo_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
+            if (fix_fused && ex) k_fix_adj_gop<true><<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, a.grid, a.gadj2, a.dt, a.fext[0], a.fext[1], a.fext[2]);
+            else if (fix_fused) k_fix_adj_gop<false><<<ggrid(), 256, 0, ctx_->stream>>>(fix_, fixb_, n_, G_, a.grid, a.gadj2, a.dt, a.fext[0], a.fext[1], a.fext[2]);
+            else if (ex) k_box_adj_gop<true><<<box_blocks(), 256, 0, ctx_->stream>>>(a.grid, a.gadj, a.gadj2, box, geo_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
             else k_box_adj_gop<false><<<box_blocks(), 256, 0, ctx_->stream>>>(a.grid, a.gadj, a.gadj2, box, geo_, a.dt, a.fext[0], a.fext[1], a.fext[2]);
             launched();
+            if (dm) fix_dirty_ = false;
             pend();
             if (P.keep_intermediates)
                 DMPM_CK(cudaMemcpy2DAsync(layers_[i].dbggdp, sizeof(node4<T>), gadj2_, 2 * sizeof(node4<T>),
@@ -1965,6 +1985,7 @@ template <class T> class Engine : public EngineBase {
     size_t part_n_ = 0;
     // deterministic mode: integer node sums (G fix4) and their bound slots
     fix4* fix_ = nullptr;
+    bool fix_dirty_ = true;  // the sums are not known to be zero
     unsigned* fixb_ = nullptr;
     size_t fix_G_ = 0;
     void* host_misc_ = nullptr;

@@ -91,15 +91,14 @@ __device__ __forceinline__ FixScale fix_scale(const unsigned* slot, long long n)
     return FixScale{fix_pow2(k), fix_pow2(-k)};
 }
 
-// Node records from the integer sums: which = 0: (p.xyz, m) with the momentum
-// and mass scales; 1: (dLdv.xyz, 0) with the adjoint scale; 2: (0, 0, 0, m)
-// with the raster scale.
-static __global__ void k_fix_to_node4(const fix4* __restrict__ acc, const unsigned* __restrict__ slots, long long n,
-                                      size_t G, int which, node4<float>* out) {
-    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    const fix4 q = acc[g];
+// A node record from the integer sums, which are zeroed behind it for the next
+// pass: which = 0: (p.xyz, m) with the momentum and mass scales; 1: (dLdv.xyz, 0)
+// with the adjoint scale; 2: (0, 0, 0, m) with the raster scale.
+__device__ __forceinline__ node4<float> fix_take(fix4* acc, const unsigned* slots, long long n, int which) {
+    const fix4 q = *acc;
     node4<float> r{0.f, 0.f, 0.f, 0.f};
+    if ((q.x | q.y | q.z | q.w) == 0) return r;
+    *acc = fix4{0, 0, 0, 0};
     if (which == 0) {
         const FixScale sp = fix_scale(slots + FIXB_MOMENTUM, n), sm = fix_scale(slots + FIXB_MASS, n);
         r = node4<float>{fix_value(q.x, sp.inv), fix_value(q.y, sp.inv), fix_value(q.z, sp.inv), fix_value(q.w, sm.inv)};
@@ -110,7 +109,13 @@ static __global__ void k_fix_to_node4(const fix4* __restrict__ acc, const unsign
         const FixScale sr = fix_scale(slots + FIXB_RASTER, n);
         r.w = fix_value(q.w, sr.inv);
     }
-    out[g] = r;
+    return r;
+}
+static __global__ void k_fix_to_node4(fix4* acc, const unsigned* __restrict__ slots, long long n, size_t G, int which,
+                                      node4<float>* out) {
+    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= G) return;
+    out[g] = fix_take(acc + g, slots, n, which);
 }
 
 // the largest particle mass of a cloud, into slot (the raster's bound)

@@ -571,21 +571,35 @@ __device__ __forceinline__ void box_clear(node4<float>* grid, int* box, const in
 static __global__ void __launch_bounds__(256) k_box_clear(node4<float>* grid, int* box, const int* prev, GridGeom g) {
     box_clear(grid, box, prev, g);
 }
-// the grid update over the box; mark: the box to set to it (the deterministic mode
-// fills its grids whole), or null; next: the next layer's grid, cleared as by
+// the grid update over the box; next: the next layer's grid, cleared as by
 // k_box_clear for a launch less per step (8.7k particles: 39.9 -> 38.7 us a step
 // forward and back), or null
 static __global__ void __launch_bounds__(256)
-    k_box_gop(node4<float>* grid, const int* box, int* mark, node4<float>* next, int* next_box, GridGeom g, float dt,
-              float f0, float f1, float f2) {
+    k_box_gop(node4<float>* grid, const int* box, node4<float>* next, int* next_box, GridGeom g, float dt, float f0,
+              float f1, float f2) {
     const NodeRange r(box);
     if (next) box_clear(next, next_box, box, g);
     const float f[3] = {f0, f1, f2};
-    if (mark && blockIdx.x == 0 && threadIdx.x < 6) mark[threadIdx.x] = box[threadIdx.x];
     for (int row = first_warp(); row < r.rows(); row += warp_count()) {
         node4<float>* p = grid + r.first(row, g);
         for (int k = threadIdx.x & 31; k < r.n[2]; k += 32) gop_node(p + k, dt, f);
     }
+}
+
+// The deterministic mode's: integer sums to (p, m) to (v, m) over the whole grid,
+// whose box becomes the layer's.  Bound by the 32 + 16 bytes per node.  As a memset
+// of the sums, a conversion and a grid update 34 us per step forward and back
+// on a 64 x 60 x 53 grid; this and k_fix_adj_gop, 17.
+static __global__ void __launch_bounds__(256)
+    k_fix_gop(fix4* acc, const unsigned* __restrict__ slots, long long n, size_t G, node4<float>* grid,
+              const int* __restrict__ whole, int* box, float dt, float f0, float f1, float f2) {
+    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < 6) box[g] = whole[g];
+    if (g >= G) return;
+    const float f[3] = {f0, f1, f2};
+    node4<float> nd = fix_take(acc + g, slots, n, 0);
+    gop_node(&nd, dt, f);
+    grid[g] = nd;
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -751,6 +765,17 @@ __global__ void __launch_bounds__(256)
             gadj[n0 + k] = node4<float>{0.f, 0.f, 0.f, 0.f};
         }
     }
+}
+
+// the deterministic mode's, from the integer sums of dLdv over the whole grid
+template <bool EXACT>
+__global__ void __launch_bounds__(256)
+    k_fix_adj_gop(fix4* acc, const unsigned* __restrict__ slots, long long n, size_t G, const node4<float>* __restrict__ grid,
+                  node4<float>* gadj2, float dt, float f0, float f1, float f2) {
+    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= G) return;
+    const float f[3] = {f0, f1, f2};
+    adj_gop_node<EXACT>(grid[g], fix_take(acc + g, slots, n, 1), gadj2 + 2 * g, dt, f);
 }
 
 // ------------------------------------------------------------------ finalize
