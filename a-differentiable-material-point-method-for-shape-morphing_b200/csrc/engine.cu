@@ -1206,8 +1206,7 @@ template <class T> class Engine : public EngineBase {
             } else {
                 a.box = box_of(g);
                 if (!done.cleared) {
-                    k_box_clear<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, a.box,
-                                                                        a.box > boxes_ ? a.box - 6 : nullptr, geo_);
+                    k_box_clear<<<box_blocks(), 256, 0, ctx_->stream>>>((node4<float>*)g, a.box, geo_);
                     launched();
                 }
             }
@@ -1257,6 +1256,7 @@ template <class T> class Engine : public EngineBase {
                 a.P_next = ctx_->prm.keep_intermediates ? (float*)layers_[l + 1].dbgP : nullptr;
                 a.n_next = n_;
             }
+            if (clear_next) a.box_next = box_of(g_next);
             pbeg(K_G2P);
             launch_g2p<false>(a, ctx_->stream);
             launched();

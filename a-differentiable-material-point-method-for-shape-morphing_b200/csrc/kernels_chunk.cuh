@@ -462,6 +462,7 @@ __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, STRESS ? DMPM_CHUNK_G2P_MI
     __shared__ float s_dump[DMPM_CHUNK_THREADS];
     const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) / SPLIT);
     if ((q & ~(32 / SPLIT - 1)) >= a.n) return;  // the whole warp
+    if (!BATCH && blockIdx.x == 0 && a.box_next) box_join(a.box_next, a.box);
     const size_t np = a.np, npl = a.npl, npn = a.npn;
     const int p = (int)a.items.order[min(q, a.n - 1)];
     const int inst = BATCH ? (int)a.pinst[p] : 0;

@@ -308,7 +308,8 @@ struct WArgs {
     const float* dfc;      // dFc of layer n
     float* G;              // [24][npl] per layer: G (9), polar R (9), polar S (6: s00 s01 s02 s11 s12 s22)
     node4<float>* grid;    // layer n grid: (p, m) after P2G, (v, m) after the grid update
-    int* box;              // node box that P2G widens to the stencils it adds to (NodeBox), or null
+    int* box;              // node box that P2G widens to the stencils it adds to (NodeRange), or null
+    int* box_next;         // G2P: the next layer's box, which takes in this one's, or null
     float* P;              // debug: stress of layer n (or null)
     unsigned* status;
     // adjoint
@@ -511,8 +512,9 @@ static __global__ void k_gop_inplace(node4<float>* grid, size_t G, float dt, flo
 // node passes of the layer -- clearing its grid before P2G, the grid update, the
 // adjoint grid update -- walk the box instead of the grid.  P2G widens the box to
 // the stencils it adds to; boxes only grow (until a new cloud is set up), and a
-// layer's takes in the layer's before it first, so that P2G finds it wide enough
-// nearly always and few warps reach the atomics (starting empty at every step,
+// layer's takes in the layer's before it first (in G2P, once the grid is cleared),
+// so that P2G finds it wide enough nearly always and few warps reach the atomics
+// (starting empty at every step,
 // P2G took 55 instead of 29 us per step on the 64^3, 267k-particle scene).
 // One warp walks a row of the box along the last axis.
 struct NodeRange {
@@ -555,30 +557,32 @@ __device__ __forceinline__ void widen_box(int* box, int have, const GridGeom& g,
     if (lane < 3 && lo < have) atomicMin(box + lane, lo);
     if (lane >= 3 && lane < 6 && hi > have) atomicMax(box + lane, hi);
 }
-// zero the nodes of the layer's box, then take in the box `prev` (or null).  A block
-// may read the box while it grows: it then clears more, which is zero already.
-__device__ __forceinline__ void box_clear(node4<float>* grid, int* box, const int* prev, const GridGeom& g) {
+// zero the nodes of the layer's box.  Nothing may write the box meanwhile: the rows
+// are numbered by it, and a warp that saw another box would leave rows to nobody.
+__device__ __forceinline__ void box_clear(node4<float>* grid, const int* box, const GridGeom& g) {
     const NodeRange r(box);
     for (int row = first_warp(); row < r.rows(); row += warp_count()) {
         node4<float>* p = grid + r.first(row, g);
         for (int k = threadIdx.x & 31; k < r.n[2]; k += 32) p[k] = node4<float>{0.f, 0.f, 0.f, 0.f};
     }
-    if (prev && blockIdx.x == 0 && threadIdx.x < 6) {
-        const int a = box[threadIdx.x], b = prev[threadIdx.x];
-        box[threadIdx.x] = threadIdx.x < 3 ? min(a, b) : max(a, b);
-    }
 }
-static __global__ void __launch_bounds__(256) k_box_clear(node4<float>* grid, int* box, const int* prev, GridGeom g) {
-    box_clear(grid, box, prev, g);
+static __global__ void __launch_bounds__(256) k_box_clear(node4<float>* grid, const int* __restrict__ box, GridGeom g) {
+    box_clear(grid, box, g);
+}
+// lanes 0..5 of one warp of G2P, between the clearing of the next layer's grid and
+// its P2G: the next layer's box takes in this one's
+__device__ __forceinline__ void box_join(int* next, const int* box) {
+    const int c = threadIdx.x;
+    if (c < 6) next[c] = c < 3 ? min(next[c], box[c]) : max(next[c], box[c]);
 }
 // the grid update over the box; next: the next layer's grid, cleared as by
 // k_box_clear for a launch less per step (8.7k particles: 39.9 -> 38.7 us a step
 // forward and back), or null
 static __global__ void __launch_bounds__(256)
-    k_box_gop(node4<float>* grid, const int* box, node4<float>* next, int* next_box, GridGeom g, float dt, float f0,
-              float f1, float f2) {
+    k_box_gop(node4<float>* grid, const int* __restrict__ box, node4<float>* next, const int* __restrict__ next_box,
+              GridGeom g, float dt, float f0, float f1, float f2) {
     const NodeRange r(box);
-    if (next) box_clear(next, next_box, box, g);
+    if (next) box_clear(next, next_box, g);
     const float f[3] = {f0, f1, f2};
     for (int row = first_warp(); row < r.rows(); row += warp_count()) {
         node4<float>* p = grid + r.first(row, g);
