@@ -1366,7 +1366,7 @@ template <class T> class Engine : public EngineBase {
                     for (int l = start; l + 1 < L_; l++) {
                         Epoch& e = epochs_[std::min((int)epochs_.size() - 1, l / sort_every())];
                         e.valid = true;
-                        e.grouped = det() || !count_;
+                        e.grouped = det();  // only that mode's sorts form the items
                     }
             } else {
                 body();
