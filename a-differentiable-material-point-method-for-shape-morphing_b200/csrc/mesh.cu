@@ -15,14 +15,14 @@
 //   The half angles are summed as the product of the complex numbers den + i det,
 // with a count of the times it passes the negative real axis: one atan2 per point
 // in place of one per triangle, whose FP64 instructions were the kernel's cost.
-//   The triangles are cut into a tree of patches.  A surface's solid angle from a
-// point is that of any surface with the same boundary that the point is not
-// between, so a warp with a point in a patch's bounding box goes on to its two
-// halves (a leaf is summed triangle by triangle), and any other takes the fan over
-// the patch's boundary edges from one of its vertices, which lies in the box too
-// (Jacobson, Kavan and Sorkine-Hornung 2013).  A fan has about 4 sqrt(triangles)
-// triangles, each with one new vertex.  2.7M points inside 4.4M candidates and
-// 1,152 triangles, kernel ms: 29.8 triangle by triangle with an atan2 each, 9.3
+//   For all but few points the triangles are cut into a tree of patches.  A
+// surface's solid angle from a point is that of any surface with the same boundary
+// that the point is not between, so a warp with a point in a patch's bounding box
+// goes on to its two halves (a leaf is summed triangle by triangle), and any other
+// takes the fan over the patch's boundary edges from one of its vertices, which lies
+// in the box too (Jacobson, Kavan and Sorkine-Hornung 2013).  A fan has about
+// 4 sqrt(triangles) triangles, each with one new vertex.  2.7M points inside 4.4M
+// candidates and 1,152 triangles, kernel ms: 29.8 triangle by triangle with an atan2 each, 9.3
 // with one level of patches of up to 64, 3.33 with the tree.
 //   The kept points are compacted on the GPU in lattice order.  The lattice
 // coordinates are formed in float with the reference's two roundings.
@@ -54,6 +54,12 @@ namespace {
 // triangles of a leaf patch, at most.  Wall ms at 1,152 / 144 / 24,000 triangles: 16: 8.7 /
 // 2.3 / 27.1; 24: 7.8 / 2.5 / 24.5; 40: 7.9 / 2.9 / 24.1; 72: 9.2 / 3.0 / 21.8.
 constexpr int kPatchTriangles = 40;
+// Candidate points from which the tree is built: it costs the host about 1.1 us a
+// triangle, the plain sum the GPU that much per triangle for this many points, so the
+// line hardly depends on the mesh.  Wall ms of a call, plain / tree, at 30k, 100k and
+// 200k candidates: 1,152 triangles 0.76 / 1.04, 1.10 / 1.15, 2.0 / 1.24; 25,600: 14.4 /
+// 22.3, 22.5 / 22.8, 41.8 / 23.2; 250,000: 140 / 278, 223 / 278, 413 / 280.
+constexpr long long kTreeCandidates = 100000;
 
 // the lattice point min_point + sampling_dx * (i, j, k): a product and a sum, each rounded to float
 struct LatticePoints {
@@ -231,6 +237,14 @@ struct Mesh {
     std::vector<float> tri, edges;
     std::vector<Patch> patches;
 };
+// all triangles as one leaf
+void one_patch(const std::vector<float>& tri, int nf, Mesh& m) {
+    m.tri = tri;
+    Patch P{};
+    P.t1 = nf;
+    P.skip = 1;
+    m.patches.push_back(P);
+}
 class PatchTree {
    public:
     PatchTree(const std::vector<float>& tri, int nf, Mesh& m) : tri_(tri), m_(m), order_((size_t)nf), vid_((size_t)nf * 3) {
@@ -360,7 +374,8 @@ int inside_points(const std::vector<float>& tri, int nf, const Points& pts, cons
     using namespace dmpm;
     const long long total = (long long)dims[0] * dims[1] * dims[2];
     Mesh m;
-    PatchTree(tri, nf, m);
+    if (total < kTreeCandidates) one_patch(tri, nf, m);
+    else PatchTree(tri, nf, m);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     const int tiles = (int)((blocks + SCAN_TILE - 1) / SCAN_TILE);
     dmpm_host::Scratch mem;
