@@ -40,7 +40,9 @@
 #include <cstdint>
 #include <cstring>
 #include <map>
+#include <new>
 #include <numeric>
+#include <stdexcept>
 #include <unordered_map>
 #include <utility>
 #include <vector>
@@ -361,6 +363,17 @@ class PatchTree {
     std::vector<const float*> at_;  // a vertex's position
 };
 
+// no C++ exception leaves a C entry: host memory that is not to be had is an error code
+template <class Fn> int guarded(Fn f) {
+    try {
+        return f();
+    } catch (const std::bad_alloc&) {
+        return DMPM_ERR_OOM;
+    } catch (const std::length_error&) {
+        return DMPM_ERR_OOM;
+    }
+}
+
 int cuda_failed() {
     cudaGetLastError();
     return DMPM_ERR_CUDA;
@@ -433,10 +446,12 @@ extern "C" int dmpm_mesh_lattice_points(const float* V, int nv, const int* F, in
     if (st != DMPM_OK) return st;
     const long long total = (long long)dims[0] * dims[1] * dims[2];
     if (total > (1ll << 31)) return DMPM_ERR_TOO_LARGE;
-    std::vector<float> tri;
-    if ((st = gather_triangles(V, nv, F, nf, tri)) != DMPM_OK) return st;
-    LatticePoints pts{{min_point[0], min_point[1], min_point[2]}, sampling_dx};
-    return inside_points(tri, nf, pts, dims, out, capacity, count);
+    const LatticePoints pts{{min_point[0], min_point[1], min_point[2]}, sampling_dx};
+    return guarded([&] {
+        std::vector<float> tri;
+        const int bad = gather_triangles(V, nv, F, nf, tri);
+        return bad != DMPM_OK ? bad : inside_points(tri, nf, pts, dims, out, capacity, count);
+    });
 }
 
 extern "C" int dmpm_mesh_jittered_points(const float* V, int nv, const int* F, int nf, const float* min_point,
@@ -453,10 +468,11 @@ extern "C" int dmpm_mesh_jittered_points(const float* V, int nv, const int* F, i
     }
     const long long total = (long long)dims[0] * dims[1] * dims[2];
     if (total > (1ll << 31)) return DMPM_ERR_TOO_LARGE;
-    std::vector<float> tri;
-    int st = gather_triangles(V, nv, F, nf, tri);
-    if (st != DMPM_OK) return st;
     const float sdx = cell_dx / (float)per_axis;
-    JitteredPoints pts{{min_point[0], min_point[1], min_point[2]}, sdx, dims[1], dims[2], seed};
-    return inside_points(tri, nf, pts, dims, out, capacity, count);
+    const JitteredPoints pts{{min_point[0], min_point[1], min_point[2]}, sdx, dims[1], dims[2], seed};
+    return guarded([&] {
+        std::vector<float> tri;
+        const int bad = gather_triangles(V, nv, F, nf, tri);
+        return bad != DMPM_OK ? bad : inside_points(tri, nf, pts, dims, out, capacity, count);
+    });
 }

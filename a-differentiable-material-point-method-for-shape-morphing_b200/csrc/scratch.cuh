@@ -9,7 +9,8 @@
 // (scratch_trim).  Pools are found by the context's unique id, so a context that
 // was reset never meets an old one's pool; where no pool can be had the
 // allocations are plain ones.  The driver's pools are safe to use from several
-// threads, and all calls order their use on the same stream.
+// threads, and all calls order their use on the same stream.  Nothing here throws:
+// C entries use it bare.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -17,6 +18,7 @@
 #include <cstddef>
 #include <map>
 #include <mutex>
+#include <new>
 #include <vector>
 
 namespace dmpm_host {
@@ -55,8 +57,13 @@ inline cudaMemPool_t scratch_pool() {
     if (id == 0) return nullptr;
     ScratchPools& p = scratch_pools();
     std::lock_guard<std::mutex> lock(p.m);
-    const auto it = p.by_context.find(id);
+    auto it = p.by_context.find(id);
     if (it != p.by_context.end()) return it->second;
+    try {
+        it = p.by_context.emplace(id, nullptr).first;
+    } catch (const std::bad_alloc&) {
+        return nullptr;
+    }
     cudaMemPool_t pool = nullptr;
     int dev = 0;
     cudaMemPoolProps props{};
@@ -71,7 +78,7 @@ inline cudaMemPool_t scratch_pool() {
             pool = nullptr;
         }
     }
-    p.by_context[id] = pool;
+    it->second = pool;
     return pool;
 }
 // give back what the current context's pool keeps
@@ -102,17 +109,23 @@ class Scratch {
     template <class T> T* alloc(size_t count) {
         const size_t bytes = count * sizeof(T) + 32;
         void* p = nullptr;
+        try {
+            blocks_.push_back({nullptr, false});
+        } catch (const std::bad_alloc&) {
+            return nullptr;
+        }
         if (pool_ && cudaMallocFromPoolAsync(&p, bytes, pool_, nullptr) == cudaSuccess) {
-            blocks_.push_back({p, true});
+            blocks_.back() = {p, true};
             return (T*)p;
         }
         cudaGetLastError();
         scratch_trim();
         if (cudaMalloc(&p, bytes) != cudaSuccess) {
             cudaGetLastError();
+            blocks_.pop_back();
             return nullptr;
         }
-        blocks_.push_back({p, false});
+        blocks_.back() = {p, false};
         return (T*)p;
     }
 
