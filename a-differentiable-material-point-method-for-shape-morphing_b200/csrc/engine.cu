@@ -930,6 +930,7 @@ template <class T> class Engine : public EngineBase {
         if (k_ == 1) DMPM_CK(cudaMemsetAsync(layers_[0].grid, 0, (size_t)L_ * G_ * sizeof(node4<T>), ctx_->stream));
         else for (node4<T>* g : seg_grid_) DMPM_CK(cudaMemsetAsync(g, 0, G_ * sizeof(node4<T>), ctx_->stream));
         boxes_fresh_ = true;
+        boxes_wide_ = false;
     }
     int* box_of(const node4<T>* g) const {
         if (k_ == 1) return boxes_ + 6 * ((g - layers_[0].grid) / (ptrdiff_t)G_);
@@ -1245,7 +1246,10 @@ template <class T> class Engine : public EngineBase {
                                                                   clear_next ? box_of(g_next) : nullptr, geo_, a.dt,
                                                                   a.fext[0], a.fext[1], a.fext[2]);
             launched();
-            if (dm) fix_dirty_ = false;
+            if (dm) {
+                fix_dirty_ = false;
+                boxes_wide_ = true;
+            }
             pend();
             // the deterministic mode keeps the standalone stress stage: it also raises the
             // next P2G's bounds, which that step clears first
@@ -1353,6 +1357,10 @@ template <class T> class Engine : public EngineBase {
         reset_status();
         ensure_fix();  // before any capture: a captured launch holds the buffers' addresses
         ensure_groups();
+        // A float pass over every layer (or over segment grids, which hold nothing between
+        // passes) starts with tight boxes again after deterministic ones.
+        if (det()) boxes_wide_ = true;
+        else if (kWarp && boxes_wide_ && (start == 0 || k_ > 1)) reset_boxes();
         if (k_ == 1) {
             auto body = [&]() {
                 StepDone done;
@@ -1700,10 +1708,14 @@ template <class T> class Engine : public EngineBase {
                 if (!layers_[l].st) throw StateError{"layer state is not stored (checkpointing)"};
                 if (field == DMPM_F_X) {
                     upload_x(in, layers_[l].st);
-                    // the stencils no longer are those that the layer's node box holds
-                    if (kWarp && k_ == 1)
-                        DMPM_CK(cudaMemcpyAsync(box_of(layers_[l].grid), box_full_, 6 * sizeof(int),
-                                                cudaMemcpyDeviceToDevice, ctx_->stream));
+                    if constexpr (kWarp) {
+                        // an adjoint step may follow without a P2G that widens the box to the new stencils
+                        if (k_ == 1) {
+                            k_box_points<<<(unsigned)((n_ + 255) / 256), 256, 0, ctx_->stream>>>(
+                                (const float*)layers_[l].st, np_, n_, geo_, box_of(layers_[l].grid));
+                            launched();
+                        }
+                    }
                     break;
                 }
                 const int off = field == DMPM_F_V ? PV : field == DMPM_F_F ? PF : PC;
@@ -2003,6 +2015,7 @@ template <class T> class Engine : public EngineBase {
     node4<T>* gadj2_ = nullptr;
     int *boxes_ = nullptr, *box_full_ = nullptr;  // FP32 path: node boxes
     bool boxes_fresh_ = false;                    // the boxes began empty with this cloud
+    bool boxes_wide_ = false;                     // a deterministic pass has set boxes to the whole grid since
     T* gridv_ = nullptr;
     T* pscratch_ = nullptr;
     // FP32 path

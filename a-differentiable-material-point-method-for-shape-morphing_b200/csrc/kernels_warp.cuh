@@ -557,6 +557,14 @@ __device__ __forceinline__ void widen_box(int* box, int have, const GridGeom& g,
     if (lane < 3 && lo < have) atomicMin(box + lane, lo);
     if (lane >= 3 && lane < 6 && hi > have) atomicMax(box + lane, hi);
 }
+// the same for the positions of a layer state
+static __global__ void __launch_bounds__(256) k_box_points(const float* st, size_t np, int n, GridGeom g, int* box) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    float t[3];
+    int base[3];
+    load_x_base(st, np, min(p, n - 1), g, t, base, 1);
+    widen_box(box, (threadIdx.x & 31) < 6 ? *(volatile int*)(box + (threadIdx.x & 31)) : 0, g, base, p < n);
+}
 // zero the nodes of the layer's box.  Nothing may write the box meanwhile: the rows
 // are numbered by it, and a warp that saw another box would leave rows to nobody.
 __device__ __forceinline__ void box_clear(node4<float>* grid, const int* box, const GridGeom& g) {

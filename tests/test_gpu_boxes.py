@@ -93,3 +93,53 @@ def test_second_evaluation_with_wider_motion(gpu_ready, eager):
             c.set_layer(0, f, a)
         assert abs(_gradient(c) - loss) <= 1e-4 * abs(loss)
         _check(c, wide, ref)
+
+
+@pytest.mark.parametrize("checkpoint", [1, 3])
+def test_positions_set_between_passes(gpu_ready, checkpoint):
+    """Positions of a layer set after the forward pass: the adjoint's stencils then lie outside the
+    box that the layer's P2G left.  The next forward pass overwrites them."""
+    sc, target = _sparse(1), _target(2)
+    kw = dict(adjoint="exact", checkpoint_every=checkpoint)
+
+    def run(c):
+        out = []
+        c.setup(L)
+        _gradient(c)
+        x3 = c.get(3, "x")
+        for edit in (np.array([0.0, 0.0, -4.0]), np.array([-6.0, 5.0, 4.5])):
+            c.set_layer(3, "x", x3 + edit)
+            c.loss()
+            c.backward(0)
+            out.append([c.get(0, f) for f in ("dLdx", "dLdv", "dLdF", "dLdC")])
+        _gradient(c)
+        out.append([c.get(0, f) for f in ("dLdx", "dLdv", "dLdF", "dLdC")])
+        return out
+
+    with make_ctx(sc, "fp32", target, deterministic=True, **kw) as ref, make_ctx(sc, "fp32", target, **kw) as c:
+        want, got = run(ref), run(c)
+    for i, (w, g) in enumerate(zip(want, got)):
+        for a, b in zip(w, g):
+            assert normrel(b, a) < 1e-3, i
+
+
+@pytest.mark.parametrize("checkpoint", [1, 2])
+def test_float_passes_after_deterministic_ones_and_a_second_cloud(gpu_ready, checkpoint):
+    """Deterministic passes leave whole grids of nodes, a second cloud of the same size starts elsewhere."""
+    a, b, target = _sparse(1, cells=20), _sparse(4, lo=40.0, cells=20), _target(2)
+    kw = dict(adjoint="exact", checkpoint_every=checkpoint)
+
+    def params(c, sc, deterministic):
+        c.set_params(dt=sc.dt, drag=sc.drag, f_ext=sc.f_ext, smoothing=sc.smoothing, deterministic=deterministic, **kw)
+
+    with make_ctx(a, "fp32", target, **kw) as c:
+        c.setup(L)
+        for sc in (a, b, a):
+            c.set_particles(sc.x, sc.m, sc.lam, sc.mu, v=sc.v, F=sc.F, C=sc.C, dFc=sc.dFc, vol=sc.vol)
+            c.setup(L)
+            ref, loss = _reference(sc, target)
+            with ref:
+                for deterministic in (False, True, False, False):
+                    params(c, sc, deterministic)
+                    assert abs(_gradient(c) - loss) <= 1e-4 * abs(loss)
+                    _check(c, sc, ref)
