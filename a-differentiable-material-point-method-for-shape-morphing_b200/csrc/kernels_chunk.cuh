@@ -347,9 +347,11 @@ __device__ __forceinline__ void load_pair(const node4<float>* p, f32x2 (&f)[4]) 
 }
 // Nodes of a particle's stencil by offset (i, j, k) from its base.  INSIDE: the
 // whole stencil lies in the grid; otherwise nodes outside it read as zero.  A grid
-// has up to 2e9 nodes, so the records of a stencil inside it span less than 2^32; a
-// stencil that reaches over the grid's edge may be longer than the grid, and its
-// rows need 64 bits (gather at 267k particles 99.2 us; 99.8 with 64 bits for all).
+// has up to 2e9 nodes, so a stencil inside it spans less than 2^31 single records and
+// 2^32 of pairs; one that reaches over the grid's edge may be longer than the grid,
+// and its rows need 64 bits.  At 267k particles G2P 49.6 us and the gather 99.0
+// (49.5 and 98.6 in ints throughout; with unsigned offsets in G2P too 50.3, with 64
+// bits for all stencils the gather 99.8).
 template <bool INSIDE, int R> struct StencilNodes {
     const node4<float>* g;  // the base node's first record (dereferenced inside the grid only)
     unsigned si, sj;        // records per slab and row
@@ -359,6 +361,7 @@ template <bool INSIDE, int R> struct StencilNodes {
           si((unsigned)R * (unsigned)(geo.dim[1] * geo.dim[2])), sj((unsigned)R * (unsigned)geo.dim[2]), b0(base[0]),
           b1(base[1]), b2(base[2]), d0(geo.dim[0]), d1(geo.dim[1]), d2(geo.dim[2]) {}
     DMPM_HD const node4<float>* row(int i, int j) const {
+        if (INSIDE && R == 1) return g + (i * (int)si + j * (int)sj);
         return g + (INSIDE ? (size_t)((unsigned)i * si + (unsigned)j * sj) : (size_t)i * si + (size_t)j * sj);
     }
     DMPM_HD bool in(int i, int j, int k) const {
