@@ -290,11 +290,14 @@ def algorithmic_bytes(kernel: str, n: int, touched: int, nodes: int) -> float:
             + PER_GRID_NODE_BYTES.get(kernel, 0) * nodes)
 
 
-def launch_bytes(kernel: str, n: int, touched: int) -> float:
+def launch_bytes(kernel: str, n: int, touched: int, deterministic: bool = False) -> float:
     """The same per launch of the kernels as they run: G2P forms the next step's G, R and S from the
     F and C it holds, the gather goes on to the finalize with its sums in registers, and the node
     passes walk the box around the cloud (its touched nodes are a lower bound): the grid update also
-    clears the next layer's node, the adjoint one the node it has read."""
+    clears the next layer's node, the adjoint one the node it has read.  0: a kernel without a figure,
+    as all of the deterministic mode's are (integer sums over whole grids, more kernels)."""
+    if deterministic:
+        return 0.0
     particle = {"g2p_p_op2": PER_PARTICLE_BYTES["g2p_p_op2"] + (9 + 4 + 24) * 4,
                 "adj_p2g_gather": (6 + 1 + 3 + 12 + 9 + 1) * 4 + (9 + 9 + 9 + 6 + 3 + 9 + 9 + 3) * 4 + 24 * 4 + 9 * 8 * 2}
     node = {"g_op": 48, "adj_g_op": 80}
@@ -314,6 +317,23 @@ def committed_traffic(kernel: str):
     except Exception:
         pass
     return None
+
+
+def roofline(kstats, n: int, touched: int, peak: float, peak_kind: str, deterministic: bool):
+    """Per kernel its times and, where its bytes are known, its share of the bandwidth; and the entry of
+    the dominant kernel (largest total device time)."""
+    kern = {k: {"total_ms": v[0], "launches": v[1], "avg_us": 1000.0 * v[0] / v[1]} for k, v in kstats.items()}
+    if not kern:
+        return kern, None
+    top = max(kern, key=lambda k: kern[k]["total_ms"])
+    rate = {k: launch_bytes(k, n, touched, deterministic) / (kern[k]["avg_us"] * 1e-6) / 1e9 for k in kern}
+    for k in kern:
+        if rate[k]:
+            kern[k]["hbm_frac"] = rate[k] / peak
+    return kern, {"kernel": top, "bound": "hbm", "achieved": rate[top] or None, "peak": peak, "unit": "GB/s",
+                  "frac": rate[top] / peak or None, "peak_source": peak_kind, "traffic": committed_traffic(top),
+                  "algorithmic_bytes_per_launch": launch_bytes(top, n, touched, deterministic) or None,
+                  "avg_launch_us": kern[top]["avg_us"]}
 
 
 # ---------------------------------------------------------------- CPU baseline
@@ -525,7 +545,6 @@ def run_ours(args):
     ms_e2e = max_over_ranks(timed_steps(torch, c, args.steps, e2e_step), world)
     e2e_value = whole_job_value(units_per_step, args.steps, world, ms_e2e)
     touched = int(np.count_nonzero(c.get_grid(0, "grid_m")))
-    nodes = int(np.prod(sc.dims))
     c.close()
 
     # plain FP64 GPU path on the same workload
@@ -554,22 +573,8 @@ def run_ours(args):
                 "grad_relerr_fp64_float32_inputs_vs_float64_inputs":
                     float(np.linalg.norm(grad64 - grad64u) / np.linalg.norm(grad64u))}
 
-    # roofline of the dominant kernel (largest total device time)
     peak, peak_kind = measured_hbm_gbs()
-    kern = {k: {"total_ms": v[0], "launches": v[1], "avg_us": 1000.0 * v[0] / v[1]} for k, v in kstats.items()}
-    top = max(kern, key=lambda k: kern[k]["total_ms"]) if kern else None
-    roof = None
-    if top:
-        alg = launch_bytes(top, sc.n, touched)
-        achieved = alg / (kern[top]["avg_us"] * 1e-6) / 1e9
-        roof = {"kernel": top, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "peak_source": peak_kind,
-                "traffic": committed_traffic(top), "algorithmic_bytes_per_launch": alg,
-                "avg_launch_us": kern[top]["avg_us"]}
-        for k in kern:
-            b = launch_bytes(k, sc.n, touched)
-            if b:
-                kern[k]["hbm_frac"] = b / (kern[k]["avg_us"] * 1e-6) / 1e9 / peak
+    kern, roof = roofline(kstats, sc.n, touched, peak, peak_kind, DETERMINISTIC)
 
     # the target's other clauses, measured in the same run on one GPU: the same
     # workload with checkpoints every 15 layers (recompute in between), and the
