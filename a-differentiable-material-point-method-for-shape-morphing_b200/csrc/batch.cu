@@ -666,23 +666,21 @@ struct dmpm_batch::Impl {
     double autotune(int reps) {
         check_ready();
         if (reps < 1) throw ArgError{"reps must be >= 1"};
+        // the sort interval is the setting that a gradient's time depends on: no kernel has a
+        // grid of ctas_per_sm, and particle_block is that of one launch
         const dmpm_batch_launch base = cfg;
         dmpm_batch_launch best = cfg;
         double best_ms = 1e300;
-        for (int se : {4, 8, 16})
-            for (int cps : {2, 3, 4, 6})
-                for (int pb : {128, 256}) {
-                    dmpm_batch_launch c = base;
-                    c.sort_every = se;
-                    c.ctas_per_sm = cps;
-                    c.particle_block = pb;
-                    set_launch(c);
-                    const double ms = time_config(reps);
-                    if (ms < best_ms) {
-                        best_ms = ms;
-                        best = c;
-                    }
-                }
+        for (int se : {4, 8, 16}) {
+            dmpm_batch_launch c = base;
+            c.sort_every = se;
+            set_launch(c);
+            const double ms = time_config(reps);
+            if (ms < best_ms) {
+                best_ms = ms;
+                best = c;
+            }
+        }
         set_launch(best);
         done = false;
         return best_ms;

@@ -342,9 +342,9 @@ int dmpm_batch_setup(dmpm_batch* b);
 /* One gradient evaluation of every instance; losses: host, count doubles
  * (EndLayerMassLoss of each instance's last layer). */
 int dmpm_batch_gradient(dmpm_batch* b, double* losses);
-/* Time each launch configuration of a small grid (sort interval, CTAs per SM,
- * particle block) over `reps` gradient evaluations, keep the fastest and
- * report its milliseconds per evaluation. */
+/* Time sort intervals of 4, 8 and 16 steps over `reps` gradient evaluations each,
+ * keep the fastest and report its milliseconds per evaluation; the other launch
+ * settings stay as they are. */
 int dmpm_batch_autotune(dmpm_batch* b, int reps, double* best_ms);
 /* dL/d dFc of instance `inst` (tied: summed over its layers), host n * 9 doubles. */
 int dmpm_batch_get_control_grad(dmpm_batch* b, int inst, double* out);
