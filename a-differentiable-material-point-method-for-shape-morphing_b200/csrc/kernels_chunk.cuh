@@ -454,7 +454,7 @@ __device__ __forceinline__ void g2p_sums(const Nodes& f, const float t[3], float
     }
 }
 
-// One thread per particle of the sorted order (four below 40k particles), as the
+// One thread per particle of the sorted order (four of small clouds), as the
 // adjoint gather.  Per step, with the next stress stage (event times; before: a
 // CTA per brick octant that staged its node tile behind two barriers, 2.1 waves of
 // them): 267k particles 49 against 64 us, 301k at 8 per cell 47 against 87, 2.0M
@@ -699,19 +699,23 @@ inline int particle_threads(int n) {
     const int blocks = 148 * 2;
     return n >= 128 * blocks ? 128 : n >= 64 * blocks ? 64 : 32;
 }
-// the same for G2P, with the next stress stage where a.G_next is set
+// Threads per particle of G2P and the gather.  Four shorten the chain of a cloud that
+// leaves SMs idle and repeat the weights of each; from 19k particles they also need a
+// second wave of blocks.  A step forward and back, us with four / with one: 8.7k
+// particles 40.3 / 45.3, 13.1k 45.7 / 48.1, 14.4k 48.3 / 48.2, 16.0k 50.1 / 49.7, 19.4k
+// 61.3 / 50.0, 32.8k 76.2 / 55.7, 39.5k 89.4 / 60.3.
+inline int particle_split(int n) { return n < 14500 ? 4 : 1; }
+// G2P, with the next stress stage where a.G_next is set
 template <bool BATCH> inline void launch_g2p(const WArgs& a, cudaStream_t st) {
-    const int split = a.n < 40000 ? 4 : 1, t = particle_threads(split * a.n);
+    const int split = particle_split(a.n), t = particle_threads(split * a.n);
     const unsigned b = (unsigned)((split * a.n + t - 1) / t);
     if (split == 4 && a.G_next) k_g2p_c<BATCH, true, 4><<<b, t, 0, st>>>(a);
     else if (split == 4) k_g2p_c<BATCH, false, 4><<<b, t, 0, st>>>(a);
     else if (a.G_next) k_g2p_c<BATCH, true, 1><<<b, t, 0, st>>>(a);
     else k_g2p_c<BATCH, false, 1><<<b, t, 0, st>>>(a);
 }
-// Four threads per particle below 40k particles (8.7k: 14.7 against 18-21 us per
-// step), one above (79k: 33 against 57 us)
 template <bool BATCH> inline void launch_gather(const WArgs& a, bool exact, cudaStream_t st) {
-    const int split = a.n < 40000 ? 4 : 1, t = particle_threads(split * a.n);
+    const int split = particle_split(a.n), t = particle_threads(split * a.n);
     const unsigned b = (unsigned)((split * a.n + t - 1) / t);
     if (split == 4 && exact) k_adj_gather_c<true, BATCH, 4><<<b, t, 0, st>>>(a);
     else if (split == 4) k_adj_gather_c<false, BATCH, 4><<<b, t, 0, st>>>(a);
