@@ -1284,7 +1284,7 @@ template <class T> class Engine : public EngineBase {
             launched();
             pend();
             pbeg(K_P2G);
-            const int chunk = scatter_chunk(n_);
+            const int chunk = scatter_chunk64(n_);
             k_p2g_c64<<<chunk_blocks(n_, chunk), DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a, order, chunk);
             launched();
             pend();
@@ -1572,7 +1572,7 @@ template <class T> class Engine : public EngineBase {
         const bool ex = P.adjoint_mode == DMPM_ADJ_EXACT;
         if constexpr (!kWarp) {
             const uint32_t* order = epoch_for(i, state_of(i), false).order;
-            const int chunk = scatter_chunk(n_);
+            const int chunk = scatter_chunk64(n_);
             const unsigned cb = chunk_blocks(n_, chunk);
             pbeg(K_ADJ_SCATTER);
             if (ex) k_adj_scatter_c64<true><<<cb, DMPM_CHUNK_THREADS, 0, ctx_->stream>>>(a, order, chunk);

@@ -265,10 +265,20 @@ __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, DMPM_CHUNK_SCATTER_MINB) k
 // Particles per warp: 32 gives the fewest reductions and record reads per
 // particle, fewer spread a small cloud over the SMs.  P2G / adjoint scatter us
 // at 8, 16, 32 per warp: 8.7k particles 9.9 / 10.1 / 11.7 and 10.3 / 10.5 /
-// 12.3; 79k 20.5 / 17.2 / 16.6 and 24.4 / 20.9 / 18.6; 267k 43.9 / 32.5 / 29.0
-// and 58.3 / 43.4 / 39.8.  So: the most that leave 8 warps for each of 148 SMs.
+// 12.3; 19k 11.1 / 10.6 / 12.4 and 11.8 / 11.8 / 12.6; 33k 13.3 / 12.7 / 12.6 and
+// 14.8 / 14.1 / 13.1; 79k 20.5 / 17.2 / 16.6 and 24.4 / 20.9 / 18.6; 267k 43.9 /
+// 32.5 / 29.0 and 58.3 / 43.4 / 39.8.  So: the most that leave 8 warps for each of
+// 148 SMs.
 inline int scatter_chunk(int n) {
     const int warps = 148 * 8;
+    return n >= 32 * warps ? 32 : n >= 16 * warps ? 16 : 8;
+}
+// The FP64 path's, whose node adds are four atomics each: fewer of them sooner pay
+// for idle SMs.  P2G and adjoint scatter together: 3.0k particles 27.8 / 30.3 / 36.9,
+// 6.3k 30.9 / 29.7 / 33.3, 13k 44.9 / 40.6 / 36.7, 19k 52.6 / 42.2 / 43.8, 33k 71.4 /
+// 57.1 / 52.8, 70k 110.8 / 82.6 / 72.7.
+inline int scatter_chunk64(int n) {
+    const int warps = 148 * 5 / 2;
     return n >= 32 * warps ? 32 : n >= 16 * warps ? 16 : 8;
 }
 // blocks of a chunk kernel over n particles, chunk particles a warp

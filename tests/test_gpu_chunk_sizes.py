@@ -1,11 +1,11 @@
-"""The chunk kernels on either side of the cloud sizes at which their launches
-change: 8, 16 or 32 sorted particles per warp of the scatters (from 18,944 and
-37,888 particles), four threads or one per particle in G2P and the adjoint gather
-(from 14,500), with ragged last warps and blocks.  tests/test_gpu_chunk.py has the
-small sizes, all of which run 8 per warp and four threads per particle.  The oracle is
-the CPU restatement of the reference in FP64; about 5 particles per cell and a crowd
-of some hundred in one, so node sums add a few hundred to a thousand float terms, and
-the bars are those of that file."""
+"""The chunk kernels on either side of the cloud sizes at which their launches change:
+8, 16 or 32 sorted particles per warp of the scatters (from 18,944 and 37,888 particles,
+in the FP64 path from 5,920 and 11,840), four threads or one per particle in G2P and the
+adjoint gather (from 14,500), with ragged last warps and blocks.  tests/test_gpu_chunk.py
+has the small sizes, all of which run 8 per warp and four threads per particle.  The
+oracle is the CPU restatement of the reference in FP64; about 5 particles per cell and a
+crowd of some hundred in one, so node sums add a few hundred to a thousand float terms,
+and the bars are those of that file."""
 import numpy as np
 import pytest
 
@@ -34,7 +34,7 @@ def _cloud(n, seed):
     return sc.float32_inputs()
 
 
-@pytest.fixture(scope="module", params=[14499, 14500, 18943, 18945, 37887, 37889, 39999, 40001, 41107])
+@pytest.fixture(scope="module", params=[5919, 5921, 11839, 11841, 14499, 14500, 18943, 18945, 37887, 37889, 39999, 40001, 41107])
 def cloud(request):
     sc = _cloud(request.param, request.param)
     exact = request.param % 4 != 1  # both adjoints over the list
