@@ -42,7 +42,7 @@ namespace {
 
 constexpr int kAux = 24;  // G (9), polar R (9), polar S (6) per particle and step
 constexpr int kDefaultSortEvery = 8;
-constexpr int kDefaultCtasPerSm = 3;
+constexpr int kDefaultCtasPerSm = 3;  // reported for callers that read the setting back; no kernel uses it
 
 // cell key of a particle of the active prefix: its instance's key offset + the
 // one-scene key of sort.cuh (the stencil base the chunk kernels form)

@@ -488,7 +488,6 @@ template <class T> class Engine : public EngineBase {
         a.s = (T)ctx_->prm.smoothing;
         for (int c = 0; c < 3; c++) a.fext[c] = (T)ctx_->prm.f_ext[c];
         a.cst = cst_;
-        a.tile_cap = tile_cap();
         a.status = status_;
         return a;
     }
@@ -1565,7 +1564,6 @@ template <class T> class Engine : public EngineBase {
         a.dbg_dLdP = P.keep_intermediates ? layers_[i].dbgdLdP : nullptr;
         a.dbg_vnext = P.keep_intermediates ? layers_[i].dbgvn : nullptr;
         a.dbg_Cnext = P.keep_intermediates ? layers_[i].dbgCn : nullptr;
-        a.tile_cap = tile_cap();
         a.status = status_;
         if (!a.st || !a.st_next || !a.grid) throw StateError{"internal: layer not materialised"};
         DMPM_CK(cudaMemsetAsync(gadj_, 0, G_ * sizeof(node4<T>), ctx_->stream));

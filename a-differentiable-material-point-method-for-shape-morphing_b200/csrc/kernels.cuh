@@ -181,7 +181,6 @@ template <class T> struct FwdArgs {
     node4<T>* grid;     // layer n grid (p, m)
     T* gridv;           // plain path: node velocities [3][G] (G_op output)
     T* P;               // [9][np] stress of layer n (plain path, or debug copy)
-    int tile_cap;
     unsigned* status;
     int strain;         // the F planes hold H = F - I (the FP32 path's layer storage)
 };
@@ -476,7 +475,6 @@ template <class T> struct AdjArgs {
     T* dbg_dLdP;          // [9][np]
     T* dbg_vnext;         // [3][np]
     T* dbg_Cnext;         // [9][np]
-    int tile_cap;
     unsigned* status;
 };
 

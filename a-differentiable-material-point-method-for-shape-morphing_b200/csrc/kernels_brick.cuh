@@ -34,8 +34,8 @@ __device__ __forceinline__ void unit_origin(uint32_t ukey, int shift, const Grid
 // stencil lies in the unit's node tile adds its (reduce-scattered) node sums to
 // the tile's shared-memory integers; the tile is then added to the global
 // integer sums, one 64-bit atomic per nonzero value.  Integer adds in any order
-// give the same sums, so the result is that of k_p2g_w / k_adj_scatter_w with
-// DET, with about (B + 3)^3 global atomics per unit instead of 64 per item and
+// give the same sums, so the result is that of k_p2g_w / k_adj_scatter_w, with
+// about (B + 3)^3 global atomics per unit instead of 64 per item and
 // node value.  Items that are not uniform or have left the unit add to global
 // memory directly.
 template <int B> __device__ __forceinline__ void fix_tile_flush(const FixTile& ft, const GridGeom& g, fix4* dst) {

@@ -10,13 +10,12 @@
 // slot q (0..7) and stencil slab s (0..3), i.e. the 16 nodes
 // (base_x + s, base_y + j, base_z + k), j, k in 0..3, fully unrolled with
 // compile-time j, k.  When all 8 particles of the warp share the cell (the
-// common case), scatters combine the 8 particles' contributions with a
+// common case), the scatters combine the 8 particles' contributions with a
 // butterfly reduce-scatter over the lanes of equal s, so each lane ends up
-// owning one node's complete sum and issues a single vector
-// red.global.add.v4.f32 per 8 nodes x 4 values; otherwise every lane issues
-// its own reductions.  Gathers sum the 16-node partial results of the 4 slab
-// lanes with two xor-shuffles.  The FP64 polar decomposition is stress_particle's
-// (k_stress, or G2P for the next step) and finalize_particle's (the gather).
+// owning one node's complete sum and adds it once, as integers (fixpoint.cuh);
+// otherwise every lane adds its own.  The FP64 polar decomposition is
+// stress_particle's (k_stress, or G2P for the next step) and finalize_particle's
+// (the gather).
 //
 // Math per stage is that of kernels.cuh (which cites the reference).
 //
@@ -145,11 +144,10 @@ __device__ __forceinline__ LaneNodes lane_nodes(const GridGeom& g, const int bas
     return r;
 }
 
-// Per-lane stencil weights: slab s of axis 0, all 4 nodes of axes 1 and 2.
+// Per-lane stencil weights: slab s of axis 0, all 4 nodes of axis 2.
 struct LaneW {
-    float d0, n0, s0;
-    float d1[4], n1[4], s1[4];
-    float d2[4], n2[4], s2[4];
+    float d0, n0;
+    float d2[4], n2[4];
 };
 // Branch-free cubic B-spline and slope (same piecewise polynomials as
 // Interpolation.h:5-30, evaluated with selects so divergent lanes do not
@@ -172,42 +170,37 @@ __device__ __forceinline__ float bsp_slope(float q) {
 // The 4 lanes of a particle (equal lane >> 2) each evaluate the weights of
 // stencil node s on all three axes; axis-2 values of the other nodes come from
 // the sibling lanes by shuffles (every lane of the warp must call this).  Axis 1
-// is left to the caller: it gets this lane's own
-// axis-1 offset, weight and slope in own1 and fetches row j's values with
-// row_weights (three shuffles) when it reaches that row, so only one row's
-// values are live at a time.  Fills d0, n0, s0 and the axis-2 arrays of w,
-// the latter in the order of node k ^ kperm (reduce_scatter8's permutation).
-__device__ __forceinline__ void lane_weights_k(const float t[3], const GridGeom& g, int s, LaneW& w, float own1[3],
-                                               bool slopes, int kperm = 0) {
+// is left to the caller: it gets this lane's own axis-1 offset and weight in own1
+// and fetches row j's values with row_weights (two shuffles) when it reaches that
+// row, so only one row's values are live at a time.  Fills d0, n0 and the axis-2
+// arrays of w, the latter in the order of node k ^ kperm (reduce_scatter8's
+// permutation).
+__device__ __forceinline__ void lane_weights_k(const float t[3], const GridGeom& g, int s, LaneW& w, float own1[2],
+                                               int kperm) {
     const float dx = (float)g.dx;
-    float d[3], n[3], sl[3];
+    float d[3], n[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         const float q = (float)s - t[c];
         d[c] = q * dx;
         n[c] = bsp(q);
-        sl[c] = slopes ? bsp_slope(q) : 0.f;
     }
     w.d0 = d[0];
     w.n0 = n[0];
-    w.s0 = sl[0];
     own1[0] = d[1];
     own1[1] = n[1];
-    own1[2] = sl[1];
     const int grp = (threadIdx.x & 31) & ~3;
 #pragma unroll
     for (int t = 0; t < 4; t++) {  // entry t holds axis-2 node t ^ kperm
         w.d2[t] = __shfl_sync(0xffffffffu, d[2], grp + (t ^ kperm));
         w.n2[t] = __shfl_sync(0xffffffffu, n[2], grp + (t ^ kperm));
-        w.s2[t] = slopes ? __shfl_sync(0xffffffffu, sl[2], grp + (t ^ kperm)) : 0.f;
     }
 }
-// row j's axis-1 (offset, weight, slope) from the lane of slab j; every lane must call it
-__device__ __forceinline__ void row_weights(const float own1[3], int j, float& d1, float& n1, float& s1) {
+// row j's axis-1 (offset, weight) from the lane of slab j; every lane must call it
+__device__ __forceinline__ void row_weights(const float own1[2], int j, float& d1, float& n1) {
     const int src = ((threadIdx.x & 31) & ~3) + j;
     d1 = __shfl_sync(0xffffffffu, own1[0], src);
     n1 = __shfl_sync(0xffffffffu, own1[1], src);
-    s1 = __shfl_sync(0xffffffffu, own1[2], src);
 }
 
 // stencil base and lattice coordinates t = (x - mn) / dx - base of particle p
@@ -263,11 +256,10 @@ __device__ __forceinline__ float store_x(float* st_next, size_t npn, int p, int 
 #ifndef DMPM_SCATTER_CTAS
 #define DMPM_SCATTER_CTAS DMPM_SCATTER_MIN_BLOCKS
 #endif
-// the adjoint scatter on its own, in blocks of 128 threads: 7 per SM (72
-// registers, 28-byte spill, 28 warps) take 53.3 us on the 64^3, 267k-particle
-// workload, against 55.4 us for 4 blocks of 256 (64 registers, 68-byte
-// spill), 59.4 us for 3 of 256 and 55.7 us for 5 of 128 (95 registers, no
-// spill); P2G is faster at 3 blocks of 256 
+// the adjoint scatter on its own, in blocks of 128 threads, 7 per SM (72 registers);
+// measured when it also formed its sources and added floats: 53.3 us on the 64^3,
+// 267k-particle scene against 55.4 us for 4 blocks of 256, 59.4 for 3 of 256 and
+// 55.7 for 5 of 128; P2G was faster at 3 blocks of 256
 #ifndef DMPM_ADJ_SCATTER_MIN_BLOCKS
 #define DMPM_ADJ_SCATTER_MIN_BLOCKS 7
 #endif
@@ -425,8 +417,8 @@ __device__ __forceinline__ void p2g_item(const WArgs& a, int item, const FixScal
         // slot (jj, kk) of each half holds node (2 half + (jj ^ P.jp), kk ^ P.kp)
         const ScatterPerm P = scatter_perm();
         LaneW w;
-        float own1[3];
-        lane_weights_k(t, geo, L.s, w, own1, false, P.kp);
+        float own1[2];
+        lane_weights_k(t, geo, L.s, w, own1, P.kp);
         const float mp = L.valid ? a.cst[(size_t)KM * np + L.p] : 0.f;
         const float damp = 1.f - a.dt * a.drag;
         float mvd[3], g0[3];
@@ -444,8 +436,8 @@ __device__ __forceinline__ void p2g_item(const WArgs& a, int item, const FixScal
             float v[32];
 #pragma unroll
             for (int jj = 0; jj < 2; jj++) {
-                float d1, n1, s1;
-                row_weights(own1, 2 * half + (jj ^ P.jp), d1, n1, s1);
+                float d1, n1;
+                row_weights(own1, 2 * half + (jj ^ P.jp), d1, n1);
                 float g1[3];
 #pragma unroll
                 for (int c = 0; c < 3; c++) g1[c] = g0[c] + G.a[c][1] * d1;
@@ -676,8 +668,8 @@ __device__ __forceinline__ void adj_scatter_items(const WArgs& a, int first, int
         const bool uniform = !GENERAL && warp_uniform_base(base);
         const ScatterPerm P = scatter_perm();  // as in p2g_item
         LaneW w;
-        float own1[3];
-        lane_weights_k(t, geo, L.s, w, own1, false, P.kp);
+        float own1[2];
+        lane_weights_k(t, geo, L.s, w, own1, P.kp);
         float vn[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) vn[c] = a.adjn[(size_t)c * np + p];
@@ -694,8 +686,8 @@ __device__ __forceinline__ void adj_scatter_items(const WArgs& a, int first, int
             float v[24];  // 8 nodes x dLdv_g (3)
 #pragma unroll
             for (int jj = 0; jj < 2; jj++) {
-                float d1, n1, s1;
-                row_weights(own1, 2 * half + (jj ^ P.jp), d1, n1, s1);
+                float d1, n1;
+                row_weights(own1, 2 * half + (jj ^ P.jp), d1, n1);
                 float c1[3];
 #pragma unroll
                 for (int r = 0; r < 3; r++) c1[r] = c0[r] + k3 * Cn.a[r][1] * d1;
@@ -797,8 +789,9 @@ __global__ void __launch_bounds__(256)
 //   REFCOMPAT: dLdF = (1-s)T + s dLdF' + stress + T + dP:dLdP,  T = (I + dt C')^T dLdF'
 //   EXACT:     dLdFe = (1-s)T + stress + dP:dLdP,  dLdF = dLdFe + s dLdF'
 //
-// Its inputs are 94 FP32 planes per particle (slots below) and, with tied
-// controls, the 9 FP64 planes of the control-gradient accumulator.
+// Its inputs are 94 floats per particle (slots below), of which the gather's 18 sums
+// are in registers and 18 are staged in shared memory by then, the rest in planes,
+// and, with tied controls, the 9 FP64 planes of the control-gradient accumulator.
 enum : int {
     FS_GATH = 0,    // 18: M (9, row-major), X (3), u (3), z (3)
     FS_F = 18,      // 9: strain H = F - I of layer n
