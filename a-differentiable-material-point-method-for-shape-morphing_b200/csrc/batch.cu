@@ -8,10 +8,10 @@
 // of that order, stored with its own plane stride S_t.  Time step t advances
 // the instances with steps > t, again a prefix: P_t particles, G_t nodes.
 //
-// Launches.  Every stage of a time step is one launch over the prefix: P2G, G2P
-// with the next step's stress stage, the adjoint scatter and the gather with the
-// finalize (kernels_chunk.cuh) over P_t particles in cell order, the node kernels
-// over G_t nodes.  A cell's particles never mix instances (cell keys carry the
+// Launches.  Every stage of a time step is one launch over the prefix: P2G and the
+// adjoint scatter over P_t particles in cell order, G2P with the next step's stress
+// stage and the gather with the finalize over them as stored (kernels_chunk.cuh), the
+// node kernels over G_t nodes.  A cell's particles never mix instances (cell keys carry the
 // instance's key offset); each lane looks up its particle's grid.  No result is
 // read back inside a gradient evaluation, so the whole evaluation can be
 // captured once as a CUDA graph.

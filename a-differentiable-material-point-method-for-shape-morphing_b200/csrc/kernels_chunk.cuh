@@ -1,4 +1,5 @@
-// kernels_chunk.cuh -- FP32 path scatters over chunks of the sorted order.
+// kernels_chunk.cuh -- FP32 path: the scatters over chunks of the sorted order, and the
+// gathers by particle.
 //
 // A warp takes up to 32 consecutive particles of the cell-sorted order (a chunk).
 // First one lane per particle loads its inputs, forms its stencil base and
@@ -301,18 +302,23 @@ __device__ __forceinline__ void axis_stencil(float t, float dx, float n[4], floa
 }
 
 // ------------------------------------------------------------------ adjoint gather + finalize
-// One thread per particle of the sorted order, reading the nodes where they lie:
-// the particles of a warp share one to three cells, so their reads are
-// broadcasts from L1.  The thread keeps the 18 sums of its particle in registers
+// One thread per particle, reading the nodes where they lie.  Particles are taken as
+// they are stored, not in cell order: their 110 planes then come in whole sectors,
+// and the nodes of a cloud lie in L2 whichever particle asks.  In a spatial order
+// (lattice, cell order) a warp's reads are broadcasts from L1 or nearly so; in a
+// random one the planes would cost a sector per value in cell order.  Gather and
+// G2P at 267k particles in lattice order 92.4 and 47.4 us (in cell order 99.1 and
+// 49.9), in random order 126.5 and 66.3 (289.9 and 157.2); 2.0M in lattice order 440
+// and 244 (471 and 275); stored in cell order the same.  The thread keeps the 18 sums of its particle in registers
 // and goes on to the finalize with them (as two kernels the sums made a round
 // trip of 144 bytes per particle, and the finalize a second and a third launch).
 // Small clouds give a particle four threads, one per stencil slab (SPLIT).
 //
-// Measured per step on the 64^3, 267k-particle rollout (event times): 98 us, and
-// the warp-item gather with the two finalize kernels behind it 82.6 + 41.4 (+ 14.6
-// beside them); 79k particles with the reference's adjoint 33 against 27 + 57 us;
-// 8.7k particles 14.7 against 12.6 + 8.7.  The node sums take 55 us of the 98 (in a
-// kernel of their own): 22.3 M warp instructions at 42 % issue with 16 warps per
+// Measured per step on the 64^3, 267k-particle rollout (event times, in cell order as
+// are the rest): 98 us, and the warp-item gather with the two finalize kernels behind
+// it 82.6 + 41.4 (+ 14.6 beside them); 79k particles with the reference's adjoint 33
+// against 27 + 57 us; 8.7k particles 14.7 against 12.6 + 8.7.  The node sums take
+// 55 us of the 98 (in a kernel of their own): 22.3 M warp instructions at 42 % issue with 16 warps per
 // SM, which wait for L1 and L2 at each of the 16 stencil rows.  What did not help:
 // the warp's nodes copied to shared memory as one box first (58.6 us: the waits
 // went, 8 M instructions came), 12 warps without spills or 20 with more (58 /
@@ -359,9 +365,9 @@ __device__ __forceinline__ void load_pair(const node4<float>* p, f32x2 (&f)[4]) 
 // whole stencil lies in the grid; otherwise nodes outside it read as zero.  A grid
 // has up to 2e9 nodes, so a stencil inside it spans less than 2^31 single records and
 // 2^32 of pairs; one that reaches over the grid's edge may be longer than the grid,
-// and its rows need 64 bits.  At 267k particles G2P 49.6 us and the gather 99.0
-// (49.5 and 98.6 in ints throughout; with unsigned offsets in G2P too 50.3, with 64
-// bits for all stencils the gather 99.8).
+// and its rows need 64 bits.  At 267k particles, in cell order, G2P 49.6 us and the
+// gather 99.0 (49.5 and 98.6 in ints throughout; with unsigned offsets in G2P too
+// 50.3, with 64 bits for all stencils the gather 99.8).
 template <bool INSIDE, int R> struct StencilNodes {
     const node4<float>* g;  // the base node's first record (dereferenced inside the grid only)
     unsigned si, sj;        // records per slab and row
@@ -464,12 +470,11 @@ __device__ __forceinline__ void g2p_sums(const Nodes& f, const float t[3], float
     }
 }
 
-// One thread per particle of the sorted order (four of small clouds), as the
-// adjoint gather.  Per step, with the next stress stage (event times; before: a
-// CTA per brick octant that staged its node tile behind two barriers, 2.1 waves of
-// them): 267k particles 49 against 64 us, 301k at 8 per cell 47 against 87, 2.0M
-// 280 against 490, 8.7k 12.7 against 14; 3 or 5 blocks per SM 51 / 52 us on the
-// first.  F' = (1 - s)(I + dt C')(F + dFc) + s F;  x' = x + dt v'.
+// One thread per particle (four of small clouds) in storage order, as the adjoint
+// gather.  Per step, with the next stress stage (event times; before: a CTA per
+// brick octant that staged its node tile behind two barriers, 2.1 waves of them):
+// 267k particles 47 against 64 us, 301k at 8 per cell 46 against 87, 2.0M 244 against
+// 490, 8.7k 12.4 against 14; 3 or 5 blocks per SM each 2 us more on the first.  F' = (1 - s)(I + dt C')(F + dFc) + s F;  x' = x + dt v'.
 // STRESS: also the next step's stress stage from the strain and C just formed
 // (stress_particle, the arithmetic of k_stress), into a.G_next, for the first
 // a.n_next particles -- one pass over the particles fewer per step.
@@ -483,7 +488,7 @@ __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, STRESS ? DMPM_CHUNK_G2P_MI
     if ((q & ~(32 / SPLIT - 1)) >= a.n) return;  // the whole warp
     if (!BATCH && blockIdx.x == 0 && a.box_next) box_join(a.box_next, a.box);
     const size_t np = a.np, npl = a.npl, npn = a.npn;
-    const int p = (int)a.items.order[min(q, a.n - 1)];
+    const int p = min(q, a.n - 1);
     const int inst = BATCH ? (int)a.pinst[p] : 0;
     const GridGeom& geo = chunk_geo<BATCH>(a, inst);
     const int goff = BATCH ? a.ig[inst].goff : 0;
@@ -674,7 +679,7 @@ __global__ void __launch_bounds__(DMPM_CHUNK_THREADS, DMPM_CHUNK_GATHER_MINB) k_
     float* col = s_col + (threadIdx.x >> 5) * 32 * kStaged + (threadIdx.x & 31);
     float2* w1s = s_w1 + (threadIdx.x >> 5) * 128 + (threadIdx.x & 31);
     const size_t np = a.np, npl = a.npl;
-    const int p = (int)a.items.order[min(q, a.n - 1)];
+    const int p = min(q, a.n - 1);
     const int inst = BATCH ? (int)a.pinst[p] : 0;
     const GridGeom& geo = chunk_geo<BATCH>(a, inst);
     const int goff = BATCH ? a.ig[inst].goff : 0;
@@ -711,9 +716,9 @@ inline int particle_threads(int n) {
 }
 // Threads per particle of G2P and the gather.  Four shorten the chain of a cloud that
 // leaves SMs idle and repeat the weights of each; from 19k particles they also need a
-// second wave of blocks.  A step forward and back, us with four / with one: 8.7k
-// particles 40.3 / 45.3, 13.1k 45.7 / 48.1, 14.4k 48.3 / 48.2, 16.0k 50.1 / 49.7, 19.4k
-// 61.3 / 50.0, 32.8k 76.2 / 55.7, 39.5k 89.4 / 60.3.
+// second wave of blocks.  A step forward and back, us with four / with one: 3.0k
+// particles 31.9 / 37.2, 8.7k 37.3 / 42.4, 13.1k 42.5 / 44.9, 14.4k 46.4 / 46.4, 16.0k
+// 47.4 / 46.0, 19.4k 58.0 / 46.5, 26.6k 66.8 / 49.0, 39.5k 84.2 / 56.8.
 inline int particle_split(int n) { return n < 14500 ? 4 : 1; }
 // G2P, with the next stress stage where a.G_next is set
 template <bool BATCH> inline void launch_g2p(const WArgs& a, cudaStream_t st) {
