@@ -16,10 +16,12 @@
 
 #include <algorithm>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <type_traits>
@@ -100,6 +102,76 @@ inline void unpack_ref_rows(const float* rows, int W, size_t a, size_t b, float*
         std::memcpy(d + kRefFixedAt, r + kRefState, (size_t)(W - kRefState) * sizeof(float));
     }
 }
+// Writes rows into the caller's structs, shared with threads that last as long as it
+// (one core's stores are slower than the copies that bring the rows).
+class RowWriters {
+   public:
+    RowWriters(float* pts, int W, int extra) : pts_(pts), W_(W) {
+        try {
+            threads_.reserve((size_t)extra);
+            for (int t = 1; t <= extra; t++) threads_.emplace_back([this, t] { work(t); });
+        } catch (...) {  // no more threads to be had: those there are share the rows
+        }
+    }
+    ~RowWriters() {
+        {
+            std::lock_guard<std::mutex> lock(m_);
+            quit_ = true;
+        }
+        go_.notify_all();
+        for (std::thread& t : threads_) t.join();
+    }
+    // rows [a, end), all written when it returns
+    void write(const float* rows, size_t a, size_t end) {
+        const size_t team = threads_.size() + 1;
+        if (team > 1) {
+            std::lock_guard<std::mutex> lock(m_);
+            job_ = Job{rows, a, end, (end - a + team - 1) / team};
+            busy_ = team - 1;
+            round_++;
+        } else {
+            job_ = Job{rows, a, end, end - a};
+        }
+        go_.notify_all();
+        share(job_, 0);
+        if (team > 1) {
+            std::unique_lock<std::mutex> lock(m_);
+            idle_.wait(lock, [this] { return busy_ == 0; });
+        }
+    }
+
+   private:
+    struct Job {
+        const float* rows = nullptr;
+        size_t a = 0, end = 0, part = 0;
+    };
+    void share(const Job& j, size_t t) const {
+        const size_t from = std::min(j.end, j.a + t * j.part), to = std::min(j.end, from + j.part);
+        if (from < to) unpack_ref_rows(j.rows + (from - j.a) * W_, W_, from, to, pts_);
+    }
+    void work(int t) {
+        std::unique_lock<std::mutex> lock(m_);
+        for (unsigned seen = 0;;) {
+            go_.wait(lock, [&] { return quit_ || round_ != seen; });
+            if (quit_) return;
+            seen = round_;
+            const Job j = job_;
+            lock.unlock();
+            share(j, (size_t)t);
+            lock.lock();
+            if (--busy_ == 0) idle_.notify_one();
+        }
+    }
+    float* pts_;
+    const int W_;
+    std::vector<std::thread> threads_;
+    std::mutex m_;
+    std::condition_variable go_, idle_;
+    Job job_;
+    size_t busy_ = 0;
+    unsigned round_ = 0;
+    bool quit_ = false;
+};
 // Grid fields of one layer.  The stored node holds (p, m), or, where the
 // FP32 path's grid update has overwritten p in place (stored_v), (v, m): then
 // v is read as stored and p is recovered as (v - dt f) m on nodes with
@@ -1872,9 +1944,12 @@ template <class T> class Engine : public EngineBase {
 
     // One kernel packs the filled fields of every point, and the packed rows come
     // through two pinned buffers, the next one's copy running while the host writes
-    // the last one's rows into the structs (on a few threads, as one core's stores
-    // are slower than the copy).  Field by field through double arrays, 79k points
-    // took 10.3 ms; 2 buffers of 4 MB serve any cloud.
+    // the last one's rows into the structs.  Field by field through double arrays, 79k
+    // points took 10.3 ms.  The buffers are of 512 KB, which the driver takes from the
+    // 2 MB that it has pinned for the status words: a context's first call takes 0.23 ms
+    // at 8.7k points and 1.1 at 58k, with buffers of 4 MB 3.1 and 13, field by field 0.9
+    // and 5.7; later calls 0.20 and 1.25 (0.44 and 1.45 with 4 MB, 3.3 and 2.9 at 172k).
+    // Four threads write clouds of more than 8 MB of rows; below, they gain nothing.
     void get_points_ref(int l, void* pts) {
         if (!pts) throw ArgError{"points is NULL"};
         if (l < 0 || l >= L_) throw ArgError{"layer out of range"};
@@ -1886,40 +1961,24 @@ template <class T> class Engine : public EngineBase {
         k_pack_ref<T, kStrain><<<(unsigned)((n_ + 127) / 128), 128, 0, ctx_->stream>>>(st, cst_, layers_[l].dfc, adj, np_,
                                                                                       n_, perm(), W, dev);
         launched();
-        const size_t rows = std::min<size_t>((size_t)n_, ((size_t)4 << 20) / (W * sizeof(float)));
+        const size_t rows = std::min<size_t>((size_t)n_, kPinned / (W * sizeof(float)));
         ensure_pinned(rows * W * sizeof(float));
         auto copy = [&](size_t a, int b) {
             const size_t cnt = std::min(rows, (size_t)n_ - a);
             DMPM_CK(cudaMemcpyAsync(pin_[b], dev + a * W, cnt * W * sizeof(float), cudaMemcpyDeviceToHost, ctx_->stream));
             DMPM_CK(cudaEventRecord(pin_ev_[b], ctx_->stream));
         };
+        const int cores = (int)std::min(4u, std::max(1u, std::thread::hardware_concurrency()));
+        RowWriters out((float*)pts, W, (size_t)n_ * W * sizeof(float) > kThreadedRows ? cores - 1 : 0);
         int b = 0;
         copy(0, 0);
         for (size_t a = 0; a < (size_t)n_; a += rows, b ^= 1) {
             if (a + rows < (size_t)n_) copy(a + rows, b ^ 1);
             DMPM_CK(cudaEventSynchronize(pin_ev_[b]));
-            const size_t end = std::min((size_t)n_, a + rows);
-            const float* src = (const float*)pin_[b];
-            // threads for chunks above 1 MB: below, starting them costs more than it saves
-            const size_t bytes = (end - a) * W * sizeof(float);
-            const int extra = bytes > (1u << 20) ? (int)std::min<unsigned>(3, std::max(1u, std::thread::hardware_concurrency()) - 1) : 0;
-            const size_t part = (end - a + extra) / (extra + 1);
-            std::vector<std::thread> th;
-            th.reserve(3);
-            size_t done = std::min(end, a + part);  // this thread's share: the first part and what no thread took
-            try {
-                for (int t = 0; t < extra && done < end; t++) {
-                    const size_t to = std::min(end, done + part);
-                    th.emplace_back(unpack_ref_rows, src + (done - a) * W, W, done, to, (float*)pts);
-                    done = to;
-                }
-            } catch (...) {  // no more threads to be had
-            }
-            unpack_ref_rows(src, W, a, std::min(end, a + part), (float*)pts);
-            if (done < end) unpack_ref_rows(src + (done - a) * W, W, done, end, (float*)pts);
-            for (std::thread& t : th) t.join();
+            out.write((const float*)pin_[b], a, std::min((size_t)n_, a + rows));
         }
     }
+    static constexpr size_t kPinned = (size_t)512 << 10, kThreadedRows = (size_t)8 << 20;
     void ensure_pinned(size_t bytes) {
         if (bytes <= pin_bytes_) return;
         for (int b = 0; b < 2; b++) {
