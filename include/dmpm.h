@@ -369,6 +369,8 @@ int dmpm_batch_stream(const dmpm_batch* b, void** stream);
  *   V: nv * 3 floats;  F: nf * 3 vertex indices (0-based)
  *   out: capacity * 3 floats (NULL with capacity 0 to count only)
  *   *count: the number of points kept; DMPM_ERR_TOO_LARGE when > capacity
+ * The device scratch of these and of the surface calls comes from a pool of the
+ * library, one per CUDA context, that keeps up to 256 MB between calls.
  * ------------------------------------------------------------------------ */
 int dmpm_mesh_lattice_dims(const float* min_point, const float* max_point, float sampling_dx, int* dims);
 int dmpm_mesh_lattice_points(const float* V, int nv, const int* F, int nf, const float* min_point,

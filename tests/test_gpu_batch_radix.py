@@ -46,3 +46,25 @@ def test_batch_over_the_radix_sort(gpu_ready, graph):
                     c.backward(0)
                     assert relerr(b.get(i, s.steps, "x"), c.get(s.steps, "x")) < 1e-5, i
                     assert normrel(b.control_grad(i), c.control_grad()) < 1e-3, i
+
+
+def test_fp64_path_over_the_radix_sort(gpu_ready):
+    """The FP64 path on a grid whose order comes from the radix sort against the same cloud, moved by
+    whole cells, on one that counts: the same sums in another order, positions to the rounding of
+    coordinates of 130 cells (an absolute 3e-14, amplified by the node masses' quotients)."""
+    a = _scene(1, (260, 260, 60), 1500, 3)
+    b = _scene(1, (260, 260, 60), 1500, 3)
+    shift = np.array([98.0, 115.0, 15.0])
+    b.x = a.x - shift  # exact: float32 positions below 256 less whole numbers
+    b.dims = (64, 30, 30)
+    out = []
+    for s in (a, b):
+        with make_ctx(s, "fp64", np.zeros(int(np.prod(s.dims))), adjoint="exact", control="tied", sort_every=2) as c:
+            c.setup(s.steps + 1)
+            c.forward(0)
+            c.loss()
+            c.backward(0)
+            out.append((c.get(s.steps, "x"), c.get(s.steps, "F"), c.control_grad()))
+    assert np.abs(out[0][0] - shift - out[1][0]).max() < 1e-10
+    assert relerr(out[0][1], out[1][1]) < 1e-10
+    assert normrel(out[0][2], out[1][2]) < 1e-8
