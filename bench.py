@@ -331,7 +331,8 @@ def roofline(kstats, n: int, touched: int, peak: float, peak_kind: str, determin
         if rate[k]:
             kern[k]["hbm_frac"] = rate[k] / peak
     return kern, {"kernel": top, "bound": "hbm", "achieved": rate[top] or None, "peak": peak, "unit": "GB/s",
-                  "frac": rate[top] / peak or None, "peak_source": peak_kind, "traffic": committed_traffic(top),
+                  "frac": rate[top] / peak or None, "peak_source": peak_kind,
+                  "traffic": None if deterministic else committed_traffic(top),
                   "algorithmic_bytes_per_launch": launch_bytes(top, n, touched, deterministic) or None,
                   "avg_launch_us": kern[top]["avg_us"]}
 

@@ -39,5 +39,6 @@ def test_roofline_entry():
     assert kern["g_op"]["hbm_frac"] == pytest.approx(480 / 7.5e-6 / 1e9 / 5000.0)
     kern, roof = bench.roofline(stats, 1000, 10, 5000.0, "measured", deterministic=True)
     assert roof["kernel"] == "adj_p2g_gather" and roof["achieved"] is None and roof["frac"] is None
+    assert roof["traffic"] is None  # the recorded figure is the float kernel's
     assert not any("hbm_frac" in v for v in kern.values())
     assert bench.roofline({}, 1000, 10, 5000.0, "measured", deterministic=False) == ({}, None)
